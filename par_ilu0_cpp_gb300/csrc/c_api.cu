@@ -396,15 +396,16 @@ int LLJBASH_IluSolverGetInfo(IluSolverHdl hdl, LLJBASH_IluInfo* info) {
     info->grid_fp64 = im->line_use64;
     info->grid_fp32 = im->line_use32;
     if (im->grid64 || im->grid32) {
-        info->grid_nx = im->GP.g.nx;
-        info->grid_ny = im->GP.g.ny;
-        info->grid_nz = im->GP.g.nz;
-        info->grid_warp_y = im->GP.g.wy;
-        info->grid_warp_z = im->GP.g.wz;
-        info->grid_cta_y = im->GP.g.by;
-        info->grid_cta_z = im->GP.g.bz;
-        info->grid_blocks = im->GP.g.nblk;
-        info->grid_cluster = im->GP.g.cl;
+        const gb300::LineGeom& g = im->grid64 ? im->GP64.g : im->GP32.g;
+        info->grid_nx = g.nx;
+        info->grid_ny = g.ny;
+        info->grid_nz = g.nz;
+        info->grid_warp_y = g.wy;
+        info->grid_warp_z = g.wz;
+        info->grid_cta_y = g.by;
+        info->grid_cta_z = g.bz;
+        info->grid_blocks = g.nblk;
+        info->grid_cluster = g.cl;
     }
     return 0;
 }
@@ -413,12 +414,12 @@ int LLJBASH_IluSolverGetSweepTimeline(IluSolverHdl hdl, int upper, int fp32, uns
     try {
         const auto* im = ilu(hdl)->impl();
         if (!im) throw std::runtime_error("SetupMatrix() has not been called");
-        const auto& buf = im->GP.tl[fp32 ? 1 : 0][upper ? 1 : 0];
+        const auto& buf = fp32 ? im->GP32.tl[upper ? 1 : 0] : im->GP64.tl[upper ? 1 : 0];
         if (buf.get() == nullptr)
             throw std::runtime_error(
                 "no sweep timeline: set LLJBASH_ILU_OPT_SWEEP_TIMELINE before IluSolverSetup (line-pipeline sweeps of "
                 "structured factors only)");
-        const int nblk = im->GP.g.nblk;
+        const int nblk = fp32 ? im->GP32.g.nblk : im->GP64.g.nblk;
         const size_t len = static_cast<size_t>(nblk) * gb300::kLineTimeline;
         if (out != nullptr) {
             if (cap < 0 || static_cast<size_t>(cap) < len) throw std::runtime_error("timeline buffer too small");

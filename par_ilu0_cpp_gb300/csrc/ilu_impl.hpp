@@ -107,29 +107,32 @@ struct BlockPack {
 // Structured-grid factor (line-pipeline sweeps, line_sweep.cuh): block geometry, ticket
 // order and the packed operand streams of L and U per value type (rebuilt from the factor
 // values after every factorisation).
+template <class T>
 struct LinePack {
     LineGeom g;
-    int threads = 0;  // CTA size: nw warps
+    int threads = 0;  // CTA size: g.threads()
     int grid = 0;     // CTAs launched
     int smem_floor = 0;  // dynamic shared memory requested at least (bytes; one CTA per SM)
-    DeviceBuffer<int> order;        // [nblk] block of each ticket
-    DeviceBuffer<double> l64, u64;  // [4 slots]
-    DeviceBuffer<float> l32, u32;
-    // per-block timelines [fp32][upper] of the last sweep of each kind (allocated only
-    // with the timeline option on)
-    DeviceBuffer<unsigned long long> tl[2][2];
+    DeviceBuffer<int> order;   // [nblk] block of each ticket
+    DeviceBuffer<T> l, u;      // operand streams
+    DeviceBuffer<T> lo, div;   // [slots] FP64 U: low part of the reciprocals, diagonal
+    // Faces handed over through L2, at the sentinel between launches: [0] for the sweeps of
+    // GMRES and Substitute (one stream at a time, as their ticket counters), [1] (FP64) for
+    // the allocation-free entry point, which may run beside them.
+    DeviceBuffer<T> xch[2];
+    // per-block timelines [upper] of the last sweep of each kind (allocated only with the
+    // timeline option on)
+    DeviceBuffer<unsigned long long> tl[2];
 
-    template <class T>
-    LineTri<T> view(bool upper) const {
+    LineTri<T> view(bool upper, int set) const {
         LineTri<T> p;
         p.g = g;
         p.order = order.get();
-        p.tl = tl[sizeof(T) == 4 ? 1 : 0][upper ? 1 : 0].get();
-        if constexpr (sizeof(T) == 8) {
-            p.coef = upper ? u64.get() : l64.get();
-        } else {
-            p.coef = upper ? u32.get() : l32.get();
-        }
+        p.tl = tl[upper ? 1 : 0].get();
+        p.coef = upper ? u.get() : l.get();
+        p.rlo = lo.get();
+        p.div = div.get();
+        p.xch = xch[set].get();
         return p;
     }
 };
@@ -188,7 +191,15 @@ struct IluSolver::Impl {
     int grid_levelsync = 0;
     // structured-grid line-pipeline sweeps (line_sweep.cuh) per value type, when the
     // factor is a 7- or 5-point stencil in natural order and grid_mode allows it
-    gb300::LinePack GP;
+    gb300::LinePack<double> GP64;
+    gb300::LinePack<float> GP32;
+    template <class T>
+    const gb300::LinePack<T>& line_pack() const {
+        if constexpr (sizeof(T) == 8)
+            return GP64;
+        else
+            return GP32;
+    }
     bool grid64 = false, grid32 = false;
     int grid_mode = 0;  // 1 or 0 (automatic): on when the pattern qualifies; -1: off
     int grid_wy = 0;    // requested lanes of a warp along y (0 automatic)
@@ -249,6 +260,8 @@ struct IluSolver::Impl {
     const void* subst_key() const;
     // Throws when a dependency wait timed out since the last call.
     void check_status(cudaStream_t s);
+    // Puts the line sweeps' exchange buffers back to the sentinel (after a timeout).
+    void reset_exchange(cudaStream_t s);
     // Writes wait_limit_us into the device status words (when they exist).
     void push_wait_limit();
 };

@@ -820,7 +820,12 @@ static bool detect_grid(int n, const int* rp, const int* ci, const std::vector<i
 // Block geometry of the line-pipeline sweeps: lanes of a warp along y (wy, and
 // wz = 32 / wy along z; a 2-D grid, ny = 1, has wy = 1) and warps of a CTA along y and z
 // (by, bz).  Requested values (0 = automatic) are clamped to what the grid allows.
-static LineGeom line_geometry(int nx, int ny, int nz, int wy_req, int by_req, int bz_req) {
+// Automatic: 2-D one warp per CTA (handoffs through distributed shared memory cost no more
+// than those in a CTA, and each warp has an SM's pipes); 3-D 2 x 2 warps for FP32 and 2 x 1
+// for FP64 (elem 8), which leaves fewer blocks waiting beside the working ones: 128^3 FP64
+// forward / backward 131 / 176 us with 2 x 1 in clusters of 4, 192 / 297 us with 2 x 2;
+// FP32 82 / 77 us with 2 x 2 in clusters of 8, 96 / 87 us with 2 x 1).
+static LineGeom line_geometry(int nx, int ny, int nz, int wy_req, int by_req, int bz_req, int elem) {
     LineGeom g;
     g.nx = nx;
     g.ny = ny;
@@ -835,9 +840,7 @@ static LineGeom line_geometry(int nx, int ny, int nz, int wy_req, int by_req, in
     g.wz = 32 / wy;
     const int wly = ceil_div(ny, g.wy), wlz = ceil_div(nz, g.wz);  // warps along y / z
     int by = ny > 1 ? (by_req > 0 ? by_req : 2) : 1;
-    // (2-D: one warp per CTA, so that the forward sweep's block-by-block rescale of the
-    // Krylov vector is spread over as many CTAs as there are warps)
-    int bz = bz_req > 0 ? bz_req : (ny > 1 ? 2 : 1);
+    int bz = bz_req > 0 ? bz_req : (ny > 1 && elem == 4 ? 2 : 1);
     by = std::max(1, std::min(by, wly));
     bz = std::max(1, std::min(bz, wlz));
     if (ny > 1) {  // the halo warp holds one line of each incoming face per lane
@@ -851,6 +854,7 @@ static LineGeom line_geometry(int nx, int ny, int nz, int wy_req, int by_req, in
     g.nbz = ceil_div(wlz, bz);
     g.nblk = g.nby * g.nbz;
     g.steps = nx + g.wy + g.wz - 2;
+    g.psteps = ceil_div(g.steps, kLineStepAlign) * kLineStepAlign;
     return g;
 }
 
@@ -885,6 +889,22 @@ static cudaLaunchConfig_t line_cluster_config(int grid, int threads, size_t smem
     return cfg;
 }
 
+// The line kernels of a geometry (lanes along y; 2-D grids have none).
+template <class T, bool UPPER>
+using LineKernel = void (*)(LineTri<T>, T*, const double*, T*, unsigned*, int*, const int*, int);
+template <class T, bool UPPER>
+static LineKernel<T, UPPER> line_kernel(const LineGeom& g, bool cluster) {
+    if (g.ny == 1) return cluster ? sptrsv_line_cluster_kernel<T, UPPER, 1, false> : sptrsv_line_kernel<T, UPPER, 1, false>;
+    if (g.wy == 1) return cluster ? sptrsv_line_cluster_kernel<T, UPPER, 1, true> : sptrsv_line_kernel<T, UPPER, 1, true>;
+    if (g.wy == 4) return cluster ? sptrsv_line_cluster_kernel<T, UPPER, 4, true> : sptrsv_line_kernel<T, UPPER, 4, true>;
+    return cluster ? sptrsv_line_cluster_kernel<T, UPPER, 8, true> : sptrsv_line_kernel<T, UPPER, 8, true>;
+}
+template <class T>
+static const void* line_kernel_ptr(const LineGeom& g, bool cluster, bool upper) {
+    return upper ? reinterpret_cast<const void*>(line_kernel<T, true>(g, cluster))
+                 : reinterpret_cast<const void*>(line_kernel<T, false>(g, cluster));
+}
+
 // Raises the kernels' shared-memory limit, sizes the grid and allocates the packed
 // operands of value type T; false when a CTA cannot be resident.  With G.g.cl > 0 the
 // cluster variant is sized (clusters of cl CTAs along z); `try_cluster` (first type
@@ -892,98 +912,109 @@ static cudaLaunchConfig_t line_cluster_config(int grid, int threads, size_t smem
 // has at least two blocks along z and such a cluster can be scheduled; with 2 .. 16,
 // clusters of at most that many CTAs; with 0, none.
 template <class T>
-static bool configure_line(LinePack& G, const DeviceInfo& dev, bool try_cluster, int max_cluster) {
-    const size_t smem = std::max(static_cast<size_t>(line_smem_bytes<T>(G.g)), static_cast<size_t>(G.smem_floor));
+static bool configure_line(LinePack<T>& G, const DeviceInfo& dev, int max_cluster) {
+    const size_t smem = std::max(static_cast<size_t>(std::max(line_smem_bytes<T, false>(G.g), line_smem_bytes<T, true>(G.g))),
+                                 static_cast<size_t>(G.smem_floor));
     if (smem + 1024 > static_cast<size_t>(dev.smem_optin)) return false;
-    if (try_cluster) {
+    {
         G.g.cl = 0;
         G.g.nbzc = 0;
-        // clusters of 16 (non-portable) where they can be scheduled, else of 8
-        const int wants[2] = {max_cluster == 1 ? 16 : max_cluster, max_cluster == 1 ? 8 : 0};
-        for (int want : wants) {
-            if (want < 2 || G.g.nbz < 2 || G.g.cl > 0) break;
+        // automatic: the largest of 16 (non-portable), 8, 4 and 2 CTAs of which all
+        // clusters are resident at once; for grids that do not fit at once, 8 for FP32 and 4
+        // for FP64 (the measurements above line_geometry)
+        const int most = G.g.ny == 1 ? 16 : (sizeof(T) == 4 ? 8 : 4);
+        for (int want : {16, 8, 4, 2}) {
+            if (max_cluster != 1) want = max_cluster;
+            if (want < 2 || G.g.nbz < 2) break;
             const int cl = std::min(want, G.g.nbz);
             const int nbzc = ceil_div(G.g.nbz, cl);
-            int ok = 1;
+            const int need = G.g.nby * nbzc;
             int nclusters = 1 << 30;
             for (bool upper : {false, true}) {
-                const void* kern = upper ? reinterpret_cast<const void*>(sptrsv_line_cluster_kernel<T, true>)
-                                         : reinterpret_cast<const void*>(sptrsv_line_cluster_kernel<T, false>);
+                const void* kern = line_kernel_ptr<T>(G.g, true, upper);
                 GB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
                 if (cl > 8) GB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
                 cudaLaunchAttribute attr[1];
-                cudaLaunchConfig_t cfg = line_cluster_config(G.g.nby * nbzc * cl, G.threads, smem, cl, nullptr, attr);
+                cudaLaunchConfig_t cfg = line_cluster_config(need * cl, G.threads, smem, cl, nullptr, attr);
                 int nc = 0;
                 if (cudaOccupancyMaxActiveClusters(&nc, kern, &cfg) != cudaSuccess) {
                     cudaGetLastError();
                     nc = 0;
                 }
-                if (nc < 1) ok = 0;
                 nclusters = std::min(nclusters, nc);
             }
-            if (ok) {
-                G.g.cl = cl;
-                G.g.nbzc = nbzc;
-                G.grid = std::min(nclusters, G.g.nby * nbzc) * cl;
+            if (nclusters >= need || (nclusters > 0 && want <= most) || max_cluster != 1) {
+                if (nclusters > 0) {
+                    G.g.cl = cl;
+                    G.g.nbzc = nbzc;
+                    G.grid = std::min(nclusters, need) * cl;
+                }
+                break;
             }
         }
     }
+    // Tickets launched at once: blocks more than kLineWaitLines lines deep would wait past
+    // about 60 us, after which a block's first steps run five times slower (seen in the
+    // timelines, whatever the waiting warps do); they are left to the CTAs that finish first
+    // (96^3 FP64 backward: 172 us with all 144 blocks resident, 125 us with 120 or 128).
+    constexpr int kLineWaitLines = sizeof(T) == 8 ? 130 : 300;
+    const int unit = std::max(1, G.g.cl);
+    int early = 0;
+    for (int iz = 0; iz < ceil_div(G.g.nbz, unit); ++iz)
+        for (int iy = 0; iy < G.g.nby; ++iy)
+            if (iy * G.g.by * G.g.wy + iz * unit * G.g.bz * G.g.wz <= kLineWaitLines) early += unit;
     if (G.g.cl > 0) {
+        G.grid = std::min(G.grid, early);
         for (bool upper : {false, true}) {
-            const void* kern = upper ? reinterpret_cast<const void*>(sptrsv_line_cluster_kernel<T, true>)
-                                     : reinterpret_cast<const void*>(sptrsv_line_cluster_kernel<T, false>);
+            const void* kern = line_kernel_ptr<T>(G.g, true, upper);
             GB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
             if (G.g.cl > 8) GB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
         }
     } else {
         int per_sm = 0;
         for (bool upper : {false, true}) {
-            const void* kern = upper ? reinterpret_cast<const void*>(sptrsv_line_kernel<T, true>)
-                                     : reinterpret_cast<const void*>(sptrsv_line_kernel<T, false>);
+            const void* kern = line_kernel_ptr<T>(G.g, false, upper);
             GB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
             int r = 0;
             GB_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, kern, G.threads, smem));
             if (r < 1) return false;
             per_sm = per_sm == 0 ? r : std::min(per_sm, r);
         }
-        G.grid = std::min(G.g.nblk, per_sm * dev.sms);
+        G.grid = std::min({G.g.nblk, per_sm * dev.sms, early});
     }
-    const size_t len = static_cast<size_t>(G.g.slots()) * 4;
-    if constexpr (sizeof(T) == 8) {
-        G.l64.reserve(len);
-        G.u64.reserve(len);
-    } else {
-        G.l32.reserve(len);
-        G.u32.reserve(len);
+    const size_t slots = static_cast<size_t>(G.g.slots());
+    G.l.reserve(slots / 32 * line_step_values<T, false>());
+    G.u.reserve(slots / 32 * line_step_values<T, true>());
+    if (sizeof(T) == 8) {
+        G.lo.reserve(slots);
+        G.div.reserve(slots);
     }
     return true;
 }
 
 // Packs the factor values into the operand streams of type T.
 template <class T>
-static void pack_line(LinePack& G, const int* rp, const int* diag, const double* lu, cudaStream_t s, int sms) {
+static void pack_line(LinePack<T>& G, const int* rp, const int* diag, const double* lu, cudaStream_t s, int sms) {
     const long long slots = G.g.slots();
     const int threads = 256;
     const int grid = static_cast<int>(std::max<long long>(1, std::min<long long>(ceil_div<long long>(slots, threads), 8LL * sms)));
-    T* l = sizeof(T) == 8 ? reinterpret_cast<T*>(G.l64.get()) : reinterpret_cast<T*>(G.l32.get());
-    T* u = sizeof(T) == 8 ? reinterpret_cast<T*>(G.u64.get()) : reinterpret_cast<T*>(G.u32.get());
-    line_pack_kernel<T, false><<<grid, threads, 0, s>>>(G.g, rp, diag, lu, l);
-    line_pack_kernel<T, true><<<grid, threads, 0, s>>>(G.g, rp, diag, lu, u);
+    line_pack_kernel<T, false><<<grid, threads, 0, s>>>(G.g, rp, diag, lu, G.l.get(), nullptr, nullptr);
+    line_pack_kernel<T, true><<<grid, threads, 0, s>>>(G.g, rp, diag, lu, G.u.get(), G.lo.get(), G.div.get());
     GB_CUDA_CHECK(cudaGetLastError());
 }
 
+// `set`: the exchange buffer (LinePack).
 template <class T, bool UPPER>
-static void launch_line(const LinePack& G, cudaStream_t s, T* in, const double* scale, T* out, unsigned* counter,
-                        int* status, const int* gate, int step) {
-    const size_t smem = std::max(static_cast<size_t>(line_smem_bytes<T>(G.g)), static_cast<size_t>(G.smem_floor));
+static void launch_line(const LinePack<T>& G, int set, cudaStream_t s, T* in, const double* scale, T* out,
+                        unsigned* counter, int* status, const int* gate, int step) {
+    const size_t smem = std::max(static_cast<size_t>(line_smem_bytes<T, UPPER>(G.g)), static_cast<size_t>(G.smem_floor));
+    const auto kern = line_kernel<T, UPPER>(G.g, G.g.cl > 0);
     if (G.g.cl > 0) {
         cudaLaunchAttribute attr[1];
         cudaLaunchConfig_t cfg = line_cluster_config(G.grid, G.threads, smem, G.g.cl, s, attr);
-        GB_CUDA_CHECK(cudaLaunchKernelEx(&cfg, sptrsv_line_cluster_kernel<T, UPPER>, G.view<T>(UPPER), in, scale, out,
-                                         counter, status, gate, step));
+        GB_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, G.view(UPPER, set), in, scale, out, counter, status, gate, step));
     } else {
-        sptrsv_line_kernel<T, UPPER><<<G.grid, G.threads, smem, s>>>(G.view<T>(UPPER), in, scale, out, counter,
-                                                                      status, gate, step);
+        kern<<<G.grid, G.threads, smem, s>>>(G.view(UPPER, set), in, scale, out, counter, status, gate, step);
     }
     GB_CUDA_CHECK(cudaGetLastError());
 }
@@ -1054,6 +1085,44 @@ static void tune_line(IluSolver::Impl& im, cudaStream_t s) {
     im.check_status(s);
 }
 
+// Sets up the line-pipeline sweeps of value type T for a grid: geometry, kernels, exchange
+// buffers, timelines.  False when a CTA of one warp cannot be resident.
+template <class T>
+static bool setup_line(IluSolver::Impl& im, LinePack<T>& G, int nx, int ny, int nz, cudaStream_t s) {
+    // the requested (or automatic) CTA shape, halved along its longer side until its
+    // shared memory fits
+    int by = im.grid_by, bz = im.grid_bz;
+    bool ok = false;
+    for (int attempt = 0; attempt < 8; ++attempt) {
+        G.g = line_geometry(nx, ny, nz, im.grid_wy, by, bz, im.sweep_timeline ? 8 : static_cast<int>(sizeof(T)));
+        G.threads = G.g.threads();
+        // one CTA per SM on request: more than half of an SM's shared memory
+        G.smem_floor = im.grid_one_cta_per_sm ? std::min(im.dev.smem_per_sm / 2 + 1024, im.dev.smem_optin - 1024) : 0;
+        ok = configure_line<T>(G, im.dev, im.grid_cluster);
+        if (ok || G.g.nw() == 1) break;
+        by = G.g.by;
+        bz = G.g.bz;
+        (bz >= by ? bz : by) = std::max(1, (bz >= by ? bz : by) / 2);
+    }
+    for (int u = 0; u < 2; ++u) {
+        G.tl[u].release();
+        if (im.sweep_timeline && ok) {
+            const size_t len = static_cast<size_t>(G.g.nblk) * kLineTimeline;
+            G.tl[u].reserve(len);
+            GB_CUDA_CHECK(cudaMemsetAsync(G.tl[u].get(), 0, len * sizeof(unsigned long long), s));
+        }
+    }
+    if (!ok) return false;
+    const std::vector<int> order = line_block_order(G.g);
+    G.order.upload(order.data(), order.size(), s);
+    for (int set = 0; set < (sizeof(T) == 8 ? 2 : 1); ++set) {
+        G.xch[set].reserve(static_cast<size_t>(G.g.nblk * G.g.xch_block()));
+        fill_sentinel(G.xch[set].get(), static_cast<long long>(G.xch[set].size()), s, im.dev.sms);
+    }
+    GB_CUDA_CHECK(cudaStreamSynchronize(s));  // `order` must outlive the copy
+    return true;
+}
+
 IluSolver::Impl::~Impl() {
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
@@ -1067,7 +1136,7 @@ void IluSolver::Impl::launch_lower(cudaStream_t s, T* b, const double* scale, T*
         return;
     }
     if ((sizeof(T) == 8 ? line_use64 : line_use32) & 1) {
-        launch_line<T, false>(GP, s, b, scale, y, counters.get() + 1, status.get(), gate, step);
+        launch_line<T, false>(line_pack<T>(), 0, s, b, scale, y, counters.get() + 1, status.get(), gate, step);
         return;
     }
     if (sizeof(T) == 8 ? blk64 : blk32) {
@@ -1086,7 +1155,7 @@ void IluSolver::Impl::launch_upper(cudaStream_t s, T* y, T* x, const int* gate, 
         return;
     }
     if ((sizeof(T) == 8 ? line_use64 : line_use32) & 2) {
-        launch_line<T, true>(GP, s, y, nullptr, x, counters.get() + 2, status.get(), gate, step);
+        launch_line<T, true>(line_pack<T>(), 0, s, y, nullptr, x, counters.get() + 2, status.get(), gate, step);
         return;
     }
     if (sizeof(T) == 8 ? blk64 : blk32) {
@@ -1102,7 +1171,7 @@ template <class T>
 const void* IluSolver::Impl::subst_key() const {
     if (levelsync) return LS.cols.get();
     if (const int bits = sizeof(T) == 8 ? line_use64 : line_use32; bits != 0)  // the schedule is part of the key
-        return (sizeof(T) == 8 ? reinterpret_cast<const char*>(GP.l64.get()) : reinterpret_cast<const char*>(GP.l32.get())) + bits;
+        return reinterpret_cast<const char*>(line_pack<T>().l.get()) + bits;
     if (sizeof(T) == 8 ? blk64 : blk32) return (sizeof(T) == 8 ? LB64 : LB32).codes.get();
     return L.cols.get();
 }
@@ -1130,8 +1199,15 @@ void IluSolver::Impl::check_status(cudaStream_t s) {
         GB_CUDA_CHECK(cudaMemcpy(status.get() + kStatusTimeout, &zero, sizeof(int), cudaMemcpyHostToDevice));
         // a kernel that gave up may leave its ticket counters or grid-barrier words set
         GB_CUDA_CHECK(cudaMemset(counters.get(), 0, sizeof(unsigned) * 8));
+        reset_exchange(s);
+        GB_CUDA_CHECK(cudaStreamSynchronize(s));
         throw std::runtime_error("dependency wait timed out on the device");
     }
+}
+
+void IluSolver::Impl::reset_exchange(cudaStream_t s) {
+    for (auto& x : GP64.xch) fill_sentinel(x.get(), static_cast<long long>(x.size()), s, dev.sms);
+    for (auto& x : GP32.xch) fill_sentinel(x.get(), static_cast<long long>(x.size()), s, dev.sms);
 }
 
 IluSolver::Impl* IluSolver::impl_ensure() {
@@ -1220,36 +1296,10 @@ void IluSolver::SetupMatrix() {
     if (im.grid_mode == 1 || (im.grid_mode == 0 && im.block_rows == 0)) {
         int gx = 0, gy = 0, gz = 0;
         if (detect_grid(n, rp, ci, im.an.diag, gx, gy, gz)) {
-            // the requested (or automatic) CTA shape, halved along its longer side until
-            // the FP64 kernels' shared memory fits
-            int by = im.grid_by, bz = im.grid_bz;
-            for (int attempt = 0; attempt < 8; ++attempt) {
-                im.GP.g = line_geometry(gx, gy, gz, im.grid_wy, by, bz);
-                im.GP.threads = (im.GP.g.nw() + 1) * kWarp;  // compute warps + the halo warp
-                // one CTA per SM on request: more than half of an SM's shared memory
-                im.GP.smem_floor = im.grid_one_cta_per_sm
-                                       ? std::min(im.dev.smem_per_sm / 2 + 1024, im.dev.smem_optin - 1024)
-                                       : 0;
-                im.grid64 = configure_line<double>(im.GP, im.dev, true, im.grid_cluster);
-                if (im.grid64 || im.GP.g.nw() == 1) break;
-                by = im.GP.g.by;
-                bz = im.GP.g.bz;
-                (bz >= by ? bz : by) = std::max(1, (bz >= by ? bz : by) / 2);
-            }
-            im.grid32 = configure_line<float>(im.GP, im.dev, false, 0);
-            for (int f = 0; f < 2; ++f)
-                for (int u = 0; u < 2; ++u) {
-                    auto& buf = im.GP.tl[f][u];
-                    buf.release();
-                    if (im.sweep_timeline && (f == 0 ? im.grid64 : im.grid32)) {
-                        const size_t len = static_cast<size_t>(im.GP.g.nblk) * kLineTimeline;
-                        buf.reserve(len);
-                        GB_CUDA_CHECK(cudaMemsetAsync(buf.get(), 0, len * sizeof(unsigned long long), s));
-                    }
-                }
-            const std::vector<int> order = line_block_order(im.GP.g);
-            im.GP.order.upload(order.data(), order.size(), s);
-            GB_CUDA_CHECK(cudaStreamSynchronize(s));  // `order` must outlive the copy
+            im.grid64 = setup_line(im, im.GP64, gx, gy, gz, s);
+            // (one geometry for both types while timelines are recorded, so that one
+            // LLJBASH_IluInfo describes them)
+            im.grid32 = setup_line(im, im.GP32, gx, gy, gz, s);
         }
     }
     // forced (grid_mode 1): every sweep of a configured type; automatic: timed against the
@@ -1555,11 +1605,11 @@ bool IluSolver::FactorizeFrom(const double* values, bool on_device) {
                 im.launches += 6;
             }
             if (im.grid64) {
-                pack_line<double>(im.GP, im.rp.get(), im.diag.get(), im.lu.get(), s, im.dev.sms);
+                pack_line<double>(im.GP64, im.rp.get(), im.diag.get(), im.lu.get(), s, im.dev.sms);
                 im.launches += 2;
             }
             if (im.grid32) {
-                pack_line<float>(im.GP, im.rp.get(), im.diag.get(), im.lu.get(), s, im.dev.sms);
+                pack_line<float>(im.GP32, im.rp.get(), im.diag.get(), im.lu.get(), s, im.dev.sms);
                 im.launches += 2;
             }
         }
@@ -1713,14 +1763,14 @@ void IluSolver::SubstituteDeviceNoAlloc(const double* d_b, double* d_x) {
     // each sweep on the schedule the solver uses for it (line-pipeline, block-local or
     // level-ordered; a level-synchronous solver's level packs give the same results)
     if (im.line_use64 & 1)
-        launch_line<double, false>(im.GP, s, b, nullptr, y, counters + 1, status, nullptr, 0);
+        launch_line<double, false>(im.GP64, 1, s, b, nullptr, y, counters + 1, status, nullptr, 0);
     else if (im.blk64)
         launch_block<double, false>(im.LB64, s, b, nullptr, y, counters + 1, status, nullptr, 0);
     else if (im.L.ntask > 0)
         launch_level_lower<double>(im.L, im.grid_solve, im.solve_threads, s, b, nullptr, y, counters + 1, status,
                                    nullptr, 0);
     if (im.line_use64 & 2)
-        launch_line<double, true>(im.GP, s, y, nullptr, d_x, counters + 2, status, nullptr, 0);
+        launch_line<double, true>(im.GP64, 1, s, y, nullptr, d_x, counters + 2, status, nullptr, 0);
     else if (im.blk64)
         launch_block<double, true>(im.UB64, s, y, nullptr, d_x, counters + 2, status, nullptr, 0);
     else if (im.U.ntask > 0)
@@ -1729,7 +1779,11 @@ void IluSolver::SubstituteDeviceNoAlloc(const double* d_b, double* d_x) {
     int h[kStatusWords];
     GB_CUDA_CHECK(cudaMemcpyAsync(h, status, sizeof(h), cudaMemcpyDeviceToHost, s));
     GB_CUDA_CHECK(cudaStreamSynchronize(s));
-    if (h[kStatusTimeout] != 0) throw std::runtime_error("dependency wait timed out on the device");
+    if (h[kStatusTimeout] != 0) {
+        im.reset_exchange(s);
+        GB_CUDA_CHECK(cudaStreamSynchronize(s));
+        throw std::runtime_error("dependency wait timed out on the device");
+    }
 }
 
 }  // namespace lljbash

@@ -13,18 +13,25 @@
 // * a warp holds wy x wz lines (lane = zz wy + yy) and lane (yy, zz) works on
 //   x' = s - (yy + zz) at step s: its y- and z-predecessors at the same x' were computed
 //   by lanes (yy - 1, zz) and (yy, zz - 1) one step earlier and arrive by warp shuffles;
-// * a CTA holds by x bz warps; a warp's first lanes along y / z take their predecessors
-//   from the previous warp's face in shared memory ([nx][wz] / [nx][wy] values per
-//   warp, written once per block, value-as-flag: reset to the sentinel with the block);
-// * a block's first warps take them from the previous block through `out` in L2,
-//   loaded PF steps ahead and polled only while they still hold the sentinel.
+// * a CTA holds by x bz compute warps; a warp's first lanes along y / z take their
+//   predecessors from a face in shared memory that the previous warp of the CTA fills
+//   ([x][wz] / [x][wy] values per warp, value-as-flag: reset to the sentinel per block);
+// * faces of a block's first warps are filled by the previous block: through distributed
+//   shared memory inside a thread-block cluster, else through an exchange buffer in L2 of
+//   the same layout that a halo warp polls and hands back at the sentinel.
 //
-// The per-step work of a lane is one row: three FMAs (z, y, x terms in the reference's
-// order) and, for U, the division by u_ii (FP64) or the product with the rounded
-// reciprocal (FP32, as the other FP32 kernels).  The operands of each step (coefficients
-// in a packed stream per warp, right-hand side) are loaded PF steps before use.  The
-// critical path is nx + ny + nz steps plus the handoffs between warps and blocks,
-// against one level per step for the level-set kernels.
+// What bounds it: the chain of nx + ny + nz steps.  The vectors lie in natural order, so a
+// lane's own accesses would touch 32 cache lines per warp and step; they were 64 of the ~70
+// L1 wavefronts of a step, and with four warps per SM they set its pace (176 ns per FP32
+// step).  So each compute warp has a helper warp on its scheduler that moves the operands and
+// the results in chunks of 8 steps through shared memory: the coefficient stream by bulk
+// copies, right-hand side and results 8 consecutive rows of a line at a time (the first
+// product with `scale` included).  The compute warp touches only staged values, its faces
+// and the shuffles, a step is 70 ns (FP32) or 160 / 235 ns (FP64 forward / backward, whose
+// FP64 instructions alone take 93 / 155 ns on a scheduler), and a handoff between warps costs
+// two to three steps.  Inside GMRES, forward / backward, us: 128^3 FP32 88 / 83 (151 / 137
+// with a lane's own accesses), FP64 128 / 177 (247 / 622, block-local backward 566); 256^2
+// FP32 43 / 39 (95 / 84), FP64 72 / 121 (204 / block-local 447).
 //
 // Blocks are taken from a ticket counter in dependency order (anti-diagonals of the block
 // grid), so a block only waits for blocks of smaller tickets, whose CTAs are running or
@@ -41,23 +48,44 @@
 
 namespace gb300 {
 
-constexpr int kLineMaxWarps = 8;  // compute warps per CTA of the line kernels (plus one halo warp)
+constexpr int kLineMaxWarps = 4;  // compute warps per CTA of the line kernels, one per scheduler (each with
+                                  // a helper warp)
+// Steps staged at a time per compute warp (between its synchronisations with its helper),
+// and chunks in flight (two were 15 - 25 % slower, four no faster).
+constexpr int kLineChunk = 8;
+constexpr int kLineSlots = 3;
+// Staged right-hand side and results: per lane a chunk's steps (16-byte accesses by the
+// compute warps) and 16 bytes more, which spread the lanes over the banks.
+template <class T>
+constexpr int kLinePitch = kLineChunk + 16 / static_cast<int>(sizeof(T));
+constexpr int kLineStepAlign = 8;  // steps of a warp are rounded up to a multiple of this
 
 struct LineGeom {
     int nx = 0, ny = 0, nz = 0;
     int wy = 1, wz = 32;  // lanes of a warp along y / z (wy * wz == 32)
     int by = 1, bz = 1;   // warps of a CTA along y / z
     int nby = 1, nbz = 1; // blocks along y / z
-    int steps = 0;        // steps of a warp: nx + wy + wz - 2
+    int steps = 0;        // steps of a warp: nx + wy + wz - 2 ...
+    int psteps = 0;       // ... rounded up to a multiple of kLineStepAlign
     int nblk = 0;         // nby * nbz
     int cl = 0;           // CTAs per thread-block cluster (consecutive blocks along z), 0: none
     int nbzc = 0;         // clusters along z: ceil(nbz / cl)
     __host__ __device__ int nw() const { return by * bz; }
+    __host__ __device__ int halo_warps() const { return ny > 1 ? 2 : 1; }
+    __host__ __device__ int threads() const { return (2 * nw() + halo_warps()) * 32; }
     // Slot of lane `lane` of warp w of block b at step s in the packed operand stream.
     __host__ __device__ long long slot(int b, int w, int s, int lane) const {
-        return ((static_cast<long long>(b) * nw() + w) * steps + s) * 32 + lane;
+        return ((static_cast<long long>(b) * nw() + w) * psteps + s) * 32 + lane;
     }
-    __host__ __device__ long long slots() const { return static_cast<long long>(nblk) * nw() * steps * 32; }
+    __host__ __device__ long long slots() const { return static_cast<long long>(nblk) * nw() * psteps * 32; }
+    // Positions of a face: x' = -pad .. psteps (a lane's x' runs from -(wy + wz - 2) to
+    // psteps - 1, faces are read one step ahead).  Only x' in [0, nx) is ever waited for.
+    __host__ __device__ int pad() const { return wy + wz - 2; }
+    __host__ __device__ int face_len() const { return psteps + pad() + 1; }
+    __host__ __device__ int face_y() const { return ny > 1 ? face_len() * wz : 0; }  // values of one y-face
+    __host__ __device__ int face_z() const { return face_len() * wy; }
+    // Exchange buffer of a block: its first warps' faces, y then z.
+    __host__ __device__ long long xch_block() const { return static_cast<long long>(bz) * face_y() + by * face_z(); }
 };
 
 template <class T>
@@ -65,7 +93,13 @@ struct LineTri {
     LineGeom g;
     const int* order = nullptr;  // [nblk] block (iy + nby iz, sweep coordinates) of each ticket;
                                  // with clusters [nby nbzc]: cluster (iy + nby izc) of each ticket
-    const T* coef = nullptr;     // [slots][4]: c_z, c_y, c_x, d (d: u_ii FP64 / RN(1 / u_ii) FP32; L: unused)
+    const T* coef = nullptr;     // per slot c_z, c_y, c_x, and for U the reciprocal of u_ii
+                                 // (FP32: RN(1 / u_ii); FP64: its high part, see line_quotient),
+                                 // in the order of line_coef_at
+    const T* rlo = nullptr;      // FP64 U: [slots] low part of the reciprocal
+    const T* div = nullptr;      // FP64 U: [slots] u_ii
+    T* xch = nullptr;            // [nblk][xch_block()] faces handed over through L2, at the sentinel
+                                 // between launches (in x' in [0, nx))
     unsigned long long* tl = nullptr;  // per-block timeline [nblk][kLineTimeline] (null: off)
 };
 
@@ -88,445 +122,642 @@ __device__ __forceinline__ void line_stamp_start(const LineTri<T>& P, int blk) {
     }
 }
 template <class T>
-__device__ __forceinline__ void line_stamp_end(const LineTri<T>& P, int blk) {
+__device__ __forceinline__ void line_stamp_end(const LineTri<T>& P, int blk, int entry) {
     if (P.tl != nullptr && (threadIdx.x & 31) == 0)
-        P.tl[static_cast<long long>(blk) * kLineTimeline + 2 + (threadIdx.x >> 5)] = global_ns();
+        P.tl[static_cast<long long>(blk) * kLineTimeline + entry] = global_ns();
 }
 
-// ---- asynchronous global -> shared copies (cp.async, per thread) ----
-// src_bytes = 0 fills the destination with zeros without reading the source.
-__device__ __forceinline__ void cp_async_16(void* smem, const void* gmem, int src_bytes) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(static_cast<unsigned>(__cvta_generic_to_shared(smem))),
-                 "l"(gmem), "r"(src_bytes));
+// Shared memory by its 32-bit address.
+__device__ __forceinline__ unsigned shared_addr(const void* p) { return static_cast<unsigned>(__cvta_generic_to_shared(p)); }
+__device__ __forceinline__ void lds(unsigned a, float& v) { asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a)); }
+__device__ __forceinline__ void lds(unsigned a, double& v) { asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(a)); }
+__device__ __forceinline__ void lds_polled(unsigned a, float& v) {
+    asm volatile("ld.volatile.shared.f32 %0, [%1];" : "=f"(v) : "r"(a));
 }
-__device__ __forceinline__ void cp_async_8(void* smem, const void* gmem, int src_bytes) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(static_cast<unsigned>(__cvta_generic_to_shared(smem))),
-                 "l"(gmem), "r"(src_bytes));
+__device__ __forceinline__ void lds_polled(unsigned a, double& v) {
+    asm volatile("ld.volatile.shared.f64 %0, [%1];" : "=d"(v) : "r"(a));
 }
-__device__ __forceinline__ void cp_async_4(void* smem, const void* gmem, int src_bytes) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(static_cast<unsigned>(__cvta_generic_to_shared(smem))),
-                 "l"(gmem), "r"(src_bytes));
+__device__ __forceinline__ void lds16(unsigned a, float (&v)[4]) {
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "r"(a));
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+__device__ __forceinline__ void lds16(unsigned a, double (&v)[2]) {
+    asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(v[0]), "=d"(v[1]) : "r"(a));
 }
-
-// Stores issued only where `on` holds, as predicated instructions (no branch).
-__device__ __forceinline__ void st_relaxed_if(bool on, double* p, double v) {
-    asm volatile("{ .reg .pred q; setp.ne.u32 q, %0, 0; @q st.relaxed.gpu.global.f64 [%1], %2; }" ::"r"(static_cast<unsigned>(on)),
-                 "l"(p), "d"(v));
+__device__ __forceinline__ void sts16(unsigned a, const float (&v)[4]) {
+    asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(a), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]));
 }
-__device__ __forceinline__ void st_relaxed_if(bool on, float* p, float v) {
-    asm volatile("{ .reg .pred q; setp.ne.u32 q, %0, 0; @q st.relaxed.gpu.global.f32 [%1], %2; }" ::"r"(static_cast<unsigned>(on)),
-                 "l"(p), "f"(v));
+__device__ __forceinline__ void sts16(unsigned a, const double (&v)[2]) {
+    asm volatile("st.shared.v2.f64 [%0], {%1, %2};" ::"r"(a), "d"(v[0]), "d"(v[1]));
 }
-__device__ __forceinline__ void st_global_if(bool on, double* p, double v) {
-    asm volatile("{ .reg .pred q; setp.ne.u32 q, %0, 0; @q st.global.f64 [%1], %2; }" ::"r"(static_cast<unsigned>(on)), "l"(p),
-                 "d"(v));
+// Relaxed store through a generic address: the next warp's face (this CTA's shared
+// memory), the next CTA's (distributed shared memory) or an exchange buffer (global).
+__device__ __forceinline__ void st_relaxed_generic(bool on, double* p, double v) {
+    asm volatile("{ .reg .pred q; setp.ne.u32 q, %0, 0; @q st.relaxed.gpu.f64 [%1], %2; }" ::"r"(static_cast<unsigned>(on)), "l"(p), "d"(v));
 }
-__device__ __forceinline__ void st_global_if(bool on, float* p, float v) {
-    asm volatile("{ .reg .pred q; setp.ne.u32 q, %0, 0; @q st.global.f32 [%1], %2; }" ::"r"(static_cast<unsigned>(on)), "l"(p),
-                 "f"(v));
+__device__ __forceinline__ void st_relaxed_generic(bool on, float* p, float v) {
+    asm volatile("{ .reg .pred q; setp.ne.u32 q, %0, 0; @q st.relaxed.gpu.f32 [%1], %2; }" ::"r"(static_cast<unsigned>(on)), "l"(p), "f"(v));
 }
-__device__ __forceinline__ void st_shared_if(bool on, double* p, double v) {
-    asm volatile("{ .reg .pred q; setp.ne.u32 q, %0, 0; @q st.volatile.shared.f64 [%1], %2; }" ::"r"(static_cast<unsigned>(on)),
-                 "r"(static_cast<unsigned>(__cvta_generic_to_shared(p))), "d"(v));
-}
-__device__ __forceinline__ void st_shared_if(bool on, float* p, float v) {
-    asm volatile("{ .reg .pred q; setp.ne.u32 q, %0, 0; @q st.volatile.shared.f32 [%1], %2; }" ::"r"(static_cast<unsigned>(on)),
-                 "r"(static_cast<unsigned>(__cvta_generic_to_shared(p))), "f"(v));
-}
-
-__device__ __forceinline__ void st_cluster_if(bool on, unsigned addr, double v) {
-    asm volatile("{ .reg .pred q; setp.ne.u32 q, %0, 0; @q st.relaxed.cluster.shared::cluster.f64 [%1], %2; }" ::"r"(
-                     static_cast<unsigned>(on)),
-                 "r"(addr), "d"(v));
-}
-__device__ __forceinline__ void st_cluster_if(bool on, unsigned addr, float v) {
-    asm volatile("{ .reg .pred q; setp.ne.u32 q, %0, 0; @q st.relaxed.cluster.shared::cluster.f32 [%1], %2; }" ::"r"(
-                     static_cast<unsigned>(on)),
-                 "r"(addr), "f"(v));
-}
-
-// Waits (bounded) until the shared-memory value *p is no longer the sentinel; after many
-// polls it sleeps between polls (a warp waiting for a block far behind).
+// Generic address of `p` (this CTA's shared memory) in cluster CTA `rank`.
 template <class T>
-__device__ __noinline__ T line_wait_shared(const T* p, int* status) {
-    T v = ld_volatile_shared(p);
+__device__ __forceinline__ T* map_generic_rank(T* p, unsigned rank) {
+    unsigned long long r;
+    asm volatile("mapa.u64 %0, %1, %2;" : "=l"(r) : "l"(p), "r"(rank));
+    return reinterpret_cast<T*>(r);
+}
+
+// mbarriers between a compute warp and its helper (arrivals by lane 0 after a warp barrier).  Their arrivals release the warp's shared-memory writes without waiting for
+// its global loads and stores in flight; a st.release flag did wait for them, which cost
+// the compute warps a memory round trip per chunk.
+__device__ __forceinline__ void mbar_init(unsigned long long* b, unsigned count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(static_cast<unsigned>(__cvta_generic_to_shared(b))), "r"(count)
+                 : "memory");
+}
+__device__ __forceinline__ void mbar_inval(unsigned long long* b) {
+    asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(static_cast<unsigned>(__cvta_generic_to_shared(b))) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(unsigned long long* b) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(static_cast<unsigned>(__cvta_generic_to_shared(b))) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive_expect(unsigned long long* b, unsigned bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(
+                     static_cast<unsigned>(__cvta_generic_to_shared(b))),
+                 "r"(bytes)
+                 : "memory");
+}
+// Bulk copy of `bytes` (a multiple of 16, both addresses 16-byte aligned) into this CTA's
+// shared memory, completed on the mbarrier `b`.
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, unsigned bytes, unsigned long long* b) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                     static_cast<unsigned>(__cvta_generic_to_shared(dst))),
+                 "l"(src), "r"(bytes), "r"(static_cast<unsigned>(__cvta_generic_to_shared(b)))
+                 : "memory");
+}
+// (test_wait, not try_wait: a warp that try_wait had suspended for about 100 us took 5 us
+// to come back)
+__device__ __forceinline__ bool mbar_test(unsigned long long* b, unsigned parity) {
+    unsigned ok;
+    asm volatile("{ .reg .pred p; mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+                 : "=r"(ok)
+                 : "r"(static_cast<unsigned>(__cvta_generic_to_shared(b))), "r"(parity)
+                 : "memory");
+    return ok != 0u;
+}
+// Waits (bounded) for the completion of the barrier's phase of this parity; false when the
+// wait gave up.  The clock is read as rarely as in line_wait_shared.
+static __device__ __noinline__ bool mbar_wait_long(unsigned long long* b, unsigned parity, int* status) {
     WaitBudget wb;
-    int polls = 0;
-    while (Sentinel<T>::is(v)) {
+    for (;;) {
+        for (int polls = 0; polls < 2048; ++polls)
+            if (mbar_test(b, parity)) return true;
+        wb.polls |= 1023;  // so that expired() looks at the clock and at the status word
+        if (wb.expired(status)) {
+            atomicExch(status + kStatusTimeout, 1);
+            return false;
+        }
+    }
+}
+__device__ __forceinline__ bool mbar_wait(unsigned long long* b, unsigned parity, int* status) {
+    return mbar_test(b, parity) || mbar_wait_long(b, parity, status);
+}
+
+// A value that may be stored where others poll for the sentinel: the sentinel's own bit
+// pattern (a NaN) becomes the canonical NaN.  Integer compares: an FP64 compare would
+// take 64 cycles of GB300's FP64 pipe in every step.
+__device__ __forceinline__ float off_sentinel(float v) {
+    return __float_as_uint(v) == 0xFFFFFFFFu ? __uint_as_float(0x7FC00000u) : v;
+}
+__device__ __forceinline__ double off_sentinel(double v) {
+    return __double2hiint(v) == -1 ? __longlong_as_double(0x7FF8000000000000ll) : v;
+}
+
+// Waits (bounded) until the value at the shared address `a` is no longer the sentinel.
+// The clock is read rarely, and not before kLinePollsFree polls (about 40 us): a read
+// takes as long as several steps, and a warp never makes up for a delay, because its
+// predecessor runs at the same pace (with a read every 64 polls each handoff between two
+// warps cost 40 steps instead of 8).  After many polls it sleeps between polls (a block
+// far behind).
+constexpr int kLinePollsFree = 2048;
+template <class T>
+__device__ __noinline__ T line_wait_shared(unsigned a, int* status) {
+    T v;
+    for (int polls = 0; polls < kLinePollsFree; ++polls) {
+        lds_polled(a, v);
+        if (!Sentinel<T>::is(v)) return v;
+    }
+    WaitBudget wb;
+    for (;;) {
+        for (int polls = 0; polls < 1024; ++polls) {
+            lds_polled(a, v);
+            if (!Sentinel<T>::is(v)) return v;
+        }
+        wb.polls |= 1023;  // so that expired() looks at the clock and at the status word
         if (wb.expired(status)) {
             atomicExch(status + kStatusTimeout, 1);
             return T(0);
         }
-        if (++polls > 4096) __nanosleep(256);  // a long wait (a block far behind)
-        v = ld_volatile_shared(p);
     }
-    return v;
 }
 
-// Coefficients of one row in the packed stream (c_z, c_y, c_x, d).
+// ---- FP64 division by a known divisor ----
+// acc / d for the rows of U: GB300 issues one FP64 instruction per warp in 64 cycles on a
+// scheduler, and a division takes about nine of them (566 cycles measured), all on the
+// chain.  With 1/d = hi + lo (hi = 1/d rounded towards zero, lo the remainder, both from
+// the factorisation's packing) the quotient is fma(acc, hi, acc * lo): two instructions
+// (128 cycles), its argument within 2^-51 ulp of the exact quotient, so it is the
+// correctly rounded quotient unless that lies within 2^-51 ulp of the middle between two
+// numbers (double-word reciprocal, as in the literature on division by constants:
+// Brisebarre, Muller, Raina, "Accelerating correctly rounded floating-point division when
+// the divisor is known in advance", IEEE TC 53(8), 2004).  hi and lo have the same sign,
+// so a zero keeps its sign.  Divisors outside 2^+-400 are packed as hi = NaN, and a
+// quotient outside 2^+-600 (or one that is not finite) is divided again.
+constexpr int kLineDivExp = 400;
+constexpr int kLineQuoExp = 600;
+
+__device__ __forceinline__ void line_reciprocal(double d, double& hi, double& lo) {
+    const int e = (__double2hiint(d) >> 20) & 0x7FF;
+    if (e < 1023 - kLineDivExp || e > 1023 + kLineDivExp) {
+        hi = __longlong_as_double(0x7FF8000000000000ll);
+        lo = 0.0;
+        return;
+    }
+    hi = __drcp_rz(d);
+    lo = fma(-d, hi, 1.0) * hi;  // 1 - d hi is exact: both factors have 53 bits, the result < 2^-52
+}
+__device__ __forceinline__ double line_quotient(double acc, double hi, double lo) { return fma(acc, hi, acc * lo); }
+// Whether acc / d must be divided again (integer operations: the FP64 pipe is what the
+// sweep waits for).  0 / d is exact already.
+__device__ __forceinline__ bool line_quotient_bad(float, float) { return false; }
+__device__ __forceinline__ bool line_quotient_bad(double q, double acc) {
+    const unsigned qh = static_cast<unsigned>(__double2hiint(q)), ah = static_cast<unsigned>(__double2hiint(acc));
+    constexpr unsigned kLow = static_cast<unsigned>(1023 - kLineQuoExp) << 21;  // exponent above the sign
+    constexpr unsigned kSpan = static_cast<unsigned>(2 * kLineQuoExp) << 21;
+    const unsigned nonzero = ((qh | ah) << 1) | static_cast<unsigned>(__double2loint(q)) | static_cast<unsigned>(__double2loint(acc));
+    return (qh << 1) - kLow > kSpan && nonzero != 0u;
+}
+static __device__ __noinline__ double line_divide(double acc, const double* d) { return acc / *d; }
+
+// Coefficients of one row in the packed stream: c_z, c_y, c_x and for U the reciprocal.  A
+// step's 32 rows lie together: FP32 four values (16 bytes) per lane; FP64 pairs (c_z, c_y)
+// per lane, then for U pairs (c_x, reciprocal), for L c_x alone.
 template <class T>
-struct alignas(4 * sizeof(T)) LineCoef {
+struct LineCoef {
     T cz, cy, cx, d;
 };
-
-// Steps of operands in flight per lane (cp.async ring in shared memory).
-template <class T>
-constexpr int kLineRing = sizeof(T) == 4 ? 16 : 8;
-
-// Shared memory of a CTA: faces (consumer-indexed: slot w holds what warp w reads; faceY
-// [nw][nx][wz] when ny > 1, faceZ [nw][nx][wy]), one word holding 0, then the operand
-// rings [R][nw * 32] of coefficients and of right-hand side values.
-__host__ __device__ inline long long line_face_slot_y(const LineGeom& g) {
-    return g.ny > 1 ? static_cast<long long>(g.nx) * g.wz : 0;
-}
-__host__ __device__ inline long long line_face_slot_z(const LineGeom& g) { return static_cast<long long>(g.nx) * g.wy; }
-template <class T>
-__host__ __device__ inline long long line_face_len(const LineGeom& g) {
-    return static_cast<long long>(g.nw()) * (line_face_slot_y(g) + line_face_slot_z(g));
-}
-template <class T>
-__host__ __device__ inline long long line_ring_offset(const LineGeom& g) {
-    return ((line_face_len<T>(g) + 1) * static_cast<long long>(sizeof(T)) + 15) & ~15ll;
-}
-template <class T>
-__host__ __device__ inline long long line_smem_bytes(const LineGeom& g) {
-    return line_ring_offset<T>(g) +
-           static_cast<long long>(kLineRing<T>) * g.nw() * 32 * (static_cast<long long>(sizeof(LineCoef<T>)) + sizeof(T));
-}
-
-// One compute warp's share of block `blk`: wy x wz lines over nx + wy + wz - 2 steps.
-// faceY / faceZ: slot w holds the y / z predecessors of warp w's first lanes along y / z,
-// written by the previous warp of the CTA or by the halo warp (previous block), or zeros
-// at the grid's boundary.
 template <class T, bool UPPER>
-__device__ __forceinline__ void line_warp(const LineTri<T>& P, int blk, T* in, bool scaled, T sc, T* out, T* faceY,
-                                          T* faceZ, const T* zero_word, LineCoef<T>* cring, T* bring,
-                                          unsigned fz_remote, int* status) {
-    constexpr int R = kLineRing<T>;
-    const int lane = threadIdx.x & 31;
-    const int w = threadIdx.x >> 5;
-    const int nx = P.g.nx, ny = P.g.ny, nz = P.g.nz;
-    const int wy = P.g.wy, wz = P.g.wz, by = P.g.by, bz = P.g.bz;
-    const int nw = by * bz;
-    const int wyi = w % by, wzi = w / by;
-    const int yy = lane % wy, zz = lane / wy;
-    const int iy = blk % P.g.nby, iz = blk / P.g.nby;
-    const int yq = (iy * by + wyi) * wy + yy;  // sweep coordinates of the lane's line
-    const int zq = (iz * bz + wzi) * wz + zz;
-    const bool line_ok = yq < ny && zq < nz;
-    const int skew = yy + zz;
-    const int steps = P.g.steps;
-    const long long plane = static_cast<long long>(nx) * ny;
-    const long long Y = UPPER ? ny - 1 - yq : yq;
-    const long long Z = UPPER ? nz - 1 - zq : zq;
-    const int sx = UPPER ? -1 : 1;
-    T* const in0 = in + ((UPPER ? nx - 1 : 0) + nx * Y + plane * Z);  // natural row of x' = 0
-    T* const out0 = out + ((UPPER ? nx - 1 : 0) + nx * Y + plane * Z);
-    const bool y_edge = ny > 1 && yy == 0;
-    const bool z_edge = zz == 0;
-    const long long fsy = line_face_slot_y(P.g), fsz = line_face_slot_z(P.g);
-    const T* fy = faceY + w * fsy + zz;  // stride wz per x'
-    const T* fz = faceZ + w * fsz + yy;  // stride wy per x'
-    T* const fy_out = (ny > 1 && yy == wy - 1 && wyi < by - 1) ? faceY + (w + 1) * fsy + zz : nullptr;
-    T* const fz_out = (zz == wz - 1 && wzi < bz - 1) ? faceZ + (w + by) * fsz + yy : nullptr;
-    // cluster variant: the last warps along z push into the next CTA of the cluster (its
-    // warp (wyi, 0) slot), fz_remote being that CTA's faceZ in the cluster's shared window
-    const unsigned fz_push = (fz_remote != 0u && zz == wz - 1 && wzi == bz - 1)
-                                 ? fz_remote + static_cast<unsigned>((wyi * fsz + yy) * static_cast<long long>(sizeof(T)))
-                                 : 0u;
-    const LineCoef<T>* const cs = reinterpret_cast<const LineCoef<T>*>(P.coef) + P.g.slot(blk, w, 0, lane);
-    LineCoef<T>* const cr = cring + w * 32 + lane;  // slot k at cr[k * nw * 32]
-    T* const br = bring + w * 32 + lane;
-    const int rs = nw * 32;
+__host__ __device__ constexpr int line_step_values() {
+    return sizeof(T) == 8 && !UPPER ? 96 : 128;
+}
+template <class T, bool UPPER>
+__host__ __device__ constexpr long long line_coef_at(long long slot, int e) {
+    const long long step = (slot / 32) * line_step_values<T, UPPER>();
+    const int lane = static_cast<int>(slot % 32);
+    if (sizeof(T) == 4) return step + lane * 4 + e;
+    if (e < 2) return step + lane * 2 + e;
+    return step + 64 + (UPPER ? lane * 2 + (e - 2) : lane);
+}
+// (a: shared address of the step)
+template <bool UPPER>
+__device__ __forceinline__ void line_load_coef(unsigned a, int lane, LineCoef<float>& c) {
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(c.cz), "=f"(c.cy), "=f"(c.cx), "=f"(c.d) : "r"(a + lane * 16));
+}
+template <bool UPPER>
+__device__ __forceinline__ void line_load_coef(unsigned a, int lane, LineCoef<double>& c) {
+    asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(c.cz), "=d"(c.cy) : "r"(a + lane * 16));
+    if constexpr (UPPER)
+        asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(c.cx), "=d"(c.d) : "r"(a + lane * 16 + 512));
+    else
+        asm volatile("ld.shared.f64 %0, [%1];" : "=d"(c.cx) : "r"(a + lane * 8 + 512));
+}
 
-    // step t's operands into ring slot t % R (zeros where the lane has no row)
-    const unsigned span = line_ok ? static_cast<unsigned>(nx) : 0u;  // active: (unsigned)(t - skew) < span
-    auto issue = [&](int t) {
-        const int xq = t - skew;
-        const bool act = static_cast<unsigned>(xq) < span;
-        const int k = t & (R - 1);
-        const LineCoef<T>* c = act ? cs + static_cast<long long>(t) * 32 : cs;
-        const T* bp = act ? in0 + static_cast<long long>(sx) * xq : in;
-        if constexpr (sizeof(T) == 4) {
-            cp_async_16(cr + k * rs, c, act ? 16 : 0);
-            cp_async_4(br + k * rs, bp, act ? 4 : 0);
-        } else {
-            cp_async_16(cr + k * rs, c, act ? 16 : 0);
-            cp_async_16(reinterpret_cast<char*>(cr + k * rs) + 16, reinterpret_cast<const char*>(c) + 16, act ? 16 : 0);
-            cp_async_8(br + k * rs, bp, act ? 8 : 0);
-        }
-        cp_async_commit();
+// Shared memory of a CTA: per compute warp and slot a chunk of the coefficient stream
+// (and for FP64 of the low reciprocals) and its right-hand side [lane][kLinePitch]; per
+// compute warp a ring of kLineSlots + 1 chunks of results [lane][kLinePitch]; then the faces (consumer-indexed: slot w holds what warp w reads;
+// y-faces [nw][face_y()], z-faces [nw][face_z()]); then kLineIdle zeros that lanes without
+// a face read and kLineIdle values that lanes without a consumer write (so that no access
+// needs a predicate); then per compute warp and slot two mbarriers: [0] the chunk is staged (and the result ring has room for it), [1] the
+// chunk is computed.
+template <class T, bool UPPER>
+struct LineStage {
+    static constexpr int kCoef = kLineChunk * line_step_values<T, UPPER>();
+    static constexpr int kLo = UPPER && sizeof(T) == 8 ? kLineChunk * 32 : 0;
+    static constexpr int kVec = 32 * kLinePitch<T>;
+    static constexpr int kSlot = kCoef + kLo + kVec;  // a multiple of 16 bytes
+    static constexpr int kWarp = kLineSlots * kSlot + (kLineSlots + 1) * kVec;
+};
+constexpr int kLineIdle = kLineStepAlign * 32 + 32;  // offsets within a chunk stay inside
+template <class T, bool UPPER>
+__host__ __device__ inline long long line_bar_offset(const LineGeom& g) {
+    return (((g.nw() * (static_cast<long long>(LineStage<T, UPPER>::kWarp) + g.face_y() + g.face_z()) + 2 * kLineIdle) *
+             static_cast<long long>(sizeof(T))) + 15) & ~15ll;
+}
+template <class T, bool UPPER>
+__host__ __device__ inline long long line_smem_bytes(const LineGeom& g) {
+    return line_bar_offset<T, UPPER>(g) + 2ll * g.nw() * kLineSlots * static_cast<long long>(sizeof(unsigned long long));
+}
+
+template <class T, bool UPPER>
+struct LineSmem {
+    T *stage, *face_y, *face_z, *idle;
+    unsigned long long* bar;
+    __device__ __forceinline__ T* slot(int w, int k) const {
+        return stage + w * LineStage<T, UPPER>::kWarp + (k % kLineSlots) * LineStage<T, UPPER>::kSlot;
+    }
+    __device__ __forceinline__ T* result(int w, int k) const {
+        return stage + w * LineStage<T, UPPER>::kWarp + kLineSlots * LineStage<T, UPPER>::kSlot +
+               (k % (kLineSlots + 1)) * LineStage<T, UPPER>::kVec;
+    }
+    __device__ __forceinline__ unsigned long long* full(int w, int k) const {
+        return bar + w * 2 * kLineSlots + k % kLineSlots;
+    }
+    __device__ __forceinline__ unsigned long long* done(int w, int k) const { return full(w, k) + kLineSlots; }
+    static __device__ __forceinline__ unsigned parity(int k) { return (k / kLineSlots) & 1; }
+};
+template <class T, bool UPPER>
+__device__ __forceinline__ LineSmem<T, UPPER> line_smem_view(const LineGeom& g, unsigned char* base) {
+    LineSmem<T, UPPER> m;
+    m.stage = reinterpret_cast<T*>(base);
+    m.face_y = m.stage + static_cast<long long>(g.nw()) * LineStage<T, UPPER>::kWarp;
+    m.face_z = m.face_y + static_cast<long long>(g.nw()) * g.face_y();
+    m.idle = m.face_z + static_cast<long long>(g.nw()) * g.face_z();
+    m.bar = reinterpret_cast<unsigned long long*>(base + line_bar_offset<T, UPPER>(g));
+    return m;
+}
+
+// Whether a face value has not arrived (lanes without a face hold zeros).
+__device__ __forceinline__ bool line_late(float y, float z) { return max(__float_as_uint(y), __float_as_uint(z)) == 0xFFFFFFFFu; }
+__device__ __forceinline__ bool line_late(double y, double z) {
+    // (only the sentinel has these upper words: published values are off it)
+    return max(static_cast<unsigned>(__double2hiint(y)), static_cast<unsigned>(__double2hiint(z))) == 0xFFFFFFFFu;
+}
+
+// One compute warp's share of block `blk`: wy x wz lines over psteps steps.  Slots without
+// a row hold zero coefficients and a zero right-hand side, so a lane outside its line
+// computes zeros (or, past the line's end, values that nobody reads) and needs no
+// predicate.  to_y / to_z: the face (generic address, this warp's lane pattern) that its
+// last lanes along y / z fill, null: none.
+template <class T, bool UPPER, int WY, bool D3>
+__device__ __forceinline__ void line_compute(const LineTri<T>& P, int blk, int w, const LineSmem<T, UPPER>& M, T* to_y, T* to_z,
+                                             int* status) {
+    constexpr int WZ = 32 / WY;
+    constexpr int PAD = WY + WZ - 2;
+    constexpr int C = kLineChunk;
+    using St = LineStage<T, UPPER>;
+    constexpr bool DIV = UPPER && sizeof(T) == 8;
+    const int lane = threadIdx.x & 31;
+    const int yy = lane % WY, zz = lane / WY;
+    const int shift = PAD - (yy + zz);  // face position of step 0
+    const bool y_edge = D3 && yy == 0;
+    const bool z_edge = zz == 0;
+    const int nchunk = P.g.psteps / C;
+    constexpr unsigned Z = sizeof(T);
+    const unsigned idle = shared_addr(M.idle);
+    const T* div = DIV ? P.div + P.g.slot(blk, w, 0, lane) : nullptr;
+    unsigned fy = y_edge ? shared_addr(M.face_y + static_cast<long long>(w) * P.g.face_y() + shift * WZ + zz) : idle;
+    unsigned fz = z_edge ? shared_addr(M.face_z + static_cast<long long>(w) * P.g.face_z() + shift * WY + yy) : idle;
+    const unsigned fy_adv = y_edge ? C * WZ * Z : 0u, fz_adv = z_edge ? C * WY * Z : 0u;
+    const bool has_y = D3 && to_y != nullptr && yy == WY - 1;
+    const bool has_z = to_z != nullptr && zz == WZ - 1;
+    T* oy = has_y ? to_y + shift * WZ + zz : M.idle + kLineIdle;
+    T* oz = has_z ? to_z + shift * WY + yy : M.idle + kLineIdle;
+    const int oy_adv = has_y ? C * WZ : 0, oz_adv = has_z ? C * WY : 0;
+
+    mbar_wait(M.full(w, 0), 0u, status);
+    __syncwarp();
+    constexpr int V = 16 / sizeof(T);  // steps per access of the right-hand side and the results
+    constexpr unsigned kLo = St::kCoef * Z, kB = kLo + St::kLo * Z, kStep = line_step_values<T, UPPER>() * Z;
+    const unsigned laneZ = lane * Z, laneP = lane * (kLinePitch<T> * Z);
+    unsigned row = shared_addr(M.slot(w, 0));
+    // operands: coefficients loaded two steps ahead, right-hand side by groups of V steps,
+    // faces one step ahead
+    LineCoef<T> c[2];
+    T lo[2] = {T(0), T(0)}, bc[V], bn[V], res[V];
+    T pfy = T(0), pfz;
+    auto load = [&](unsigned slot, int step, int e) {
+        line_load_coef<UPPER>(slot + step * kStep, lane, c[e]);
+        if constexpr (DIV) lds(slot + laneZ + (kLo + step * 32 * Z), lo[e]);
+    };
+    load(row, 0, 0);
+    load(row, 1, 1);
+    lds16(row + laneP + kB, bc);
+    if (D3) lds_polled(fy, pfy);
+    lds_polled(fz, pfz);
+    T prev = T(0), sh_y = T(0), sh_z = T(0);  // the previous step's results: own, y- and z-neighbour
+    auto shuffle = [&](T r, T& y, T& z) {
+        if (D3 && WY > 1) y = __shfl_up_sync(0xffffffffu, r, 1);
+        z = __shfl_up_sync(0xffffffffu, r, WY);
     };
 #pragma unroll 1
-    for (int t = 0; t < R - 1; ++t) issue(t);
-    // face reads: edge lanes at x' (clamped: no read outside the face where the lane has no
-    // row), the other lanes from a word that holds 0; each step's values are loaded one
-    // step ahead, so that the check for a late predecessor is resolved off the chain
-    const T* const fy_rd = y_edge ? fy : zero_word;
-    const T* const fz_rd = z_edge ? fz : zero_word;
-    const int fy_st = y_edge ? wz : 0, fz_st = z_edge ? wy : 0;
-    auto face_at = [&](int t, const T* base, int st) -> const T* {
-        const int xq = t - skew;
-        return base + (static_cast<unsigned>(xq) < span ? xq : 0) * st;
-    };
-    T pfy = ld_volatile_shared(face_at(0, fy_rd, fy_st));
-    T pfz = ld_volatile_shared(face_at(0, fz_rd, fz_st));
-    T* out_p = out0 - static_cast<long long>(sx) * skew;  // row of step s: out_p (advanced by sx per step)
-    T prev = T(0);  // the lane's result of the previous step (used only where it had a row)
-#pragma unroll 2
-    for (int s = 0; s < steps; ++s) {
-        cp_async_wait<R - 2>();  // step s has landed
-        const int k = s & (R - 1);
-        const LineCoef<T> c = cr[k * rs];
-        const T bv = br[k * rs];
-        issue(s + R - 1);  // into the slot read one step ago
-        const int xq = s - skew;
-        const bool act = static_cast<unsigned>(xq) < span;
-        T fyv = pfy, fzv = pfz;
-        pfy = ld_volatile_shared(face_at(s + 1, fy_rd, fy_st));
-        pfz = ld_volatile_shared(face_at(s + 1, fz_rd, fz_st));
-        const bool late = act && (Sentinel<T>::is(fyv) || Sentinel<T>::is(fzv));
-        const T sh_y = __shfl_up_sync(0xffffffffu, prev, 1);
-        const T sh_z = __shfl_up_sync(0xffffffffu, prev, wy);
-        const T xin = xq > 0 ? prev : T(0);
-        const T a0 = scaled ? bv * sc : bv;
-        auto row = [&](T fy_v, T fz_v) -> T {
-            const T vy = y_edge ? fy_v : (ny > 1 ? sh_y : T(0));
-            const T vz = z_edge ? fz_v : sh_z;
-            T acc = fma(-c.cz, vz, a0);
-            acc = fma(-c.cy, vy, acc);
-            acc = fma(-c.cx, xin, acc);
-            // FP64: the reference's division (lanes without a row divide by 1: no slow
-            // path); FP32 (mixed path): d holds 1 / u_ii
-            if constexpr (UPPER) acc = sizeof(T) == 8 ? acc / (act ? c.d : T(1)) : acc * c.d;
-            return acc;
-        };
-        T r = row(fyv, fzv);
-        if (__any_sync(0xffffffffu, late)) {  // a predecessor was not there yet: wait, redo
-            const int xc = act ? xq : 0;
-            if (late && Sentinel<T>::is(fyv)) fyv = line_wait_shared(fy_rd + xc * fy_st, status);
-            if (late && Sentinel<T>::is(fzv)) fzv = line_wait_shared(fz_rd + xc * fz_st, status);
-            r = row(fyv, fzv);
-        }
-        // the next step reads r directly (an active lane's shuffle partners and its own
-        // previous step are active at the same x'); only the stored copies, which other
-        // warps and blocks poll, are kept off the sentinel
-        prev = r;
-        const T rs_ = Sentinel<T>::canon(r);
-        st_relaxed_if(act, out_p, rs_);
-        out_p += sx;
-        const int xc = act ? xq : 0;
-        st_shared_if(act && fy_out != nullptr, fy_out + xc * wz, rs_);
-        st_shared_if(act && fz_out != nullptr, fz_out + xc * wy, rs_);
-        st_cluster_if(act && fz_push != 0u, fz_push + static_cast<unsigned>(xc * wy * static_cast<int>(sizeof(T))), rs_);
-    }
-    cp_async_wait<0>();
-}
-
-// The halo warp of block `blk`: copies the predecessors that the block's first warps
-// along y and z read from the previous blocks (their last lines, in `out`) into the
-// faces.  Lane e owns entry e of the y-face (the block's z-line e, at most 32) and entry
-// e of the z-face (its y-line e, at most 32) and walks each in x' with its own cursor;
-// each round loads the next kLineHalo positions of both (one L2 round trip) and retires,
-// in order, those that no longer hold the sentinel.
-constexpr int kLineHalo = 16;
-
-template <class T>
-struct HaloCursor {
-    const T* src = nullptr;  // natural row of x' = 0 of the source line (null: no entry)
-    T* dst = nullptr;        // face slot of x' = 0
-    int stride = 0;          // face stride per x'
-    int x = 0;               // next x' to copy
-};
-
-// Loads positions [x, x + kLineHalo) of a cursor (0 past the line's end or without entry).
-template <class T, bool UPPER>
-__device__ __forceinline__ void halo_load(const HaloCursor<T>& h, int nx, T (&v)[kLineHalo]) {
-    constexpr long long sx = UPPER ? -1 : 1;
+    for (int k = 0; k < nchunk; ++k) {
+        unsigned next = row;
+        const unsigned out = shared_addr(M.result(w, k)) + laneP;
 #pragma unroll
-    for (int u = 0; u < kLineHalo; ++u)
-        v[u] = (h.src != nullptr && h.x + u < nx) ? ld_relaxed_nb(h.src + sx * (h.x + u)) : T(0);
-}
-
-// Copies, in order, the loaded positions that no longer hold the sentinel; true when
-// the cursor moved.
-template <class T>
-__device__ __forceinline__ bool halo_retire(HaloCursor<T>& h, int nx, const T (&v)[kLineHalo]) {
-    if (h.src == nullptr || h.x >= nx) return false;
-    int adv = 0;
-    bool stop = false;
-#pragma unroll
-    for (int u = 0; u < kLineHalo; ++u) {
-        stop = stop || h.x + u >= nx || Sentinel<T>::is(v[u]);
-        st_shared_if(!stop, h.dst + static_cast<long long>(h.x + u) * h.stride, v[u]);
-        adv += stop ? 0 : 1;
-    }
-    h.x += adv;
-    return adv > 0;
-}
-
-template <class T, bool UPPER>
-__device__ __forceinline__ void line_halo(const LineTri<T>& P, int blk, const T* out, T* faceY, T* faceZ,
-                                          bool z_from_l2, int* status) {
-    const int lane = threadIdx.x & 31;
-    const int nx = P.g.nx, ny = P.g.ny, nz = P.g.nz;
-    const int wy = P.g.wy, wz = P.g.wz, by = P.g.by, bz = P.g.bz;
-    const int iy = blk % P.g.nby, iz = blk / P.g.nby;
-    const long long plane = static_cast<long long>(nx) * ny;
-    auto row0 = [&](int ys, int zs) {
-        const long long Y = UPPER ? ny - 1 - ys : ys;
-        const long long Z = UPPER ? nz - 1 - zs : zs;
-        return (UPPER ? nx - 1 : 0) + nx * Y + plane * Z;
-    };
-    HaloCursor<T> hy, hz;
-    if (ny > 1 && iy > 0 && lane < bz * wz) {  // line (y0 - 1, z) of block (iy - 1, iz)
-        const int wzi = lane / wz, zz = lane % wz;
-        const int zs = (iz * bz + wzi) * wz + zz;
-        if (zs < nz) {
-            hy.src = out + row0(iy * by * wy - 1, zs);
-            hy.dst = faceY + (wzi * by) * line_face_slot_y(P.g) + zz;
-            hy.stride = wz;
-        }
-    }
-    if (z_from_l2 && iz > 0 && lane < by * wy) {  // line (y, z0 - 1) of block (iy, iz - 1)
-        const int wyi = lane / wy, yy = lane % wy;
-        const int ys = (iy * by + wyi) * wy + yy;
-        if (ys < ny) {
-            hz.src = out + row0(ys, iz * bz * wz - 1);
-            hz.dst = faceZ + wyi * line_face_slot_z(P.g) + yy;
-            hz.stride = wy;
-        }
-    }
-    WaitBudget wb;
-    while ((hy.src != nullptr && hy.x < nx) || (hz.src != nullptr && hz.x < nx)) {
-        // both cursors' loads in flight together: one L2 round trip per round
-        T vy[kLineHalo], vz[kLineHalo];
-        halo_load<T, UPPER>(hy, nx, vy);
-        halo_load<T, UPPER>(hz, nx, vz);
-        const bool a = halo_retire<T>(hy, nx, vy);
-        const bool b = halo_retire<T>(hz, nx, vz);
-        if (!a && !b && wb.expired(status)) {
-            atomicExch(status + kStatusTimeout, 1);
-            // unblock the compute warps: the remaining entries become 0
-            for (; hy.src != nullptr && hy.x < nx; ++hy.x) st_volatile_shared(hy.dst + static_cast<long long>(hy.x) * hy.stride, T(0));
-            for (; hz.src != nullptr && hz.x < nx; ++hz.x) st_volatile_shared(hz.dst + static_cast<long long>(hz.x) * hz.stride, T(0));
-            break;
-        }
-    }
-}
-
-// Resets a block's faces: the sentinel where a value will be written, 0 where the lines
-// lie at the grid's boundary (slots of the first warps along y / z of the first blocks).
-template <class T>
-__device__ __forceinline__ void line_reset_faces(const LineGeom& g, int iy, int iz, T* faceY, T* zero_word) {
-    const long long fsy = line_face_slot_y(g), fsz = line_face_slot_z(g);
-    const long long fy_len = g.nw() * fsy;
-    const long long face_len = line_face_len<T>(g);
-    for (long long i = threadIdx.x; i < face_len; i += blockDim.x) {
-        const bool zero = i < fy_len ? (iy == 0 && static_cast<int>(i / fsy) % g.by == 0)
-                                     : (iz == 0 && static_cast<int>((i - fy_len) / fsz) / g.by == 0);
-        faceY[i] = zero ? T(0) : Sentinel<T>::value();
-    }
-    if (threadIdx.x == 0) *zero_word = T(0);
-}
-
-// GMRES normalises its new Krylov vector in the forward sweep: once a compute warp is
-// done with its lines (its own lanes are the only readers of their rows of `in`, and
-// all their copies have landed), it rescales them in place, the same product b * scale
-// its rows used.  Its y-lines of one plane z are one contiguous run of rows, walked by
-// the whole warp, 16 bytes per access where the runs allow it (eight accesses in flight
-// per lane).
-template <class T>
-__device__ __forceinline__ void line_rescale_warp(const LineGeom& g, int blk, T* in, T sc) {
-    const int lane = threadIdx.x & 31;
-    const int w = threadIdx.x >> 5;
-    const int wyi = w % g.by, wzi = w / g.by;
-    const int iy = blk % g.nby, iz = blk / g.nby;
-    const int y0 = (iy * g.by + wyi) * g.wy, y1 = min(g.ny, y0 + g.wy);
-    const int z0 = (iz * g.bz + wzi) * g.wz, z1 = min(g.nz, z0 + g.wz);
-    if (y0 >= y1 || z0 >= z1) return;
-    const long long run = static_cast<long long>(g.nx) * (y1 - y0);
-    const long long plane = static_cast<long long>(g.nx) * g.ny;
-    T* const base = in + static_cast<long long>(g.nx) * y0 + plane * z0;
-    constexpr int V = 16 / sizeof(T);  // rows per 16-byte access
-    const bool vec = run % V == 0 && plane % V == 0 && (reinterpret_cast<unsigned long long>(base) & 15ull) == 0;
-    if (vec) {
-        const int rv = static_cast<int>(run / V);
-        for (int zi = 0; zi < z1 - z0; ++zi) {
-#pragma unroll 8
-            for (int e = lane; e < rv; e += 32) {
-                T* p = base + zi * plane + static_cast<long long>(e) * V;
-                if constexpr (sizeof(T) == 4) {
-                    float4 v = *reinterpret_cast<const float4*>(p);
-                    v.x *= sc;
-                    v.y *= sc;
-                    v.z *= sc;
-                    v.w *= sc;
-                    *reinterpret_cast<float4*>(p) = v;
-                } else {
-                    double2 v = *reinterpret_cast<const double2*>(p);
-                    v.x *= sc;
-                    v.y *= sc;
-                    *reinterpret_cast<double2*>(p) = v;
+        for (int i = 0; i < C; ++i) {
+            const LineCoef<T> q = c[i % 2];
+            const T ql = lo[i % 2], a0 = bc[i % V];
+            const T fyv = pfy, fzv = pfz;
+            // the row, as if every predecessor were there and the quotient final
+            T acc;
+            auto solve = [&](T fy_v, T fz_v) -> T {
+                acc = fma(-q.cz, z_edge ? fz_v : sh_z, a0);
+                if (D3) acc = fma(-q.cy, y_edge ? fy_v : sh_y, acc);
+                acc = fma(-q.cx, prev, acc);
+                if constexpr (DIV) return line_quotient(acc, q.d, ql);  // the reference's division
+                if constexpr (UPPER) return acc * q.d;
+                return acc;
+            };
+            T r = solve(fyv, fzv);
+            T ny = T(0), nz;
+            shuffle(r, ny, nz);
+            if (i == C - 2 && k + 1 < nchunk) {
+                mbar_wait(M.full(w, k + 1), M.parity(k + 1), status);
+                __syncwarp();
+                next = shared_addr(M.slot(w, k + 1));
+            }
+            if (D3) lds_polled(fy + (i + 1) * WZ * Z, pfy);
+            lds_polled(fz + (i + 1) * WY * Z, pfz);
+            // (after the last step values that nothing uses)
+            load(i + 2 < C ? row : next, (i + 2) % C, i % 2);
+            if (i % V == V - 2) lds16((i + 2 < C ? row : next) + laneP + (kB + (i + 2) % C * Z), bn);
+            // otherwise: wait for the faces, divide again
+            if (__any_sync(0xffffffffu, line_late(fyv, fzv) || (DIV && line_quotient_bad(r, acc)))) {
+                T fy_v = fyv, fz_v = fzv;
+                if (D3 && Sentinel<T>::is(fyv)) fy_v = line_wait_shared<T>(fy + i * WZ * Z, status);
+                if (Sentinel<T>::is(fzv)) fz_v = line_wait_shared<T>(fz + i * WY * Z, status);
+                __syncwarp();
+                r = solve(fy_v, fz_v);
+                if constexpr (DIV) {
+                    if (line_quotient_bad(r, acc)) r = line_divide(acc, div + i * 32);
+                    __syncwarp();
                 }
+                shuffle(r, ny, nz);
+            }
+            prev = r;
+            sh_y = ny;
+            sh_z = nz;
+            // only the stored copies, which others poll, are kept off the sentinel
+            const T rs = off_sentinel(r);
+            if (D3) st_relaxed_generic(has_y, oy + i * WZ, rs);
+            st_relaxed_generic(has_z, oz + i * WY, rs);
+            res[i % V] = rs;
+            if (i % V == V - 1) {
+                sts16(out + (i - (V - 1)) * Z, res);
+#pragma unroll
+                for (int e = 0; e < V; ++e) bc[e] = bn[e];
             }
         }
-    } else {
-        for (int zi = 0; zi < z1 - z0; ++zi) {
-            T* const q = base + zi * plane;
-#pragma unroll 8
-            for (long long e = lane; e < run; e += 32) q[e] = q[e] * sc;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(M.done(w, k));
+        row = next;
+        if constexpr (DIV) div += C * 32;
+        fy += fy_adv;
+        fz += fz_adv;
+        oy += oy_adv;
+        oz += oz_adv;
+    }
+}
+
+// The helper of compute warp w: stages the operands chunk by chunk (the coefficients by
+// bulk copies; the right-hand side times `sc`, and written back so, when GMRES normalises
+// its new Krylov vector in the forward sweep) and writes the results out.  Its lanes take
+// kLineChunk consecutive rows of 32 / kLineChunk lines at a time.
+template <class T, bool UPPER>
+__device__ __forceinline__ void line_helper(const LineTri<T>& P, int blk, int w, const LineSmem<T, UPPER>& M, T* in, bool scaled,
+                                            T sc, T* out, int* status) {
+    constexpr int C = kLineChunk;
+    constexpr int S = kLineSlots;
+    constexpr int Q = 32 / C;  // lines per access
+    using St = LineStage<T, UPPER>;
+    const int lane = threadIdx.x & 31;
+    const int i = lane % C, q = lane / C;
+    const int nx = P.g.nx, ny = P.g.ny, nz = P.g.nz;
+    const int wyi = w % P.g.by, wzi = w / P.g.by;
+    const int iy = blk % P.g.nby, iz = blk / P.g.nby;
+    constexpr int sx = UPPER ? -1 : 1;
+    int x0[C], row0[C];  // x' and row of this lane's value of chunk 0 on line Q r + q
+#pragma unroll
+    for (int r = 0; r < C; ++r) {
+        const int l = Q * r + q;
+        const int yy = l % P.g.wy, zz = l / P.g.wy;
+        const int yq = (iy * P.g.by + wyi) * P.g.wy + yy;
+        const int zq = (iz * P.g.bz + wzi) * P.g.wz + zz;
+        const bool ok = yq < ny && zq < nz;
+        const int Y = UPPER ? ny - 1 - yq : yq;
+        const int Z = UPPER ? nz - 1 - zq : zq;
+        const int x = i - (yy + zz);
+        x0[r] = ok ? x : -(1 << 30);
+        row0[r] = ok ? static_cast<int>((UPPER ? nx - 1 : 0) + sx * x + static_cast<long long>(nx) * (Y + static_cast<long long>(ny) * Z)) : 0;
+    }
+    const int nchunk = P.g.psteps / C;
+    const long long first = P.g.slot(blk, w, 0, 0);
+    auto valid = [&](int r, int k) { return static_cast<unsigned>(x0[r] + C * k) < static_cast<unsigned>(nx); };
+    auto fetch = [&](int k, T (&v)[C]) {
+#pragma unroll
+        for (int r = 0; r < C; ++r) v[r] = valid(r, k) ? in[row0[r] + sx * C * k] : T(0);
+    };
+    auto flush = [&](int k) {
+        const T* const o = M.result(w, k) + q * kLinePitch<T> + i;
+#pragma unroll
+        for (int r = 0; r < C; ++r)
+            if (valid(r, k)) out[row0[r] + sx * C * k] = o[Q * r * kLinePitch<T>];
+    };
+    // chunk k, its right-hand side in v; v is left with that of chunk k + 2
+    auto stage = [&](int k, T (&v)[C]) {
+        if (k >= S) {  // the slot's previous chunk is computed
+            mbar_wait(M.done(w, k - S), M.parity(k - S), status);
+            __syncwarp();
+        }
+        T* const slot = M.slot(w, k);
+        unsigned long long* const full = M.full(w, k);
+        if (lane == 0) {
+            constexpr unsigned cb = St::kCoef * sizeof(T);
+            constexpr unsigned lb = St::kLo * sizeof(T);
+            mbar_arrive_expect(full, cb + lb);
+            bulk_load(slot, P.coef + line_coef_at<T, UPPER>(first + static_cast<long long>(k) * C * 32, 0), cb, full);
+            if (lb > 0) bulk_load(slot + St::kCoef, P.rlo + first + static_cast<long long>(k) * C * 32, lb, full);
+        }
+        T* const b = slot + St::kCoef + St::kLo + q * kLinePitch<T> + i;
+#pragma unroll
+        for (int r = 0; r < C; ++r) {
+            if (scaled) v[r] = v[r] * sc;
+            b[Q * r * kLinePitch<T>] = v[r];
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(full);
+        if (scaled) {
+#pragma unroll
+            for (int r = 0; r < C; ++r)
+                if (valid(r, k)) in[row0[r] + sx * C * k] = v[r];
+        }
+        if (k + 2 < nchunk) fetch(k + 2, v);
+        if (k >= S) flush(k - S);
+    };
+    // right-hand sides are loaded two chunks ahead: a chunk's loads take as long as the
+    // rest of the work on a chunk
+    T va[C], vb[C];
+    fetch(0, va);
+    if (nchunk > 1) fetch(1, vb);
+    for (int k = 0; k < nchunk; k += 2) {
+        stage(k, va);
+        if (k + 1 < nchunk) stage(k + 1, vb);
+    }
+    for (int k = max(0, nchunk - S); k < nchunk; ++k) {
+        mbar_wait(M.done(w, k), M.parity(k), status);
+        __syncwarp();
+        flush(k);
+    }
+}
+
+// A halo warp of block `blk`: copies faces that the previous block hands over through its
+// exchange buffer into shared memory as they arrive, and puts the buffer back to the
+// sentinel.  Lane e owns line e of the face (at most 32: `width` lines in each of the
+// `nslot` warps' faces, a warp's face being `face` values, and face slots `stride` warps
+// apart) and walks it in x' with its own cursor; a round loads the next kLineHalo
+// positions (one L2 round trip) and retires, in order, those that have arrived.
+constexpr int kLineHalo = 8;
+
+template <class T>
+__device__ __forceinline__ void line_halo(T* xch, T* faces, int face, int stride, int nslot, int width, int pad, int nx,
+                                          int* status) {
+    const int lane = threadIdx.x & 31;
+    const int slot = lane / width;
+    const bool on = slot < nslot;
+    T* const src = xch + static_cast<long long>(on ? slot : 0) * face + pad * width + lane % width;
+    T* const dst = faces + static_cast<long long>(on ? slot : 0) * stride * face + pad * width + lane % width;
+    int x = on ? 0 : nx;
+    bool idle = true;  // nothing arrived in the last round: poll one position per lane only
+    WaitBudget wb;
+    while (__any_sync(0xffffffffu, x < nx)) {
+        T v[kLineHalo];
+#pragma unroll
+        for (int u = 0; u < kLineHalo; ++u)
+            v[u] = x + u < nx && (u == 0 || !idle) ? ld_relaxed_nb(src + (x + u) * width) : Sentinel<T>::value();
+        int adv = 0;
+        bool stop = false;
+#pragma unroll
+        for (int u = 0; u < kLineHalo; ++u) {
+            stop = stop || Sentinel<T>::is(v[u]);
+            if (!stop) {
+                st_volatile_shared(dst + (x + u) * width, v[u]);
+                src[(x + u) * width] = Sentinel<T>::value();
+                ++adv;
+            }
+        }
+        x += adv;
+        idle = !__any_sync(0xffffffffu, adv > 0);
+        if (!idle) {
+            wb = WaitBudget();
+        } else if (wb.expired(status)) {
+            atomicExch(status + kStatusTimeout, 1);
+            // unblock the compute warps: the remaining entries become 0
+            for (; x < nx; ++x) st_volatile_shared(dst + x * width, T(0));
         }
     }
+}
+
+// Resets a block's faces, each warp whole faces: the sentinel where a value will be
+// written (x' in [0, nx)), 0 elsewhere and in the faces of lines at the grid's boundary;
+// and the mbarriers (`again`: they were used before).
+template <class T, bool UPPER>
+__device__ __forceinline__ void line_reset(const LineGeom& g, int iy, int iz, const LineSmem<T, UPPER>& M, bool again) {
+    const int lane = threadIdx.x & 31;
+    const int nwarp = static_cast<int>(blockDim.x >> 5);
+    const int nw = g.nw();
+    for (int f = static_cast<int>(threadIdx.x >> 5); f < (g.ny > 1 ? 2 * nw : nw); f += nwarp) {
+        const bool z = f < nw;
+        const int w = z ? f : f - nw;
+        const int width = z ? g.wy : g.wz;
+        const int len = z ? g.face_z() : g.face_y();
+        T* const p = (z ? M.face_z : M.face_y) + static_cast<long long>(w) * len;
+        const bool zero = z ? (iz == 0 && w / g.by == 0) : (iy == 0 && w % g.by == 0);
+        const int lo = zero ? len : g.pad() * width, hi = (g.pad() + g.nx) * width;
+        for (int j = lane; j < len; j += 32) p[j] = j >= lo && j < hi ? Sentinel<T>::value() : T(0);
+    }
+    constexpr int S = kLineSlots;
+    for (int j = threadIdx.x; j < kLineIdle; j += blockDim.x) M.idle[j] = T(0);
+    for (int j = threadIdx.x; j < 2 * nw * S; j += blockDim.x) {
+        if (again) mbar_inval(M.bar + j);
+        mbar_init(M.bar + j, j % (2 * S) < S ? 2 : 1);  // staged: bulk copies and right-hand side
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");  // (before the bulk copies use them)
+}
+
+// Block `blk` by this CTA (faces reset, all threads past a barrier).  next_z: the faceZ of
+// the next CTA along z in distributed shared memory (null: through L2); z_from_l2: this
+// CTA's first warps along z take their predecessors from the exchange buffer.
+template <class T, bool UPPER, int WY, bool D3>
+__device__ __forceinline__ void line_block(const LineTri<T>& P, int blk, const LineSmem<T, UPPER>& M, T* in, bool scaled, T sc,
+                                           T* out, T* next_z, bool z_from_l2, int* status) {
+    const LineGeom& g = P.g;
+    const int nw = g.nw();
+    const int w = threadIdx.x >> 5;
+    const int iy = blk % g.nby, iz = blk / g.nby;
+    line_stamp_start(P, blk);
+    if (w < nw) {
+        const int wyi = w % g.by, wzi = w / g.by;
+        T* to_y = nullptr;
+        T* to_z = nullptr;
+        if (D3) {
+            if (wyi + 1 < g.by)
+                to_y = M.face_y + static_cast<long long>(w + 1) * g.face_y();
+            else if (iy + 1 < g.nby)
+                to_y = P.xch + (blk + 1) * g.xch_block() + static_cast<long long>(wzi) * g.face_y();
+        }
+        if (wzi + 1 < g.bz)
+            to_z = M.face_z + static_cast<long long>(w + g.by) * g.face_z();
+        else if (next_z != nullptr)
+            to_z = next_z + static_cast<long long>(wyi) * g.face_z();
+        else if (iz + 1 < g.nbz)
+            to_z = P.xch + (blk + g.nby) * g.xch_block() + static_cast<long long>(g.bz) * g.face_y() +
+                   static_cast<long long>(wyi) * g.face_z();
+        line_compute<T, UPPER, WY, D3>(P, blk, w, M, to_y, to_z, status);
+        line_stamp_end(P, blk, 2 + w);
+    } else if (w < 2 * nw) {
+        line_helper<T, UPPER>(P, blk, w - nw, M, in, scaled, sc, out, status);
+    } else if (w == 2 * nw) {
+        T* const x = P.xch + blk * g.xch_block() + static_cast<long long>(g.bz) * g.face_y();
+        if (iz > 0 && z_from_l2) line_halo(x, M.face_z, g.face_z(), 1, g.by, WY, g.pad(), g.nx, status);
+        line_stamp_end(P, blk, 2 + nw);
+    } else if (D3) {
+        T* const x = P.xch + blk * g.xch_block();
+        if (iy > 0) line_halo(x, M.face_y, g.face_y(), g.by, g.bz, 32 / WY, g.pad(), g.nx, status);
+    }
+}
+
+// Streams the block's operands into L2 (they come from HBM: the Krylov vectors evict them
+// between sweeps).
+template <class T, bool UPPER>
+__device__ __forceinline__ void line_prefetch(const LineTri<T>& P, int blk) {
+    const int w = threadIdx.x >> 5;
+    if (w >= P.g.nw()) return;
+    const long long s0 = P.g.slot(blk, w, 0, 0);
+    const long long n = static_cast<long long>(P.g.psteps) * static_cast<long long>(sizeof(T));
+    prefetch_l2_range(P.coef + line_coef_at<T, UPPER>(s0, 0), n * line_step_values<T, UPPER>(), threadIdx.x & 31);
+    if (UPPER && sizeof(T) == 8) prefetch_l2_range(P.rlo + s0, n * 32, threadIdx.x & 31);
 }
 
 // Forward (UPPER = false): out = L^{-1} (scale * in), in rescaled in place when `scale`
-// is given (each compute warp's lines once that warp has solved them); backward (UPPER = true):
-// out = U^{-1} in.  in / out in natural order; out holds the sentinel at every row on
-// entry.  nw compute warps + 1 halo warp; dynamic shared memory line_smem_bytes.
-template <class T, bool UPPER>
-__global__ void __launch_bounds__((kLineMaxWarps + 1) * kWarp, 1)
+// is given; backward (UPPER = true): out = U^{-1} in.  in / out in natural order; what out
+// holds on entry does not matter.  g.threads() threads: compute warps, their helpers, halo
+// warps; dynamic shared memory line_smem_bytes.
+template <class T, bool UPPER, int WY, bool D3>
+__global__ void __launch_bounds__((2 * kLineMaxWarps + 2) * kWarp, sizeof(T) == 4 ? 2 : 1)
     sptrsv_line_kernel(LineTri<T> P, T* in, const double* scale, T* out, unsigned* counter, int* status,
                        const int* gate, int step) {
     if (gate_closed(gate, step)) return;
     extern __shared__ __align__(16) unsigned char line_smem[];
-    const int nw = P.g.nw();
-    const long long fsy = line_face_slot_y(P.g), fsz = line_face_slot_z(P.g);
-    const long long fy_len = nw * fsy;
-    const long long face_len = line_face_len<T>(P.g);
-    T* faceY = reinterpret_cast<T*>(line_smem);
-    T* faceZ = faceY + fy_len;
-    T* zero_word = faceY + face_len;  // holds 0
-    LineCoef<T>* cring = reinterpret_cast<LineCoef<T>*>(line_smem + line_ring_offset<T>(P.g));
-    T* bring = reinterpret_cast<T*>(cring + static_cast<long long>(kLineRing<T>) * nw * 32);
+    const LineSmem<T, UPPER> M = line_smem_view<T, UPPER>(P.g, line_smem);
     __shared__ int s_ticket;
     const bool scaled = !UPPER && scale != nullptr;
     const T sc = scaled ? static_cast<T>(*scale) : T(1);
-    const int w = threadIdx.x >> 5;
+    bool again = false;
     for (int tk = draw_block_ticket(counter, P.g.nblk, &s_ticket); tk < P.g.nblk;
          tk = draw_block_ticket(counter, P.g.nblk, &s_ticket)) {
         const int blk = P.order[tk];
-        const int iy = blk % P.g.nby, iz = blk / P.g.nby;
-        line_reset_faces<T>(P.g, iy, iz, faceY, zero_word);
-        // stream the warps' operands into L2 (the right-hand side was written by the
-        // previous kernel and is there already)
-        if (w < nw)
-            prefetch_l2_range(P.coef + P.g.slot(blk, w, 0, 0) * 4,
-                              static_cast<long long>(P.g.steps) * 128 * static_cast<long long>(sizeof(T)),
-                              threadIdx.x & 31);
+        line_reset<T, UPPER>(P.g, blk % P.g.nby, blk / P.g.nby, M, again);
+        again = true;
+        line_prefetch<T, UPPER>(P, blk);
         __syncthreads();
-        line_stamp_start(P, blk);
-        if (w < nw)
-            line_warp<T, UPPER>(P, blk, in, scaled, sc, out, faceY, faceZ, zero_word, cring, bring, 0u, status);
-        else
-            line_halo<T, UPPER>(P, blk, out, faceY, faceZ, true, status);
-        line_stamp_end(P, blk);
-        if (scaled && w < nw) line_rescale_warp<T>(P.g, blk, in, sc);
+        line_block<T, UPPER, WY, D3>(P, blk, M, in, scaled, sc, out, nullptr, true, status);
     }
 }
 
@@ -535,29 +766,22 @@ __global__ void __launch_bounds__((kLineMaxWarps + 1) * kWarp, 1)
 // grid: a cluster only waits for clusters of smaller tickets, whose CTAs are running or
 // done; the CTAs of one cluster are co-scheduled).  A CTA's last warps along z push
 // their results into the next CTA's face in distributed shared memory, so only the first
-// CTA of a cluster and the y-direction take their predecessors from L2 (halo warp).
-template <class T, bool UPPER>
-__global__ void __launch_bounds__((kLineMaxWarps + 1) * kWarp, 1)
+// CTA of a cluster and the y-direction take their predecessors from L2 (halo warps).
+template <class T, bool UPPER, int WY, bool D3>
+__global__ void __launch_bounds__((2 * kLineMaxWarps + 2) * kWarp, sizeof(T) == 4 ? 2 : 1)
     sptrsv_line_cluster_kernel(LineTri<T> P, T* in, const double* scale, T* out, unsigned* counter, int* status,
                                const int* gate, int step) {
     if (gate_closed(gate, step)) return;
     extern __shared__ __align__(16) unsigned char line_smem[];
-    const int nw = P.g.nw();
-    const long long fy_len = static_cast<long long>(nw) * line_face_slot_y(P.g);
-    const long long face_len = line_face_len<T>(P.g);
-    T* faceY = reinterpret_cast<T*>(line_smem);
-    T* faceZ = faceY + fy_len;
-    T* zero_word = faceY + face_len;
-    LineCoef<T>* cring = reinterpret_cast<LineCoef<T>*>(line_smem + line_ring_offset<T>(P.g));
-    T* bring = reinterpret_cast<T*>(cring + static_cast<long long>(kLineRing<T>) * nw * 32);
+    const LineSmem<T, UPPER> M = line_smem_view<T, UPPER>(P.g, line_smem);
     __shared__ int s_ticket;
     const bool scaled = !UPPER && scale != nullptr;
     const T sc = scaled ? static_cast<T>(*scale) : T(1);
-    const int w = threadIdx.x >> 5;
     const unsigned rank = cluster_rank_u32();
     const unsigned CL = cluster_size_u32();
     const int nq = P.g.nby * P.g.nbzc;
     const int nclusters = static_cast<int>(gridDim.x / CL);
+    bool again = false;
     for (;;) {
         // the previous round is complete in every CTA of the cluster (no push in flight)
         // before the ticket and the faces are reset
@@ -576,25 +800,17 @@ __global__ void __launch_bounds__((kLineMaxWarps + 1) * kWarp, 1)
         const bool active = iz < P.g.nbz;
         const int blk = iy + P.g.nby * iz;
         if (active) {
-            line_reset_faces<T>(P.g, iy, iz, faceY, zero_word);
-            if (w < nw)
-                prefetch_l2_range(P.coef + P.g.slot(blk, w, 0, 0) * 4,
-                                  static_cast<long long>(P.g.steps) * 128 * static_cast<long long>(sizeof(T)),
-                                  threadIdx.x & 31);
-        }
+            line_reset<T, UPPER>(P.g, iy, iz, M, again);
+            again = true;
+            line_prefetch<T, UPPER>(P, blk);
+            }
         __syncthreads();
         // every face of the cluster is reset before any CTA pushes into it
         cluster_sync_all();
         if (active) {
             const bool push = rank + 1 < CL && iz + 1 < P.g.nbz;
-            const unsigned remote = push ? map_shared_rank(faceZ, rank + 1) : 0u;
-            line_stamp_start(P, blk);
-            if (w < nw)
-                line_warp<T, UPPER>(P, blk, in, scaled, sc, out, faceY, faceZ, zero_word, cring, bring, remote, status);
-            else
-                line_halo<T, UPPER>(P, blk, out, faceY, faceZ, rank == 0, status);
-            line_stamp_end(P, blk);
-            if (scaled && w < nw) line_rescale_warp<T>(P.g, blk, in, sc);
+            T* const next = push ? map_generic_rank(M.face_z, rank + 1) : nullptr;
+            line_block<T, UPPER, WY, D3>(P, blk, M, in, scaled, sc, out, next, rank == 0, status);
         }
         __syncthreads();
     }
@@ -602,21 +818,22 @@ __global__ void __launch_bounds__((kLineMaxWarps + 1) * kWarp, 1)
 
 // Packs the operand stream of a structured factor from its CSR values: one thread per
 // slot.  L: c_z, c_y, c_x are the row's strict-lower entries (columns ascending:
-// r - nx ny, r - nx, r - 1, each present only inside the grid), d = 0.  U: c_z, c_y, c_x
-// are the strict-upper entries r + nx ny, r + nx, r + 1 (columns descending) and d = u_ii
-// (FP64) or RN(1 / u_ii), computed in FP64 and rounded once (FP32, as the other FP32
-// kernels).  Slots without a row hold zeros.
+// r - nx ny, r - nx, r - 1, each present only inside the grid).  U: c_z, c_y, c_x are the
+// strict-upper entries r + nx ny, r + nx, r + 1 (columns descending) and the reciprocal of
+// u_ii: FP32 RN(1 / u_ii), computed in FP64 and rounded once (as the other FP32 kernels);
+// FP64 in two parts (line_reciprocal), and u_ii itself.  Slots without a row hold zeros.
 template <class T, bool UPPER>
 __global__ void line_pack_kernel(LineGeom g, const int* __restrict__ rp, const int* __restrict__ diag,
-                                 const double* __restrict__ lu, T* __restrict__ dst) {
+                                 const double* __restrict__ lu, T* __restrict__ dst, T* __restrict__ rlo,
+                                 T* __restrict__ div) {
     const long long total = g.slots();
     const int nw = g.nw();
     for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
          i += static_cast<long long>(gridDim.x) * blockDim.x) {
         const int lane = static_cast<int>(i & 31);
         long long t = i >> 5;
-        const int s = static_cast<int>(t % g.steps);
-        t /= g.steps;
+        const int s = static_cast<int>(t % g.psteps);
+        t /= g.psteps;
         const int w = static_cast<int>(t % nw);
         const int b = static_cast<int>(t / nw);
         const int wyi = w % g.by, wzi = w / g.by;
@@ -625,7 +842,7 @@ __global__ void line_pack_kernel(LineGeom g, const int* __restrict__ rp, const i
         const int yq = (iy * g.by + wyi) * g.wy + yy;
         const int zq = (iz * g.bz + wzi) * g.wz + zz;
         const int xq = s - (yy + zz);
-        double cz = 0.0, cy = 0.0, cx = 0.0, d = 0.0;
+        double cz = 0.0, cy = 0.0, cx = 0.0, d = 0.0, lo = 0.0, u = 0.0;
         if (yq < g.ny && zq < g.nz && xq >= 0 && xq < g.nx) {
             const int X = UPPER ? g.nx - 1 - xq : xq;
             const int Y = UPPER ? g.ny - 1 - yq : yq;
@@ -638,18 +855,24 @@ __global__ void line_pack_kernel(LineGeom g, const int* __restrict__ rp, const i
                 if (X > 0) cx = lu[p++];
             } else {
                 int p = diag[r];
-                d = lu[p++];
+                u = lu[p++];
                 if (X < g.nx - 1) cx = lu[p++];
                 if (Y < g.ny - 1) cy = lu[p++];
                 if (Z < g.nz - 1) cz = lu[p++];
-                if (sizeof(T) == 4) d = 1.0 / d;
+                if (sizeof(T) == 4)
+                    d = 1.0 / u;
+                else
+                    line_reciprocal(u, d, lo);
             }
         }
-        T* o = dst + 4 * i;
-        o[0] = static_cast<T>(cz);
-        o[1] = static_cast<T>(cy);
-        o[2] = static_cast<T>(cx);
-        o[3] = static_cast<T>(d);
+        dst[line_coef_at<T, UPPER>(i, 0)] = static_cast<T>(cz);
+        dst[line_coef_at<T, UPPER>(i, 1)] = static_cast<T>(cy);
+        dst[line_coef_at<T, UPPER>(i, 2)] = static_cast<T>(cx);
+        if constexpr (UPPER || sizeof(T) == 4) dst[line_coef_at<T, UPPER>(i, 3)] = static_cast<T>(d);
+        if constexpr (UPPER && sizeof(T) == 8) {
+            rlo[i] = lo;
+            div[i] = u;
+        }
     }
 }
 
