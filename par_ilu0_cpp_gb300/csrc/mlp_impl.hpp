@@ -29,7 +29,6 @@ struct ShiftTrainer {
     int step = 0;
     DeviceBuffer<float> params, adam_m, adam_v, grad, partial, X, T, y;
     DeviceBuffer<int> idx;
-    DeviceBuffer<unsigned> counter;
     DeviceBuffer<double> loss;
 
     explicit ShiftTrainer(unsigned seed);

@@ -161,3 +161,30 @@ def test_committed_model_repairs_breakdowns():
     for r in res:
         assert not np.isfinite(r["plain_residual"]), r
         assert np.isfinite(r["learned_residual"]) and r["learned_residual"] < 0.1, r
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 255, 257, 8191])
+def test_training_step_at_partial_warps_and_blocks(n):
+    """Loss, gradient and Adam step where the last warp or block of the batch is partly
+    filled, on all samples and through an index list (a subset in another order).  The
+    network runs in FP32 (tanhf and the fast exponential: 1e-6 relative each, up to 20
+    terms of either sign per sum), so 1e-4 of the largest entry."""
+    rng = np.random.default_rng(n)
+    X = rng.normal(0, 1, (n, 4)).astype(np.float32)
+    T = np.abs(rng.normal(0, 0.2, n)).astype(np.float32)
+    p = _rand_params(n)
+    tr = api.ShiftTrainer(seed=1)
+    tr.set_data(X, T)
+    tr.params = p
+    grad, loss = tr.gradient()
+    lo, go = mo.loss_and_grad(p, X, T)
+    assert abs(loss - lo) <= 1e-5 * max(1.0, lo)
+    assert np.max(np.abs(grad - go)) <= 1e-4 * np.max(np.abs(go))
+    assert tr.gradient()[1] == loss and np.array_equal(tr.gradient()[0], grad)  # fixed order of the sums
+    idx = rng.permutation(n)[: (n + 1) // 2].astype(np.int32)
+    ls, gs = mo.loss_and_grad(p, X[idx], T[idx])
+    assert abs(tr.step(idx, 1e-2) - ls) <= 1e-5 * max(1.0, ls)
+    moved = tr.params - p
+    clear = np.abs(gs) > 1e-3 * np.max(np.abs(gs))  # the first Adam step is lr sign(g) there
+    assert np.max(np.abs(moved[clear] + 1e-2 * np.sign(gs[clear]))) <= 1e-4
