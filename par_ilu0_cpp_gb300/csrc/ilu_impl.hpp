@@ -7,6 +7,7 @@
 
 #include "device_util.hpp"
 #include "factor_lane.cuh"
+#include "line_factor.cuh"
 #include "line_sweep.cuh"
 #include "ilu_kernels.cuh"
 #include "ilu_solver.hpp"
@@ -137,6 +138,24 @@ struct LinePack {
     }
 };
 
+// Line-pipeline factorisation of a structured-grid factor (line_factor.cuh).
+struct LineFactorPack {
+    LineGeom g;
+    int grid = 0;  // CTAs launched
+    DeviceBuffer<int> order;    // blocks (clusters) by ticket
+    DeviceBuffer<double> rows;  // operand stream, packed from A by every factorisation
+    DeviceBuffer<double> xch;   // faces handed over through L2, at the sentinel between launches
+
+    LineFactor view() const {
+        LineFactor p;
+        p.g = g;
+        p.order = order.get();
+        p.rows = rows.get();
+        p.xch = xch.get();
+        return p;
+    }
+};
+
 // Host-side results of the pattern analysis (integer output identical to the
 // reference's; see analysis.hpp).
 struct Analysis {
@@ -201,6 +220,8 @@ struct IluSolver::Impl {
             return GP32;
     }
     bool grid64 = false, grid32 = false;
+    gb300::LineFactorPack GF;  // line-pipeline factorisation of the same factors
+    bool fact_line = false;
     int grid_mode = 0;  // 1 or 0 (automatic): on when the pattern qualifies; -1: off
     int grid_wy = 0;    // requested lanes of a warp along y (0 automatic)
     int grid_by = 0;    // requested warps of a CTA along y (0 automatic)
@@ -260,7 +281,7 @@ struct IluSolver::Impl {
     const void* subst_key() const;
     // Throws when a dependency wait timed out since the last call.
     void check_status(cudaStream_t s);
-    // Puts the line sweeps' exchange buffers back to the sentinel (after a timeout).
+    // Puts the line kernels' exchange buffers back to the sentinel (after a timeout).
     void reset_exchange(cudaStream_t s);
     // Writes wait_limit_us into the device status words (when they exist).
     void push_wait_limit();

@@ -279,22 +279,26 @@ static void launch_level_upper(const LevelPack& U, int grid, int threads, cudaSt
     }
 }
 
-static void gather_level_pack(const LevelPack& P, bool lower, const double* lu, cudaStream_t s, int sms) {
+// Packs the factor values for the level-ordered kernels of the wanted types; returns the launches.
+static int gather_level_pack(const LevelPack& P, bool lower, bool f64, bool f32, const double* lu, cudaStream_t s, int sms) {
     const int threads = 256;
     auto grid_for = [&](long long count) {
         long long g = ceil_div<long long>(count, threads);
         return static_cast<int>(std::max<long long>(1, std::min<long long>(g, 8LL * sms)));
     };
-    if (P.slots > 0) {
-        pack_gather_kernel<double><<<grid_for(P.slots), threads, 0, s>>>(P.slots, P.src.get(), lu, P.v64.get());
-        pack_gather_kernel<float><<<grid_for(P.slots), threads, 0, s>>>(P.slots, P.src.get(), lu, P.v32.get());
-    }
-    if (!lower) {
-        const long long nd = static_cast<long long>(P.ntask) * kWarp;
-        pack_gather_kernel<double><<<grid_for(nd), threads, 0, s>>>(nd, P.dsrc.get(), lu, P.d64.get());
-        pack_gather_recip_kernel<<<grid_for(nd), threads, 0, s>>>(nd, P.dsrc.get(), lu, P.d32.get());
-    }
+    int launches = 0;
+    auto gather = [&](auto kern, long long count, const int* src, auto* dst) {
+        if (count == 0) return;
+        kern<<<grid_for(count), threads, 0, s>>>(count, src, lu, dst);
+        ++launches;
+    };
+    const long long nd = lower ? 0 : static_cast<long long>(P.ntask) * kWarp;
+    if (f64) gather(pack_gather_kernel<double>, P.slots, P.src.get(), P.v64.get());
+    if (f32) gather(pack_gather_kernel<float>, P.slots, P.src.get(), P.v32.get());
+    if (f64) gather(pack_gather_kernel<double>, nd, P.dsrc.get(), P.d64.get());
+    if (f32) gather(pack_gather_recip_kernel, nd, P.dsrc.get(), P.d32.get());
     GB_CUDA_CHECK(cudaGetLastError());
+    return launches;
 }
 
 // Block-internal levels of rows [lo, hi): dependencies on rows outside the block do
@@ -905,83 +909,88 @@ static const void* line_kernel_ptr(const LineGeom& g, bool cluster, bool upper) 
                  : reinterpret_cast<const void*>(line_kernel<T, false>(g, cluster));
 }
 
-// Raises the kernels' shared-memory limit, sizes the grid and allocates the packed
-// operands of value type T; false when a CTA cannot be resident.  With G.g.cl > 0 the
-// cluster variant is sized (clusters of cl CTAs along z); `try_cluster` (first type
-// configured) decides G.g.cl: with `max_cluster` 1, clusters of 16, else 8, where the grid
-// has at least two blocks along z and such a cluster can be scheduled; with 2 .. 16,
-// clusters of at most that many CTAs; with 0, none.
+// Sizes the launch of line kernels of geometry g with `smem` bytes of dynamic shared memory
+// (raising their limit): chooses g.cl and returns the CTAs to launch, 0 when a CTA cannot be
+// resident.  With `max_cluster` 1 (automatic) clusters along z of the largest of 16
+// (non-portable), 8, 4 and 2 CTAs of which all are resident at once, or else of at most
+// `most`; with 2 .. 16, clusters of at most that many CTAs; with 0, none.  `wait_lines`:
+// blocks of tickets more than that many grid lines deep are left to the CTAs that finish
+// first.
+static int size_line_launch(LineGeom& g, int threads, size_t smem, int max_cluster, int most, int wait_lines,
+                            const std::vector<const void*>& clustered, const std::vector<const void*>& plain,
+                            const DeviceInfo& dev) {
+    auto prepare = [&](const void* kern, int cl) {
+        GB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+        if (cl > 8) GB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    };
+    g.cl = 0;
+    g.nbzc = 0;
+    int grid = 0;
+    for (int want : {16, 8, 4, 2}) {
+        if (max_cluster != 1) want = max_cluster;
+        if (want < 2 || g.nbz < 2) break;
+        const int cl = std::min(want, g.nbz);
+        const int nbzc = ceil_div(g.nbz, cl);
+        const int need = g.nby * nbzc;
+        int nclusters = 1 << 30;
+        for (const void* kern : clustered) {
+            prepare(kern, cl);
+            cudaLaunchAttribute attr[1];
+            cudaLaunchConfig_t cfg = line_cluster_config(need * cl, threads, smem, cl, nullptr, attr);
+            int nc = 0;
+            if (cudaOccupancyMaxActiveClusters(&nc, kern, &cfg) != cudaSuccess) {
+                cudaGetLastError();
+                nc = 0;
+            }
+            nclusters = std::min(nclusters, nc);
+        }
+        if (nclusters >= need || (nclusters > 0 && want <= most) || max_cluster != 1) {
+            if (nclusters > 0) {
+                g.cl = cl;
+                g.nbzc = nbzc;
+                grid = std::min(nclusters, need) * cl;
+            }
+            break;
+        }
+    }
+    const int unit = std::max(1, g.cl);
+    int early = 0;
+    for (int iz = 0; iz < ceil_div(g.nbz, unit); ++iz)
+        for (int iy = 0; iy < g.nby; ++iy)
+            if (iy * g.by * g.wy + iz * unit * g.bz * g.wz <= wait_lines) early += unit;
+    if (g.cl > 0) {
+        for (const void* kern : clustered) prepare(kern, g.cl);
+        return std::min(grid, early);
+    }
+    int per_sm = 1 << 30;
+    for (const void* kern : plain) {
+        prepare(kern, 0);
+        int r = 0;
+        GB_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, kern, threads, smem));
+        per_sm = std::min(per_sm, r);
+    }
+    return per_sm < 1 ? 0 : std::min({g.nblk, per_sm * dev.sms, early});
+}
+
+// Configures the sweeps of value type T and allocates their packed operands; false when a
+// CTA cannot be resident.
 template <class T>
 static bool configure_line(LinePack<T>& G, const DeviceInfo& dev, int max_cluster) {
     const size_t smem = std::max(static_cast<size_t>(std::max(line_smem_bytes<T, false>(G.g), line_smem_bytes<T, true>(G.g))),
                                  static_cast<size_t>(G.smem_floor));
     if (smem + 1024 > static_cast<size_t>(dev.smem_optin)) return false;
-    {
-        G.g.cl = 0;
-        G.g.nbzc = 0;
-        // automatic: the largest of 16 (non-portable), 8, 4 and 2 CTAs of which all
-        // clusters are resident at once; for grids that do not fit at once, 8 for FP32 and 4
-        // for FP64 (the measurements above line_geometry)
-        const int most = G.g.ny == 1 ? 16 : (sizeof(T) == 4 ? 8 : 4);
-        for (int want : {16, 8, 4, 2}) {
-            if (max_cluster != 1) want = max_cluster;
-            if (want < 2 || G.g.nbz < 2) break;
-            const int cl = std::min(want, G.g.nbz);
-            const int nbzc = ceil_div(G.g.nbz, cl);
-            const int need = G.g.nby * nbzc;
-            int nclusters = 1 << 30;
-            for (bool upper : {false, true}) {
-                const void* kern = line_kernel_ptr<T>(G.g, true, upper);
-                GB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-                if (cl > 8) GB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-                cudaLaunchAttribute attr[1];
-                cudaLaunchConfig_t cfg = line_cluster_config(need * cl, G.threads, smem, cl, nullptr, attr);
-                int nc = 0;
-                if (cudaOccupancyMaxActiveClusters(&nc, kern, &cfg) != cudaSuccess) {
-                    cudaGetLastError();
-                    nc = 0;
-                }
-                nclusters = std::min(nclusters, nc);
-            }
-            if (nclusters >= need || (nclusters > 0 && want <= most) || max_cluster != 1) {
-                if (nclusters > 0) {
-                    G.g.cl = cl;
-                    G.g.nbzc = nbzc;
-                    G.grid = std::min(nclusters, need) * cl;
-                }
-                break;
-            }
-        }
-    }
-    // Tickets launched at once: blocks more than kLineWaitLines lines deep would wait past
-    // about 60 us, after which a block's first steps run five times slower (seen in the
-    // timelines, whatever the waiting warps do); they are left to the CTAs that finish first
-    // (96^3 FP64 backward: 172 us with all 144 blocks resident, 125 us with 120 or 128).
+    // for grids that do not fit at once clusters of 8 for FP32 and 4 for FP64 (the
+    // measurements above line_geometry)
+    const int most = G.g.ny == 1 ? 16 : (sizeof(T) == 4 ? 8 : 4);
+    // Blocks more than kLineWaitLines lines deep would wait past about 60 us, after which a
+    // block's first steps run five times slower (seen in the timelines, whatever the waiting
+    // warps do) (96^3 FP64 backward: 172 us with all 144 blocks resident, 125 us with 120 or
+    // 128).
     constexpr int kLineWaitLines = sizeof(T) == 8 ? 130 : 300;
-    const int unit = std::max(1, G.g.cl);
-    int early = 0;
-    for (int iz = 0; iz < ceil_div(G.g.nbz, unit); ++iz)
-        for (int iy = 0; iy < G.g.nby; ++iy)
-            if (iy * G.g.by * G.g.wy + iz * unit * G.g.bz * G.g.wz <= kLineWaitLines) early += unit;
-    if (G.g.cl > 0) {
-        G.grid = std::min(G.grid, early);
-        for (bool upper : {false, true}) {
-            const void* kern = line_kernel_ptr<T>(G.g, true, upper);
-            GB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-            if (G.g.cl > 8) GB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-        }
-    } else {
-        int per_sm = 0;
-        for (bool upper : {false, true}) {
-            const void* kern = line_kernel_ptr<T>(G.g, false, upper);
-            GB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-            int r = 0;
-            GB_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, kern, G.threads, smem));
-            if (r < 1) return false;
-            per_sm = per_sm == 0 ? r : std::min(per_sm, r);
-        }
-        G.grid = std::min({G.g.nblk, per_sm * dev.sms, early});
-    }
+    G.grid = size_line_launch(G.g, G.threads, smem, max_cluster, most, kLineWaitLines,
+                              {line_kernel_ptr<T>(G.g, true, false), line_kernel_ptr<T>(G.g, true, true)},
+                              {line_kernel_ptr<T>(G.g, false, false), line_kernel_ptr<T>(G.g, false, true)}, dev);
+    if (G.grid == 0) return false;
     const size_t slots = static_cast<size_t>(G.g.slots());
     G.l.reserve(slots / 32 * line_step_values<T, false>());
     G.u.reserve(slots / 32 * line_step_values<T, true>());
@@ -992,15 +1001,17 @@ static bool configure_line(LinePack<T>& G, const DeviceInfo& dev, int max_cluste
     return true;
 }
 
-// Packs the factor values into the operand streams of type T.
+// Packs the factor values into the operand streams of type T (`sweeps`: bit 0 L, bit 1 U);
+// returns the launches.
 template <class T>
-static void pack_line(LinePack<T>& G, const int* rp, const int* diag, const double* lu, cudaStream_t s, int sms) {
+static int pack_line(LinePack<T>& G, int sweeps, const int* rp, const int* diag, const double* lu, cudaStream_t s, int sms) {
     const long long slots = G.g.slots();
     const int threads = 256;
     const int grid = static_cast<int>(std::max<long long>(1, std::min<long long>(ceil_div<long long>(slots, threads), 8LL * sms)));
-    line_pack_kernel<T, false><<<grid, threads, 0, s>>>(G.g, rp, diag, lu, G.l.get(), nullptr, nullptr);
-    line_pack_kernel<T, true><<<grid, threads, 0, s>>>(G.g, rp, diag, lu, G.u.get(), G.lo.get(), G.div.get());
+    if (sweeps & 1) line_pack_kernel<T, false><<<grid, threads, 0, s>>>(G.g, rp, diag, lu, G.l.get(), nullptr, nullptr);
+    if (sweeps & 2) line_pack_kernel<T, true><<<grid, threads, 0, s>>>(G.g, rp, diag, lu, G.u.get(), G.lo.get(), G.div.get());
     GB_CUDA_CHECK(cudaGetLastError());
+    return (sweeps & 1) + (sweeps >> 1);
 }
 
 // `set`: the exchange buffer (LinePack).
@@ -1016,6 +1027,60 @@ static void launch_line(const LinePack<T>& G, int set, cudaStream_t s, T* in, co
     } else {
         kern<<<G.grid, G.threads, smem, s>>>(G.view(UPPER, set), in, scale, out, counter, status, gate, step);
     }
+    GB_CUDA_CHECK(cudaGetLastError());
+}
+
+// The line-pipeline factorisation's kernel for a geometry.
+using LineFactorKernel = void (*)(LineFactor, unsigned*, int*);
+static LineFactorKernel line_factor_kernel(const LineGeom& g, bool cluster) {
+    if (g.ny == 1) return cluster ? ilu_factor_line_kernel<1, false, true> : ilu_factor_line_kernel<1, false, false>;
+    if (g.wy == 4) return cluster ? ilu_factor_line_kernel<4, true, true> : ilu_factor_line_kernel<4, true, false>;
+    return cluster ? ilu_factor_line_kernel<8, true, true> : ilu_factor_line_kernel<8, true, false>;
+}
+
+// Sets up the line-pipeline factorisation for a grid; false when a CTA cannot be resident.
+static bool setup_line_factor(LineFactorPack& G, int nx, int ny, int nz, int max_cluster, const DeviceInfo& dev,
+                              cudaStream_t s) {
+    if (nx < 3 || ny == 2) return false;  // elimination would change more than the diagonal
+    G.grid = 0;
+    for (int by : {kLineFactorWarps, 1}) {
+        G.g = line_geometry(nx, ny, nz, 0, by, 1, 8);
+        const size_t smem = static_cast<size_t>(line_factor_smem_bytes(G.g));
+        if (smem + 1024 > static_cast<size_t>(dev.smem_optin)) continue;
+        // (clusters only where all blocks are resident at once: 200^3 2.5 ms without, 2.9 ms
+        // with clusters of 4; 128^3 the same)
+        G.grid = size_line_launch(G.g, line_factor_threads(G.g), smem, max_cluster, 0, 1 << 30,
+                                  {reinterpret_cast<const void*>(line_factor_kernel(G.g, true))},
+                                  {reinterpret_cast<const void*>(line_factor_kernel(G.g, false))}, dev);
+        if (G.grid > 0) break;
+    }
+    if (G.grid == 0) return false;
+    const std::vector<int> order = line_block_order(G.g);
+    G.order.upload(order.data(), order.size(), s);
+    G.rows.reserve(static_cast<size_t>(line_factor_at(G.g.slots(), 0)));
+    G.xch.reserve(static_cast<size_t>(3 * G.g.nblk * G.g.xch_block()));
+    fill_sentinel(G.xch.get(), static_cast<long long>(G.xch.size()), s, dev.sms);
+    GB_CUDA_CHECK(cudaStreamSynchronize(s));  // `order` must outlive the copy
+    return true;
+}
+
+// Factorises the values in lu (A's on entry) with the optional diagonal shift.
+static void launch_line_factor(const LineFactorPack& G, const int* rp, const int* diag, double* lu, const double* shift,
+                               unsigned* counter, int* status, const DeviceInfo& dev, cudaStream_t s) {
+    const long long slots = G.g.slots();
+    const int threads = 256;
+    const int grid = static_cast<int>(std::min<long long>(ceil_div<long long>(slots, threads), 8LL * dev.sms));
+    line_factor_pack_kernel<<<grid, threads, 0, s>>>(G.g, rp, diag, lu, shift, G.rows.get());
+    const size_t smem = static_cast<size_t>(line_factor_smem_bytes(G.g));
+    const auto kern = line_factor_kernel(G.g, G.g.cl > 0);
+    if (G.g.cl > 0) {
+        cudaLaunchAttribute attr[1];
+        cudaLaunchConfig_t cfg = line_cluster_config(G.grid, line_factor_threads(G.g), smem, G.g.cl, s, attr);
+        GB_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, G.view(), counter, status));
+    } else {
+        kern<<<G.grid, line_factor_threads(G.g), smem, s>>>(G.view(), counter, status);
+    }
+    line_factor_unpack_kernel<<<grid, threads, 0, s>>>(G.g, rp, G.rows.get(), lu, status);
     GB_CUDA_CHECK(cudaGetLastError());
 }
 
@@ -1208,6 +1273,7 @@ void IluSolver::Impl::check_status(cudaStream_t s) {
 void IluSolver::Impl::reset_exchange(cudaStream_t s) {
     for (auto& x : GP64.xch) fill_sentinel(x.get(), static_cast<long long>(x.size()), s, dev.sms);
     for (auto& x : GP32.xch) fill_sentinel(x.get(), static_cast<long long>(x.size()), s, dev.sms);
+    fill_sentinel(GF.xch.get(), static_cast<long long>(GF.xch.size()), s, dev.sms);
 }
 
 IluSolver::Impl* IluSolver::impl_ensure() {
@@ -1292,7 +1358,7 @@ void IluSolver::SetupMatrix() {
     ++im.setup_gen;
     // structured-grid line-pipeline sweeps: 7- / 5-point stencil factors in natural order
     // (automatic, grid_mode 0: when the other schedules are automatic too; 1: always)
-    im.grid64 = im.grid32 = false;
+    im.grid64 = im.grid32 = im.fact_line = false;
     if (im.grid_mode == 1 || (im.grid_mode == 0 && im.block_rows == 0)) {
         int gx = 0, gy = 0, gz = 0;
         if (detect_grid(n, rp, ci, im.an.diag, gx, gy, gz)) {
@@ -1300,6 +1366,11 @@ void IluSolver::SetupMatrix() {
             // (one geometry for both types while timelines are recorded, so that one
             // LLJBASH_IluInfo describes them)
             im.grid32 = setup_line(im, im.GP32, gx, gy, gz, s);
+            // Factorisation: the line pipeline unless a kernel or a ticket order is asked for
+            // (five to nine times faster than the warp-per-row kernel from 32^2 and 16^3 to
+            // 1024^2 and 200^3, flat and deep grids included)
+            if (im.factor_kernel == 0 && im.ticket_order == 0)
+                im.fact_line = setup_line_factor(im.GF, gx, gy, gz, im.grid_cluster, im.dev, s);
         }
     }
     // forced (grid_mode 1): every sweep of a configured type; automatic: timed against the
@@ -1542,7 +1613,11 @@ bool IluSolver::FactorizeFrom(const double* values, bool on_device) {
             } else if (shift_kind == 1) {
                 shift = im.shift.get();
             }
-            if (im.fact_lane) {
+            if (im.fact_line) {
+                launch_line_factor(im.GF, im.rp.get(), im.diag.get(), im.lu.get(), shift, im.counters.get(),
+                                   im.status.get(), im.dev, s);
+                im.launches += 3;
+            } else if (im.fact_lane) {
                 fill_sentinel(im.lf_pub.get(), im.lf_pub_len, s, im.dev.sms);
                 LaneFactor F;
                 F.n = n;
@@ -1560,7 +1635,7 @@ bool IluSolver::FactorizeFrom(const double* values, bool on_device) {
                 im.launches += 2;
             }
             auto kern = im.fact_pre == 8 ? ilu_factor_kernel<8> : ilu_factor_kernel<2>;
-            if (!im.fact_lane && im.ticket_order == 2) {
+            if (!im.fact_line && !im.fact_lane && im.ticket_order == 2) {
                 // subtree partitions first (one CTA each, no waits), then the separator rows
                 if (im.sub_parts > 0) {
                     auto sk = im.fact_pre == 8 ? ilu_factor_subtree_kernel<8> : ilu_factor_subtree_kernel<2>;
@@ -1576,7 +1651,7 @@ bool IluSolver::FactorizeFrom(const double* values, bool on_device) {
                         im.done.get(), im.stamp, im.counters.get(), im.status.get(), im.fact_cap, im.fact_hcap);
                     im.launches += 1;
                 }
-            } else if (!im.fact_lane) {
+            } else if (!im.fact_line && !im.fact_lane) {
                 kern<<<im.grid_fact, im.fact_warps * kWarp, im.fact_smem, s>>>(
                     n, im.rp.get(), im.ci.get(), im.diag.get(),
                     im.ticket_order == 1 ? im.order_fact.get() : im.order_l.get(), im.lu.get(), shift, im.done.get(),
@@ -1584,34 +1659,31 @@ bool IluSolver::FactorizeFrom(const double* values, bool on_device) {
                 im.launches += 1;
             }
             GB_CUDA_CHECK(cudaGetLastError());
-            if (im.blk64) {
-                gather_block(im.LB64, true, im.lu.get(), s, im.dev.sms);
-                gather_block(im.UB64, false, im.lu.get(), s, im.dev.sms);
-                im.launches += 2;
-            }
-            if (im.blk32) {
-                gather_block(im.LB32, true, im.lu.get(), s, im.dev.sms);
-                gather_block(im.UB32, false, im.lu.get(), s, im.dev.sms);
-                im.launches += 2;
-            }
+            // Packs of the schedules in use (all of them until the sweeps are chosen: on 128^3
+            // the packs that nothing reads took 0.4 ms of every factorisation)
+            const int line64 = im.line_tuned ? im.line_use64 : 0, line32 = im.line_tuned ? im.line_use32 : 0;
+            const bool l64 = (line64 & 1) == 0, u64 = (line64 & 2) == 0;  // sweeps on another schedule
+            const bool l32 = (line32 & 1) == 0, u32 = (line32 & 2) == 0;
+            auto pack_blocks = [&](const BlockPack& P, bool lower) {
+                gather_block(P, lower, im.lu.get(), s, im.dev.sms);
+                im.launches += 1;
+            };
+            if (im.blk64 && l64) pack_blocks(im.LB64, true);
+            if (im.blk64 && u64) pack_blocks(im.UB64, false);
+            if (im.blk32 && l32) pack_blocks(im.LB32, true);
+            if (im.blk32 && u32) pack_blocks(im.UB32, false);
             if (im.level_packs) {
-                gather_level_pack(im.L, true, im.lu.get(), s, im.dev.sms);
-                gather_level_pack(im.U, false, im.lu.get(), s, im.dev.sms);
-                im.launches += 6;
+                im.launches += gather_level_pack(im.L, true, !im.blk64 && l64, !im.blk32 && l32, im.lu.get(), s, im.dev.sms);
+                im.launches += gather_level_pack(im.U, false, !im.blk64 && u64, !im.blk32 && u32, im.lu.get(), s, im.dev.sms);
             }
             if (im.levelsync) {
-                gather_level_pack(im.LS, true, im.lu.get(), s, im.dev.sms);
-                gather_level_pack(im.US, false, im.lu.get(), s, im.dev.sms);
-                im.launches += 6;
+                im.launches += gather_level_pack(im.LS, true, true, true, im.lu.get(), s, im.dev.sms);
+                im.launches += gather_level_pack(im.US, false, true, true, im.lu.get(), s, im.dev.sms);
             }
-            if (im.grid64) {
-                pack_line<double>(im.GP64, im.rp.get(), im.diag.get(), im.lu.get(), s, im.dev.sms);
-                im.launches += 2;
-            }
-            if (im.grid32) {
-                pack_line<float>(im.GP32, im.rp.get(), im.diag.get(), im.lu.get(), s, im.dev.sms);
-                im.launches += 2;
-            }
+            if (im.grid64)
+                im.launches += pack_line<double>(im.GP64, im.line_tuned ? line64 : 3, im.rp.get(), im.diag.get(), im.lu.get(), s, im.dev.sms);
+            if (im.grid32)
+                im.launches += pack_line<float>(im.GP32, im.line_tuned ? line32 : 3, im.rp.get(), im.diag.get(), im.lu.get(), s, im.dev.sms);
         }
         GB_CUDA_CHECK(cudaEventRecord(im.ev1, s));
         std::array<int, kStatusWords> h{};
@@ -1622,6 +1694,9 @@ bool IluSolver::FactorizeFrom(const double* values, bool on_device) {
         im.last_factor_ms += ms;
         if (h[kStatusTimeout] != 0) {
             im.factorized = false;
+            GB_CUDA_CHECK(cudaMemsetAsync(im.counters.get(), 0, sizeof(unsigned) * 8, s));
+            im.reset_exchange(s);
+            GB_CUDA_CHECK(cudaStreamSynchronize(s));
             throw std::runtime_error("dependency wait timed out on the device");
         }
         return h;
