@@ -898,10 +898,14 @@ template <class T, bool UPPER>
 using LineKernel = void (*)(LineTri<T>, T*, const double*, T*, unsigned*, int*, const int*, int);
 template <class T, bool UPPER>
 static LineKernel<T, UPPER> line_kernel(const LineGeom& g, bool cluster) {
-    if (g.ny == 1) return cluster ? sptrsv_line_cluster_kernel<T, UPPER, 1, false> : sptrsv_line_kernel<T, UPPER, 1, false>;
-    if (g.wy == 1) return cluster ? sptrsv_line_cluster_kernel<T, UPPER, 1, true> : sptrsv_line_kernel<T, UPPER, 1, true>;
-    if (g.wy == 4) return cluster ? sptrsv_line_cluster_kernel<T, UPPER, 4, true> : sptrsv_line_kernel<T, UPPER, 4, true>;
-    return cluster ? sptrsv_line_cluster_kernel<T, UPPER, 8, true> : sptrsv_line_kernel<T, UPPER, 8, true>;
+    constexpr bool W3 = sizeof(T) == 8 && UPPER;  // (line_stays_warm of 3-D grids)
+    if (g.ny == 1 && line_stays_warm(g, sizeof(T), UPPER))
+        return cluster ? sptrsv_line_cluster_kernel<T, UPPER, 1, false, true> : sptrsv_line_kernel<T, UPPER, 1, false, true>;
+    if (g.ny == 1)
+        return cluster ? sptrsv_line_cluster_kernel<T, UPPER, 1, false, false> : sptrsv_line_kernel<T, UPPER, 1, false, false>;
+    if (g.wy == 1) return cluster ? sptrsv_line_cluster_kernel<T, UPPER, 1, true, W3> : sptrsv_line_kernel<T, UPPER, 1, true, W3>;
+    if (g.wy == 4) return cluster ? sptrsv_line_cluster_kernel<T, UPPER, 4, true, W3> : sptrsv_line_kernel<T, UPPER, 4, true, W3>;
+    return cluster ? sptrsv_line_cluster_kernel<T, UPPER, 8, true, W3> : sptrsv_line_kernel<T, UPPER, 8, true, W3>;
 }
 template <class T>
 static const void* line_kernel_ptr(const LineGeom& g, bool cluster, bool upper) {
@@ -982,12 +986,12 @@ static bool configure_line(LinePack<T>& G, const DeviceInfo& dev, int max_cluste
     // for grids that do not fit at once clusters of 8 for FP32 and 4 for FP64 (the
     // measurements above line_geometry)
     const int most = G.g.ny == 1 ? 16 : (sizeof(T) == 4 ? 8 : 4);
-    // Blocks more than kLineWaitLines lines deep would wait past about 60 us, after which a
-    // block's first steps run five times slower (seen in the timelines, whatever the waiting
-    // warps do) (96^3 FP64 backward: 172 us with all 144 blocks resident, 125 us with 120 or
-    // 128).
-    constexpr int kLineWaitLines = sizeof(T) == 8 ? 130 : 300;
-    G.grid = size_line_launch(G.g, G.threads, smem, max_cluster, most, kLineWaitLines,
+    // 3-D blocks more than 130 (FP64) or 300 lines deep would wait past about 50 us, after which
+    // a block's first steps run five times slower (their instructions have left the cache):
+    // they are left to the CTAs that finish first (96^3 FP64 backward: 172 us with all 144
+    // blocks resident, 125 us with 120 or 128).  2-D sweeps keep them warm (line_stays_warm).
+    const int wait_lines = G.g.ny == 1 ? 1 << 30 : (sizeof(T) == 8 ? 130 : 300);
+    G.grid = size_line_launch(G.g, G.threads, smem, max_cluster, most, wait_lines,
                               {line_kernel_ptr<T>(G.g, true, false), line_kernel_ptr<T>(G.g, true, true)},
                               {line_kernel_ptr<T>(G.g, false, false), line_kernel_ptr<T>(G.g, false, true)}, dev);
     if (G.grid == 0) return false;

@@ -68,21 +68,6 @@ struct LinePivot {
     double d, hi, lo;
 };
 
-// Bound of the waits for faces, looked at about every microsecond of waiting.
-struct LineWait {
-    WaitBudget wb;
-    int calls = 0;
-    __device__ __forceinline__ bool expired(int* status) {
-        if ((++calls & 15) != 0) return false;
-        return slow(status);
-    }
-    __device__ __noinline__ bool slow(int* status) {
-        wb.polls |= 1023;  // so that expired() looks at the clock and at the status word
-        const bool out = wb.expired(status);
-        if (out) atomicExch(status + kStatusTimeout, 1);
-        return out;
-    }
-};
 __device__ __forceinline__ bool line_late(const LinePivot& y, const LinePivot& z) {
     return line_late(y.d, z.d) || line_late(y.hi, z.hi) || line_late(y.lo, z.lo);
 }

@@ -58,6 +58,7 @@ constexpr int kLineSlots = 3;
 // compute warps) and 16 bytes more, which spread the lanes over the banks.
 template <class T>
 constexpr int kLinePitch = kLineChunk + 16 / static_cast<int>(sizeof(T));
+constexpr int kLineWarmLines = 300;  // FP32: lines that are passed in about 50 us
 constexpr int kLineStepAlign = 8;  // steps of a warp are rounded up to a multiple of this
 
 struct LineGeom {
@@ -258,6 +259,51 @@ __device__ __noinline__ T line_wait_shared(unsigned a, int* status) {
     }
 }
 
+// Whether a face value has not arrived (lanes without a face hold zeros).
+__device__ __forceinline__ bool line_late(float y, float z) { return max(__float_as_uint(y), __float_as_uint(z)) == 0xFFFFFFFFu; }
+__device__ __forceinline__ bool line_late(double y, double z) {
+    // (only the sentinel has these upper words: published values are off it)
+    return max(static_cast<unsigned>(__double2hiint(y)), static_cast<unsigned>(__double2hiint(z))) == 0xFFFFFFFFu;
+}
+
+// Whether waiting warps keep their instructions warm (WARM, line_compute), chosen per grid,
+// type (elem bytes) and sweep.  us, without / with, forward and backward: 1000^2 (blocks wait
+// for 300 us and more) FP32 214 / 156 and 195 / 139, FP64 392 / 267 and 694 / 405; FP64
+// backward 96^3 143 / 128 and 256^2 121 / 111.  It costs a little where the waits are short:
+// 256^2 FP32 44 / 46 and 39 / 41; 128^3, whose deep blocks are left to later CTAs, FP32 87 /
+// 90 and 83 / 85, FP64 forward 128 / 135.
+inline bool line_stays_warm(const LineGeom& g, int elem, bool upper) {
+    if (g.ny == 1) return elem == 8 || g.nz > kLineWarmLines;
+    return elem == 8 && upper;
+}
+// Polls a warp's faces at its first step for about 20 us; whether all have arrived.
+template <class T>
+__device__ __forceinline__ bool line_first_faces(unsigned fy, unsigned fz) {
+    for (int i = 0; i < 640; ++i) {
+        T y, z;
+        lds_polled(fy, y);
+        lds_polled(fz, z);
+        if (!__any_sync(0xffffffffu, line_late(y, z))) return true;
+    }
+    return false;
+}
+
+// Bound of a wait made of many polls at a time: the clock is read every 16th time.
+struct LineWait {
+    WaitBudget wb;
+    int calls = 0;
+    __device__ __forceinline__ bool expired(int* status) {
+        if ((++calls & 15) != 0) return false;
+        return slow(status);
+    }
+    __device__ __noinline__ bool slow(int* status) {
+        wb.polls |= 1023;  // so that expired() looks at the clock and at the status word
+        const bool out = wb.expired(status);
+        if (out) atomicExch(status + kStatusTimeout, 1);
+        return out;
+    }
+};
+
 // ---- FP64 division by a known divisor ----
 // acc / d for the rows of U: GB300 issues one FP64 instruction per warp in 64 cycles on a
 // scheduler, and a division takes about nine of them (566 cycles measured), all on the
@@ -383,21 +429,18 @@ __device__ __forceinline__ LineSmem<T, UPPER> line_smem_view(const LineGeom& g, 
     return m;
 }
 
-// Whether a face value has not arrived (lanes without a face hold zeros).
-__device__ __forceinline__ bool line_late(float y, float z) { return max(__float_as_uint(y), __float_as_uint(z)) == 0xFFFFFFFFu; }
-__device__ __forceinline__ bool line_late(double y, double z) {
-    // (only the sentinel has these upper words: published values are off it)
-    return max(static_cast<unsigned>(__double2hiint(y)), static_cast<unsigned>(__double2hiint(z))) == 0xFFFFFFFFu;
-}
-
 // One compute warp's share of block `blk`: wy x wz lines over psteps steps.  Slots without
 // a row hold zero coefficients and a zero right-hand side, so a lane outside its line
 // computes zeros (or, past the line's end, values that nobody reads) and needs no
 // predicate.  to_y / to_z: the face (generic address, this warp's lane pattern) that its
 // last lanes along y / z fill, null: none.
-template <class T, bool UPPER, int WY, bool D3>
-__device__ __forceinline__ void line_compute(const LineTri<T>& P, int blk, int w, const LineSmem<T, UPPER>& M, T* to_y, T* to_z,
-                                             int* status) {
+//
+// False (WARM) when the first faces have not arrived: then only the first chunk was
+// run, on the idle area, and the caller tries again.  A warp that only polls for about 50 us
+// finds the instructions of its steps gone from the cache, and its first chunk took 8 us.
+template <class T, bool UPPER, int WY, bool D3, bool WARM>
+__device__ __forceinline__ bool line_compute(const LineTri<T>& P, int blk, int w, const LineSmem<T, UPPER>& M, T* to_y, T* to_z,
+                                             LineWait& wait, int* status) {
     constexpr int WZ = 32 / WY;
     constexpr int PAD = WY + WZ - 2;
     constexpr int C = kLineChunk;
@@ -408,18 +451,20 @@ __device__ __forceinline__ void line_compute(const LineTri<T>& P, int blk, int w
     const int shift = PAD - (yy + zz);  // face position of step 0
     const bool y_edge = D3 && yy == 0;
     const bool z_edge = zz == 0;
-    const int nchunk = P.g.psteps / C;
     constexpr unsigned Z = sizeof(T);
     const unsigned idle = shared_addr(M.idle);
     const T* div = DIV ? P.div + P.g.slot(blk, w, 0, lane) : nullptr;
     unsigned fy = y_edge ? shared_addr(M.face_y + static_cast<long long>(w) * P.g.face_y() + shift * WZ + zz) : idle;
     unsigned fz = z_edge ? shared_addr(M.face_z + static_cast<long long>(w) * P.g.face_z() + shift * WY + yy) : idle;
+    const bool dry = WARM && !line_first_faces<T>(fy, fz) && !wait.expired(status);
+    if (dry) fy = fz = idle;
     const unsigned fy_adv = y_edge ? C * WZ * Z : 0u, fz_adv = z_edge ? C * WY * Z : 0u;
-    const bool has_y = D3 && to_y != nullptr && yy == WY - 1;
-    const bool has_z = to_z != nullptr && zz == WZ - 1;
+    const bool has_y = !dry && D3 && to_y != nullptr && yy == WY - 1;
+    const bool has_z = !dry && to_z != nullptr && zz == WZ - 1;
     T* oy = has_y ? to_y + shift * WZ + zz : M.idle + kLineIdle;
     T* oz = has_z ? to_z + shift * WY + yy : M.idle + kLineIdle;
     const int oy_adv = has_y ? C * WZ : 0, oz_adv = has_z ? C * WY : 0;
+    const int nchunk = dry ? 1 : P.g.psteps / C;
 
     mbar_wait(M.full(w, 0), 0u, status);
     __syncwarp();
@@ -506,7 +551,7 @@ __device__ __forceinline__ void line_compute(const LineTri<T>& P, int blk, int w
             }
         }
         __syncwarp();
-        if (lane == 0) mbar_arrive(M.done(w, k));
+        if (lane == 0 && !dry) mbar_arrive(M.done(w, k));
         row = next;
         if constexpr (DIV) div += C * 32;
         fy += fy_adv;
@@ -514,6 +559,7 @@ __device__ __forceinline__ void line_compute(const LineTri<T>& P, int blk, int w
         oy += oy_adv;
         oz += oz_adv;
     }
+    return !dry;
 }
 
 // The helper of compute warp w: stages the operands chunk by chunk (the coefficients by
@@ -684,7 +730,7 @@ __device__ __forceinline__ void line_reset(const LineGeom& g, int iy, int iz, co
 // Block `blk` by this CTA (faces reset, all threads past a barrier).  next_z: the faceZ of
 // the next CTA along z in distributed shared memory (null: through L2); z_from_l2: this
 // CTA's first warps along z take their predecessors from the exchange buffer.
-template <class T, bool UPPER, int WY, bool D3>
+template <class T, bool UPPER, int WY, bool D3, bool WARM>
 __device__ __forceinline__ void line_block(const LineTri<T>& P, int blk, const LineSmem<T, UPPER>& M, T* in, bool scaled, T sc,
                                            T* out, T* next_z, bool z_from_l2, int* status) {
     const LineGeom& g = P.g;
@@ -693,23 +739,30 @@ __device__ __forceinline__ void line_block(const LineTri<T>& P, int blk, const L
     const int iy = blk % g.nby, iz = blk / g.nby;
     line_stamp_start(P, blk);
     if (w < nw) {
-        const int wyi = w % g.by, wzi = w / g.by;
-        T* to_y = nullptr;
-        T* to_z = nullptr;
-        if (D3) {
-            if (wyi + 1 < g.by)
-                to_y = M.face_y + static_cast<long long>(w + 1) * g.face_y();
-            else if (iy + 1 < g.nby)
-                to_y = P.xch + (blk + 1) * g.xch_block() + static_cast<long long>(wzi) * g.face_y();
+        LineWait wait;
+        for (bool done = false; !done;) {
+            // (addresses are worked out anew rather than held in registers through the steps)
+            int b = blk, cw = w;
+            if (WARM) asm volatile("" : "+r"(b), "+r"(cw));
+            const int by = b % g.nby, bz = b / g.nby;
+            const int wyi = cw % g.by, wzi = cw / g.by;
+            T* to_y = nullptr;
+            T* to_z = nullptr;
+            if (D3) {
+                if (wyi + 1 < g.by)
+                    to_y = M.face_y + static_cast<long long>(cw + 1) * g.face_y();
+                else if (by + 1 < g.nby)
+                    to_y = P.xch + (b + 1) * g.xch_block() + static_cast<long long>(wzi) * g.face_y();
+            }
+            if (wzi + 1 < g.bz)
+                to_z = M.face_z + static_cast<long long>(cw + g.by) * g.face_z();
+            else if (next_z != nullptr)
+                to_z = next_z + static_cast<long long>(wyi) * g.face_z();
+            else if (bz + 1 < g.nbz)
+                to_z = P.xch + (b + g.nby) * g.xch_block() + static_cast<long long>(g.bz) * g.face_y() +
+                       static_cast<long long>(wyi) * g.face_z();
+            done = line_compute<T, UPPER, WY, D3, WARM>(P, b, cw, M, to_y, to_z, wait, status);
         }
-        if (wzi + 1 < g.bz)
-            to_z = M.face_z + static_cast<long long>(w + g.by) * g.face_z();
-        else if (next_z != nullptr)
-            to_z = next_z + static_cast<long long>(wyi) * g.face_z();
-        else if (iz + 1 < g.nbz)
-            to_z = P.xch + (blk + g.nby) * g.xch_block() + static_cast<long long>(g.bz) * g.face_y() +
-                   static_cast<long long>(wyi) * g.face_z();
-        line_compute<T, UPPER, WY, D3>(P, blk, w, M, to_y, to_z, status);
         line_stamp_end(P, blk, 2 + w);
     } else if (w < 2 * nw) {
         line_helper<T, UPPER>(P, blk, w - nw, M, in, scaled, sc, out, status);
@@ -739,7 +792,7 @@ __device__ __forceinline__ void line_prefetch(const LineTri<T>& P, int blk) {
 // is given; backward (UPPER = true): out = U^{-1} in.  in / out in natural order; what out
 // holds on entry does not matter.  g.threads() threads: compute warps, their helpers, halo
 // warps; dynamic shared memory line_smem_bytes.
-template <class T, bool UPPER, int WY, bool D3>
+template <class T, bool UPPER, int WY, bool D3, bool WARM>
 __global__ void __launch_bounds__((2 * kLineMaxWarps + 2) * kWarp, sizeof(T) == 4 ? 2 : 1)
     sptrsv_line_kernel(LineTri<T> P, T* in, const double* scale, T* out, unsigned* counter, int* status,
                        const int* gate, int step) {
@@ -757,7 +810,7 @@ __global__ void __launch_bounds__((2 * kLineMaxWarps + 2) * kWarp, sizeof(T) == 
         again = true;
         line_prefetch<T, UPPER>(P, blk);
         __syncthreads();
-        line_block<T, UPPER, WY, D3>(P, blk, M, in, scaled, sc, out, nullptr, true, status);
+        line_block<T, UPPER, WY, D3, WARM>(P, blk, M, in, scaled, sc, out, nullptr, true, status);
     }
 }
 
@@ -767,7 +820,7 @@ __global__ void __launch_bounds__((2 * kLineMaxWarps + 2) * kWarp, sizeof(T) == 
 // done; the CTAs of one cluster are co-scheduled).  A CTA's last warps along z push
 // their results into the next CTA's face in distributed shared memory, so only the first
 // CTA of a cluster and the y-direction take their predecessors from L2 (halo warps).
-template <class T, bool UPPER, int WY, bool D3>
+template <class T, bool UPPER, int WY, bool D3, bool WARM>
 __global__ void __launch_bounds__((2 * kLineMaxWarps + 2) * kWarp, sizeof(T) == 4 ? 2 : 1)
     sptrsv_line_cluster_kernel(LineTri<T> P, T* in, const double* scale, T* out, unsigned* counter, int* status,
                                const int* gate, int step) {
@@ -810,7 +863,7 @@ __global__ void __launch_bounds__((2 * kLineMaxWarps + 2) * kWarp, sizeof(T) == 
         if (active) {
             const bool push = rank + 1 < CL && iz + 1 < P.g.nbz;
             T* const next = push ? map_generic_rank(M.face_z, rank + 1) : nullptr;
-            line_block<T, UPPER, WY, D3>(P, blk, M, in, scaled, sc, out, next, rank == 0, status);
+            line_block<T, UPPER, WY, D3, WARM>(P, blk, M, in, scaled, sc, out, next, rank == 0, status);
         }
         __syncthreads();
     }
