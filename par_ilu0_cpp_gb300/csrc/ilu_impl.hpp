@@ -196,6 +196,7 @@ struct IluSolver::Impl {
     int lf_ntask = 0, grid_lane_fact = 0;
     gb300::DeviceBuffer<double> lu;
     gb300::DeviceBuffer<double> shift;      // per-row diagonal shift (learned), optional
+    gb300::DeviceBuffer<double2> rinv;      // per-row reciprocal of the pivot in two parts (warp per row)
     gb300::DeviceBuffer<int> done;          // per-row ready stamps of the factorisation
     gb300::DeviceBuffer<unsigned> counters;  // ticket counters [0] fact, [1] L, [2] U
     gb300::DeviceBuffer<int> status;         // StatusWord array

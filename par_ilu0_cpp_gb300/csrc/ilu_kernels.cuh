@@ -15,12 +15,13 @@
 #pragma once
 
 #include "common.cuh"
+#include "division.cuh"
 
 namespace gb300 {
 
 constexpr int kFactWarps = 8;    // most warps per block of the factorisation kernel
 constexpr int kFactCap = 128;    // least row length staged in shared memory per warp
-constexpr int kFactEntryBytes = 2 * sizeof(double) + 3 * sizeof(int);  // staged bytes per entry
+constexpr int kFactEntryBytes = sizeof(double) + 3 * sizeof(int);  // staged bytes per entry
 constexpr int kFactHashMin = 24;  // rows longer than this locate update positions by hashing
 constexpr int kFactSmemMax = 200 * 1024;  // dynamic shared memory of one factorisation block
 constexpr int kSolveWarps = 8;   // warps per block of the substitution kernels
@@ -67,13 +68,18 @@ __device__ __forceinline__ bool gate_closed(const int* gate, int step) {
 // entries; every entry of row j therefore receives its updates in ascending k, the same
 // sequence of operations as the reference.
 //
-// Row j is staged in shared memory together with, for every pivot k, diag[k], the end
-// of row k and u_kk, all loaded in parallel once the pivots' ready flags are acquired;
-// the strict-upper entries of the next pivot row (PRE per lane: 2, or 8 for matrices
-// whose rows have more than 64 entries above the diagonal) are loaded into registers
-// while the current pivot is eliminated.  The sequential chain per pivot is then one
-// division (one lane) and a shared-memory search-and-update, instead of three dependent
-// global round trips.  The update position of a column in row j is found by binary
+// Row j is staged in shared memory together with, for every pivot k, diag[k] and the end
+// of row k.  Pivots are eliminated as they become ready (WAIT: leading ready flags acquired
+// 32 at a time), so that most of a row is done before its last pivot is final: a level then
+// costs the elimination of the last few pivots, not of all of them.  1 / u_kk and the
+// strict-upper entries of the next pivot row (PRE per lane: 2, or 8 for matrices whose rows
+// have more than 64 entries above the diagonal) are loaded into registers while the current
+// pivot is eliminated, if that is ready.  A finished row leaves the two-part reciprocal of its
+// pivot (rinv), so that the sequential chain per pivot is two FP64 instructions instead of
+// a division, and a shared-memory search-and-update.  Factorisations, ms, with all pivots
+// awaited first and a division each / now: 27-point ILU(2) of 30 x 27 x 25 41.4 / 2.7,
+// ILU(1) of 44 x 40 x 42 18.5 / 3.9, ILU(0) of 60^3 7.6 / 2.3; 7-point ILU(1) of 64^3 4.0 /
+// 2.1; 5-point ILU(2) of 300^2 9.3 / 4.2.  The update position of a column in row j is found by binary
 // search over the staged columns for short rows; rows longer than kFactHashMin entries
 // build an open-addressing table (column -> position, hcap slots per warp, linear
 // probing) once and look positions up in one or two probes: a binary search over tens
@@ -88,7 +94,6 @@ __device__ __forceinline__ bool gate_closed(const int* gate, int step) {
 // factorisation kernels, `cap` entries and `hcap` table slots per warp).
 struct FactStage {
     double* sval;
-    double* sukk;
     int* scol;
     int* skd;
     int* ske;
@@ -102,8 +107,7 @@ __device__ __forceinline__ FactStage fact_stage(double* fact_smem, int cap, int 
     const size_t wc = static_cast<size_t>(w) * cap, nc_ = static_cast<size_t>(nw) * cap;
     FactStage st;
     st.sval = fact_smem + wc;
-    st.sukk = fact_smem + nc_ + wc;
-    int* ibase = reinterpret_cast<int*>(fact_smem + 2 * nc_);
+    int* ibase = reinterpret_cast<int*>(fact_smem + nc_);
     st.scol = ibase + wc;
     st.skd = ibase + nc_ + wc;
     st.ske = ibase + 2 * nc_ + wc;
@@ -112,15 +116,15 @@ __device__ __forceinline__ FactStage fact_stage(double* fact_smem, int cap, int 
     return st;
 }
 
-// Elimination of row j by one warp, every pivot row already final (see ilu_factor_kernel).
-template <int PRE>
+// Elimination of row j by one warp.  WAIT: pivot k is final once done[k] == stamp, and so is
+// set done[j]; otherwise every pivot row is final already.
+template <int PRE, bool WAIT>
 __device__ __forceinline__ void ilu_factor_row(int j, const int* __restrict__ rp, const int* __restrict__ ci,
                                                const int* __restrict__ diag, double* lu,
-                                               const double* __restrict__ shift, int* status, int cap,
-                                               const FactStage& st) {
+                                               const double* __restrict__ shift, double2* rinv, int* done, int stamp,
+                                               int* status, int cap, const FactStage& st) {
     const int lane = threadIdx.x & 31;
     double* sval = st.sval;
-    double* sukk = st.sukk;
     int* scol = st.scol;
     int* skd = st.skd;
     int* ske = st.ske;
@@ -140,7 +144,6 @@ __device__ __forceinline__ void ilu_factor_row(int j, const int* __restrict__ rp
                 const int kd = diag[c];
                 skd[t] = kd;
                 ske[t] = rp[c + 1];
-                sukk[t] = __ldcg(lu + kd);
             }
         }
         // column -> position table of row j (long rows): hsize slots, a power of two
@@ -178,9 +181,11 @@ __device__ __forceinline__ void ilu_factor_row(int j, const int* __restrict__ rp
         // strict-upper entries of pivot row t held by this lane: p = kd + 1 + lane + 32 u
         int nc[PRE];
         double nv[PRE];
+        double2 nr = make_double2(0.0, 0.0);
         auto load_pivot = [&](int t) {
             const int p0 = skd[t] + 1 + lane;
             const int pe = ske[t];
+            nr = __ldcg(rinv + scol[t]);
 #pragma unroll
             for (int u = 0; u < PRE; ++u) {
                 const int p = p0 + u * kWarp;
@@ -188,8 +193,27 @@ __device__ __forceinline__ void ilu_factor_row(int j, const int* __restrict__ rp
                 nv[u] = p < pe ? __ldcg(lu + p) : 0.0;
             }
         };
-        if (dloc > 0) load_pivot(0);
+        int ready = WAIT ? 0 : dloc;  // leading pivots known to be final
+        bool loaded = false;          // pivot t is in nc, nv, nu
         for (int t = 0; t < dloc; ++t) {
+            if (WAIT && ready <= t) {
+                WaitBudget wb;
+                for (;;) {
+                    const int q = ready + lane;
+                    const unsigned f = __ballot_sync(0xffffffffu, q < dloc && ld_acquire(done + scol[q]) == stamp);
+                    ready += f == 0xffffffffu ? 32 : __ffs(~f) - 1;
+                    if (ready > t) break;
+                    if (__any_sync(0xffffffffu, wb.expired(status))) {
+                        if (lane == 0) atomicExch(status + kStatusTimeout, 1);
+                        ready = dloc;
+                        break;
+                    }
+                    if (wb.polls > kSpinBeforeSleep) __nanosleep(32);
+                }
+                __syncwarp();
+            }
+            if (!loaded) load_pivot(t);
+            const double2 r = nr;
             int cc[PRE];
             double cv[PRE];
 #pragma unroll
@@ -197,20 +221,18 @@ __device__ __forceinline__ void ilu_factor_row(int j, const int* __restrict__ rp
                 cc[u] = nc[u];
                 cv[u] = nv[u];
             }
-            if (t + 1 < dloc) load_pivot(t + 1);
-            double l = 0.0;
-            if (lane == 0) {
-                l = sval[t] / sukk[t];
-                sval[t] = l;
-            }
-            l = __shfl_sync(0xffffffffu, l, 0);
+            loaded = t + 1 < ready;
+            if (loaded) load_pivot(t + 1);
+            const double a = sval[t];
+            double l = line_quotient(a, r.x, r.y);
+            int pos[PRE];  // (looked up while the quotient is computed)
 #pragma unroll
-            for (int u = 0; u < PRE; ++u) {
-                if (cc[u] >= 0) {
-                    const int pos = locate(cc[u], t);
-                    if (pos >= 0) sval[pos] = fma(-cv[u], l, sval[pos]);
-                }
-            }
+            for (int u = 0; u < PRE; ++u) pos[u] = cc[u] >= 0 ? locate(cc[u], t) : -1;
+            if (line_quotient_bad(l, a)) l = a / __ldcg(lu + skd[t]);
+            if (lane == 0) lu[b + t] = l;
+#pragma unroll
+            for (int u = 0; u < PRE; ++u)
+                if (pos[u] >= 0) sval[pos[u]] = fma(-cv[u], l, sval[pos[u]]);
             // strict-upper entries beyond the register window (long pivot rows)
             for (int p = skd[t] + 1 + lane + PRE * kWarp; p < ske[t]; p += kWarp) {
                 const int pos = locate(ci[p], t);
@@ -218,7 +240,15 @@ __device__ __forceinline__ void ilu_factor_row(int j, const int* __restrict__ rp
             }
             __syncwarp();
         }
-        for (int t = lane; t < len; t += kWarp) lu[b + t] = sval[t];
+        for (int t = dloc + lane; t < len; t += kWarp) lu[b + t] = sval[t];
+        double2 r;
+        line_pivot_reciprocal(sval[dloc], r.x, r.y);
+        if (lane == 0) rinv[j] = r;
+        if (WAIT) {
+            __threadfence();
+            __syncwarp();
+            if (lane == 0) st_release(done + j, stamp);
+        }
         if (lane == 0) {
             const double u = sval[dloc];
             if (!(fabs(u) > 0.0) || !isfinite(u)) {
@@ -229,6 +259,10 @@ __device__ __forceinline__ void ilu_factor_row(int j, const int* __restrict__ rp
     } else {
         const int* col = ci + b;
         double* val = lu + b;
+        if (WAIT) {
+            for (int t = lane; t < dloc; t += kWarp) wait_flag(done + col[t], stamp, status);
+            __syncwarp();
+        }
         if (shift != nullptr && lane == 0) __stcg(val + dloc, __ldcg(val + dloc) + shift[j]);
         __syncwarp();
         for (int t = 0; t < dloc; ++t) {
@@ -244,6 +278,14 @@ __device__ __forceinline__ void ilu_factor_row(int j, const int* __restrict__ rp
             }
             __syncwarp();
         }
+        double2 r;
+        line_pivot_reciprocal(__ldcg(val + dloc), r.x, r.y);
+        if (lane == 0) rinv[j] = r;
+        if (WAIT) {
+            __threadfence();
+            __syncwarp();
+            if (lane == 0) st_release(done + j, stamp);
+        }
         if (lane == 0) {
             const double u = __ldcg(val + dloc);
             if (!(fabs(u) > 0.0) || !isfinite(u)) {
@@ -257,7 +299,7 @@ __device__ __forceinline__ void ilu_factor_row(int j, const int* __restrict__ rp
 template <int PRE>
 __global__ void __launch_bounds__(kFactWarps * kWarp)
     ilu_factor_kernel(int n, const int* __restrict__ rp, const int* __restrict__ ci, const int* __restrict__ diag,
-                      const int* __restrict__ order, double* lu, const double* __restrict__ shift, int* done,
+                      const int* __restrict__ order, double* lu, const double* __restrict__ shift, double2* rinv, int* done,
                       int stamp, unsigned* counter, int* status, int cap, int hcap) {
     extern __shared__ double fact_smem[];
     const int lane = threadIdx.x & 31;
@@ -266,14 +308,8 @@ __global__ void __launch_bounds__(kFactWarps * kWarp)
     while (q < n) {
         const int qn = draw_ticket(counter, n, lane);
         const int j = order[q];
-        const int b = rp[j];
-        const int dloc = diag[j] - b;
-        for (int t = lane; t < dloc; t += kWarp) wait_flag(done + ci[b + t], stamp, status);
+        ilu_factor_row<PRE, true>(j, rp, ci, diag, lu, shift, rinv, done, stamp, status, cap, st);
         __syncwarp();
-        ilu_factor_row<PRE>(j, rp, ci, diag, lu, shift, status, cap, st);
-        __threadfence();
-        __syncwarp();
-        if (lane == 0) st_release(done + j, stamp);
         q = qn;
     }
 }
@@ -292,8 +328,8 @@ template <int PRE>
 __global__ void __launch_bounds__(kSubtreeWarps * kWarp)
     ilu_factor_subtree_kernel(const int* __restrict__ part_ptr, const int* __restrict__ grp_ptr,
                               const int* __restrict__ rows, const int* __restrict__ rp, const int* __restrict__ ci,
-                              const int* __restrict__ diag, double* lu, const double* __restrict__ shift, int* done,
-                              int stamp, int* status, int cap, int hcap) {
+                              const int* __restrict__ diag, double* lu, const double* __restrict__ shift, double2* rinv,
+                              int* done, int stamp, int* status, int cap, int hcap) {
     extern __shared__ double fact_smem[];
     const int lane = threadIdx.x & 31;
     const int w = threadIdx.x >> 5;
@@ -302,7 +338,7 @@ __global__ void __launch_bounds__(kSubtreeWarps * kWarp)
     const int p = blockIdx.x;
     for (int gidx = part_ptr[p]; gidx < part_ptr[p + 1]; ++gidx) {
         for (int q = grp_ptr[gidx] + w; q < grp_ptr[gidx + 1]; q += nw)
-            ilu_factor_row<PRE>(rows[q], rp, ci, diag, lu, shift, status, cap, st);
+            ilu_factor_row<PRE, false>(rows[q], rp, ci, diag, lu, shift, rinv, done, stamp, status, cap, st);
         // the group's rows (global memory, written by this CTA) before the next group reads them
         __syncthreads();
     }

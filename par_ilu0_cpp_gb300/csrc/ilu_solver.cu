@@ -1468,6 +1468,7 @@ void IluSolver::SetupMatrix() {
     if (im.factor_kernel == 2 && im.ticket_order != 2 && n > 0)
         im.fact_lane = build_lane_factor(n, rp, ci, im.an.diag,
                                          im.ticket_order == 1 ? tree_order : im.an.order_l, im, s);
+    if (!im.fact_line && !im.fact_lane) im.rinv.reserve(static_cast<size_t>(std::max(n, 1)));
     // Factorisation launch: rows staged in shared memory up to the longest row where a
     // warp's share fits (fewer warps per block for long rows), a wider register window
     // of the next pivot row when pivot rows are long.
@@ -1645,20 +1646,20 @@ bool IluSolver::FactorizeFrom(const double* values, bool on_device) {
                     auto sk = im.fact_pre == 8 ? ilu_factor_subtree_kernel<8> : ilu_factor_subtree_kernel<2>;
                     sk<<<im.sub_parts, im.sub_warps * kWarp, im.sub_smem, s>>>(
                         im.sub_part_ptr.get(), im.sub_grp_ptr.get(), im.sub_rows_d.get(), im.rp.get(), im.ci.get(),
-                        im.diag.get(), im.lu.get(), shift, im.done.get(), im.stamp, im.status.get(), im.fact_cap,
+                        im.diag.get(), im.lu.get(), shift, im.rinv.get(), im.done.get(), im.stamp, im.status.get(), im.fact_cap,
                         im.fact_hcap);
                     im.launches += 1;
                 }
                 if (im.sub_queue > 0) {
                     kern<<<im.grid_fact, im.fact_warps * kWarp, im.fact_smem, s>>>(
                         im.sub_queue, im.rp.get(), im.ci.get(), im.diag.get(), im.order_fact.get(), im.lu.get(), shift,
-                        im.done.get(), im.stamp, im.counters.get(), im.status.get(), im.fact_cap, im.fact_hcap);
+                        im.rinv.get(), im.done.get(), im.stamp, im.counters.get(), im.status.get(), im.fact_cap, im.fact_hcap);
                     im.launches += 1;
                 }
             } else if (!im.fact_line && !im.fact_lane) {
                 kern<<<im.grid_fact, im.fact_warps * kWarp, im.fact_smem, s>>>(
                     n, im.rp.get(), im.ci.get(), im.diag.get(),
-                    im.ticket_order == 1 ? im.order_fact.get() : im.order_l.get(), im.lu.get(), shift, im.done.get(),
+                    im.ticket_order == 1 ? im.order_fact.get() : im.order_l.get(), im.lu.get(), shift, im.rinv.get(), im.done.get(),
                     im.stamp, im.counters.get(), im.status.get(), im.fact_cap, im.fact_hcap);
                 im.launches += 1;
             }

@@ -46,24 +46,6 @@ __host__ __device__ constexpr long long line_factor_at(long long slot, int e) {
     return (slot / 32) * (32 * kLineFactorRow) + (e / 2) * 64 + (slot % 32) * 2 + e % 2;
 }
 
-// 1 / d = hi + lo as line_reciprocal gives it: |hi| <= |1 / d| within an ulp and lo = hi (1 -
-// d hi).  From the 20-bit estimate r0 of rcp.approx by one step of the third-order iteration
-// (Chebyshev), r0 (1 + e + e^2) with e = 1 - d r0: r0 is taken 2^-18 below, so that e > 0 and
-// the truncated series stays below 1 / d (by e^3 < 2^-52); both roundings go towards zero.
-__device__ __forceinline__ void line_pivot_reciprocal(double d, double& hi, double& lo) {
-    double r0;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r0) : "d"(d));
-    r0 = __hiloint2double(__double2hiint(r0) - 4, 0);
-    const double e = fma(-d, r0, 1.0);
-    hi = __fma_rz(r0, __fma_rz(e, e, e), r0);
-    lo = hi * fma(-d, hi, 1.0);
-    const int ex = (__double2hiint(d) >> 20) & 0x7FF;
-    if (ex < 1023 - kLineDivExp || ex > 1023 + kLineDivExp) {
-        hi = __longlong_as_double(0x7FF8000000000000ll);
-        lo = 0.0;
-    }
-}
-
 struct LinePivot {
     double d, hi, lo;
 };

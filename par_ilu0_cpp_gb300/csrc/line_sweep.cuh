@@ -31,7 +31,7 @@
 // FP64 instructions alone take 93 / 155 ns on a scheduler), and a handoff between warps costs
 // two to three steps.  Inside GMRES, forward / backward, us: 128^3 FP32 88 / 83 (151 / 137
 // with a lane's own accesses), FP64 128 / 177 (247 / 622, block-local backward 566); 256^2
-// FP32 43 / 39 (95 / 84), FP64 72 / 121 (204 / block-local 447).
+// FP32 43 / 39 (95 / 84), FP64 72 / 111 (204 / block-local 447).
 //
 // Blocks are taken from a ticket counter in dependency order (anti-diagonals of the block
 // grid), so a block only waits for blocks of smaller tickets, whose CTAs are running or
@@ -44,6 +44,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "division.cuh"
 #include "ilu_kernels.cuh"
 
 namespace gb300 {
@@ -303,44 +304,6 @@ struct LineWait {
         return out;
     }
 };
-
-// ---- FP64 division by a known divisor ----
-// acc / d for the rows of U: GB300 issues one FP64 instruction per warp in 64 cycles on a
-// scheduler, and a division takes about nine of them (566 cycles measured), all on the
-// chain.  With 1/d = hi + lo (hi = 1/d rounded towards zero, lo the remainder, both from
-// the factorisation's packing) the quotient is fma(acc, hi, acc * lo): two instructions
-// (128 cycles), its argument within 2^-51 ulp of the exact quotient, so it is the
-// correctly rounded quotient unless that lies within 2^-51 ulp of the middle between two
-// numbers (double-word reciprocal, as in the literature on division by constants:
-// Brisebarre, Muller, Raina, "Accelerating correctly rounded floating-point division when
-// the divisor is known in advance", IEEE TC 53(8), 2004).  hi and lo have the same sign,
-// so a zero keeps its sign.  Divisors outside 2^+-400 are packed as hi = NaN, and a
-// quotient outside 2^+-600 (or one that is not finite) is divided again.
-constexpr int kLineDivExp = 400;
-constexpr int kLineQuoExp = 600;
-
-__device__ __forceinline__ void line_reciprocal(double d, double& hi, double& lo) {
-    const int e = (__double2hiint(d) >> 20) & 0x7FF;
-    if (e < 1023 - kLineDivExp || e > 1023 + kLineDivExp) {
-        hi = __longlong_as_double(0x7FF8000000000000ll);
-        lo = 0.0;
-        return;
-    }
-    hi = __drcp_rz(d);
-    lo = fma(-d, hi, 1.0) * hi;  // 1 - d hi is exact: both factors have 53 bits, the result < 2^-52
-}
-__device__ __forceinline__ double line_quotient(double acc, double hi, double lo) { return fma(acc, hi, acc * lo); }
-// Whether acc / d must be divided again (integer operations: the FP64 pipe is what the
-// sweep waits for).  0 / d is exact already.
-__device__ __forceinline__ bool line_quotient_bad(float, float) { return false; }
-__device__ __forceinline__ bool line_quotient_bad(double q, double acc) {
-    const unsigned qh = static_cast<unsigned>(__double2hiint(q)), ah = static_cast<unsigned>(__double2hiint(acc));
-    constexpr unsigned kLow = static_cast<unsigned>(1023 - kLineQuoExp) << 21;  // exponent above the sign
-    constexpr unsigned kSpan = static_cast<unsigned>(2 * kLineQuoExp) << 21;
-    const unsigned nonzero = ((qh | ah) << 1) | static_cast<unsigned>(__double2loint(q)) | static_cast<unsigned>(__double2loint(acc));
-    return (qh << 1) - kLow > kSpan && nonzero != 0u;
-}
-static __device__ __noinline__ double line_divide(double acc, const double* d) { return acc / *d; }
 
 // Coefficients of one row in the packed stream: c_z, c_y, c_x and for U the reciprocal.  A
 // step's 32 rows lie together: FP32 four values (16 bytes) per lane; FP64 pairs (c_z, c_y)
