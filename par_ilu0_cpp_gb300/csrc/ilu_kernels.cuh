@@ -390,6 +390,7 @@ __device__ __forceinline__ void progressive_rows(int row, int K, const int (&c)[
                                                  int* status) {
     int k = 0;
     bool done = row < 0;
+    const RowFinish<UPPER, T> finish(d);
     WaitBudget wb;
     while (!__all_sync(0xffffffffu, done)) {
         if (!done) {
@@ -409,9 +410,7 @@ __device__ __forceinline__ void progressive_rows(int row, int K, const int (&c)[
                 }
             }
             if (k >= K) {
-                // FP64: the reference's division; FP32 (mixed path): d holds 1 / u_ii
-                const T r = UPPER ? (sizeof(T) == 8 ? acc / d : acc * d) : acc;
-                st_relaxed(out + row, Sentinel<T>::canon(r));
+                st_relaxed(out + row, Sentinel<T>::canon(finish(acc)));
                 done = true;
             }
         }
@@ -444,6 +443,7 @@ __device__ __forceinline__ void group_rows(int row, int K, int lane, const int (
     T x[kLaneEntries];
 #pragma unroll
     for (int u = 0; u < kLaneEntries; ++u) x[u] = Sentinel<T>::value();
+    const RowFinish<UPPER, T> finish(d);
     int o = 0;  // owner: group position of the first unconsumed entry (G = row done)
     int k = 0;  // next entry of this lane to consume (meaningful in the owner)
     bool done = row < 0;
@@ -478,11 +478,7 @@ __device__ __forceinline__ void group_rows(int row, int K, int lane, const int (
             if (moved) {
                 ++o;
                 if (o == G) {
-                    if (j == 0) {
-                        // FP64: the reference's division; FP32 (mixed path): d holds 1 / u_ii
-                        const T r = UPPER ? (sizeof(T) == 8 ? acc / d : acc * d) : acc;
-                        st_relaxed(out + row, Sentinel<T>::canon(r));
-                    }
+                    if (j == 0) st_relaxed(out + row, Sentinel<T>::canon(finish(acc)));
                     done = true;
                 }
             }
@@ -822,6 +818,7 @@ __device__ __forceinline__ void block_progressive(int row, int K, const int (&c)
                                                   int* status) {
     int k = 0;
     bool done = row < 0;
+    const RowFinish<UPPER, T> finish(d);
     WaitBudget wb;
     while (!__all_sync(0xffffffffu, done)) {
         if (!done) {
@@ -841,8 +838,7 @@ __device__ __forceinline__ void block_progressive(int row, int K, const int (&c)
                 }
             }
             if (k >= K) {
-                // FP64: the reference's division; FP32 (mixed path): d holds 1 / u_ii
-                const T r = Sentinel<T>::canon(UPPER ? (sizeof(T) == 8 ? acc / d : acc * d) : acc);
+                const T r = Sentinel<T>::canon(finish(acc));
                 block_publish(row, r, xs, base, out, remote, remote2, ex);
                 done = true;
             }
