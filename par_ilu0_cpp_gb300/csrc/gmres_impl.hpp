@@ -90,12 +90,14 @@ struct PreconditionedGmres::Impl {
     int grid_spmv = 0, grid_blas = 0, grid_update = 0;
     int grid_blas64 = 0, grid_blas32 = 0;  // resident Gram-Schmidt blocks per value type
 
-    // Gram-Schmidt grid for `nchunks` row chunks of value type T: at most the resident
+    // Gram-Schmidt grid for `nchunks` row chunks of value type T: FP64 a block per chunk up to
+    // the resident blocks (first_chunk); FP32 at most the resident
     // blocks, and no more blocks than needed for every warp to take the same number of
     // chunks (a warp with one chunk more than the others would set the pass's length).
     template <class T>
     int cgs_grid(long long nchunks) const {
         const long long cap = sizeof(T) == 8 ? grid_blas64 : grid_blas32;
+        if (sizeof(T) == 8) return static_cast<int>(std::max<long long>(1, std::min(nchunks, cap)));
         const long long warps = cap * gb300::kBlasWarps;
         const long long per_warp = std::max<long long>(1, (nchunks + warps - 1) / warps);
         const long long g = (nchunks + per_warp * gb300::kBlasWarps - 1) / (per_warp * gb300::kBlasWarps);

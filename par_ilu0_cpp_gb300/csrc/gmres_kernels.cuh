@@ -372,6 +372,19 @@ __device__ __forceinline__ void zero_warp_rows(Acc (*acc_s)[kMaxKrylov + 1], int
     (void)nv;
 }
 
+// First chunk of warp w of this block.  FP64 chunks go round the blocks first, so that every
+// SM's FP64 pipe, which bounds these kernels, has the same work to a chunk: a few chunks
+// (7,500 rows are 30) would else lie on one or two SMs, and 3,375 chunks (100 x 96 x 90) on
+// 106 blocks of 16 warps with two each.  The three kernels of a step, us, before / now (averages
+// over the steps): 100 x 96 x 90 76 / 61, 130 / 102, 70 / 59; 256^2 30 / 18, 48 / 24, 33 / 22;
+// 7,487 rows 24 / 14, 37 / 19, 28 / 19.
+// FP32 blocks take neighbouring chunks (their kernels are bound by memory).
+template <class T>
+__device__ __forceinline__ long long first_chunk(int w) {
+    return sizeof(T) == 8 ? w * static_cast<long long>(gridDim.x) + blockIdx.x
+                          : blockIdx.x * static_cast<long long>(kBlasWarps) + w;
+}
+
 template <class T>
 __global__ void __launch_bounds__(kBlasThreads, kBlasMinBlocks<T>)
     cgs_dot_kernel(long long nchunks, long long ld, const T* __restrict__ V, int s, double* partial, double* h1,
@@ -386,8 +399,7 @@ __global__ void __launch_bounds__(kBlasThreads, kBlasMinBlocks<T>)
     const int nv = s + 1;
     zero_warp_rows(acc_s, nv);
     const T* wvec = V + static_cast<long long>(s + 1) * ld;
-    for (long long c = blockIdx.x * static_cast<long long>(kBlasWarps) + w; c < nchunks;
-         c += static_cast<long long>(gridDim.x) * kBlasWarps) {
+    for (long long c = first_chunk<T>(w); c < nchunks; c += static_cast<long long>(gridDim.x) * kBlasWarps) {
         const long long r0 = c * R + lane * RPL;
         T a[RPL];
         load_rpl<T, RPL>(wvec + r0, a);
@@ -417,8 +429,7 @@ __global__ void __launch_bounds__(kBlasThreads, kBlasMinBlocks<T>)
     for (int j = threadIdx.x; j < nv; j += blockDim.x) sh[j] = static_cast<Acc>(__ldcg(h1 + j));
     zero_warp_rows(acc_s, nv);
     T* wvec = V + static_cast<long long>(s + 1) * ld;
-    for (long long c = blockIdx.x * static_cast<long long>(kBlasWarps) + w; c < nchunks;
-         c += static_cast<long long>(gridDim.x) * kBlasWarps) {
+    for (long long c = first_chunk<T>(w); c < nchunks; c += static_cast<long long>(gridDim.x) * kBlasWarps) {
         const long long r0 = c * R + lane * RPL;
         T a[RPL];
         Acc x[RPL];
@@ -526,8 +537,7 @@ __global__ void __launch_bounds__(kBlasThreads, kBlasMinBlocks<T>)
     __syncthreads();
     T* wv = V + static_cast<long long>(s + 1) * ld;
     double ss = 0.0;
-    for (long long c = blockIdx.x * static_cast<long long>(kBlasWarps) + w; c < nchunks;
-         c += static_cast<long long>(gridDim.x) * kBlasWarps) {
+    for (long long c = first_chunk<T>(w); c < nchunks; c += static_cast<long long>(gridDim.x) * kBlasWarps) {
         const long long r0 = c * R + lane * RPL;
         T a[RPL];
         Acc x[RPL];

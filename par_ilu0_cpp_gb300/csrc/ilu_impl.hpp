@@ -187,7 +187,7 @@ struct IluSolver::Impl {
     int sub_warps = 0;      // warps per subtree CTA
     size_t sub_smem = 0;    // its dynamic shared memory
     // lane-per-row factorisation (factor_lane.cuh) for factors with short rows
-    int factor_kernel = 0;  // 0 automatic, 1 warp per row, 2 lane per row (when the rows qualify)
+    int factor_kernel = 0;  // 0 automatic (line pipeline for stencils), 1 warp per row, 2 lane per row (short rows)
     bool fact_lane = false;
     gb300::DeviceBuffer<int> lf_rows, lf_pub_off, lf_upd_ptr;
     gb300::DeviceBuffer<int2> lf_upd;
@@ -227,7 +227,7 @@ struct IluSolver::Impl {
     int grid_wy = 0;    // requested lanes of a warp along y (0 automatic)
     int grid_by = 0;    // requested warps of a CTA along y (0 automatic)
     int grid_bz = 0;    // requested warps of a CTA along z (0 automatic)
-    int grid_cluster = 1;  // 1: clusters along z of 16, else 8 CTAs; 2 .. 16: at most that many; 0: none
+    int grid_cluster = 1;  // CTAs of a cluster along z, 1: automatic (size_line_launch); 2 .. 16: at most that many; 0: none
     bool sweep_timeline = false;  // record per-block timelines of the line-pipeline sweeps
     bool grid_one_cta_per_sm = false;  // line-pipeline CTAs request enough shared memory to be alone on an SM
     // line-pipeline sweeps in use per value type (bit 0: forward, bit 1: backward); in
