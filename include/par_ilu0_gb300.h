@@ -104,7 +104,7 @@ enum {
     LLJBASH_ILU_OPT_GRID = 6,
     /* shape of the line-pipeline sweeps (0 = automatic), next IluSolverSetup: lanes of a
      * warp along y (1, 4, 8; the rest along z; 2-D grids use 1), warps of a CTA along y
-     * and along z (at most 8 warps in all). */
+     * and along z (at most 4 compute warps in all). */
     LLJBASH_ILU_OPT_GRID_WARP_Y = 7,
     LLJBASH_ILU_OPT_GRID_CTA_Y = 8,
     LLJBASH_ILU_OPT_GRID_CTA_Z = 9,
@@ -118,14 +118,17 @@ enum {
      * IluSolverSetup. */
     LLJBASH_ILU_OPT_TICKET_ORDER = 11,
     /* factorisation kernel (results are the same for every choice): 0 (default,
-     * automatic) and 1: one warp per row; 2: one lane per row when no row has more than
+     * automatic): the line pipeline for 7- / 5-point stencils in natural order (when
+     * LLJBASH_ILU_OPT_GRID allows it and the ticket order is 0), else one warp per row;
+     * 1: one warp per row; 2: one lane per row when no row has more than
      * 16 entries (each finished row publishes u_kk and its upper entries, rows waiting for
      * it poll exactly those values), else one warp per row.  Next IluSolverSetup. */
     LLJBASH_ILU_OPT_FACTOR_KERNEL = 12,
-    /* line-pipeline sweeps in thread-block clusters of 8 CTAs along z, the handoffs inside
-     * a cluster through distributed shared memory: 1 (default) clusters of 16 CTAs, else
-     * of 8, where such clusters can be scheduled; 2 .. 16 clusters of at most that many
-     * CTAs; 0 never.  Results are the same.  Next IluSolverSetup. */
+    /* line-pipeline kernels in thread-block clusters along z, the handoffs inside a cluster
+     * through distributed shared memory: 1 (default) the largest of 16, 8, 4 and 2 CTAs of
+     * which all clusters are resident at once, for larger grids a size per kernel; 2 .. 16
+     * clusters of at most that many CTAs; 0 never.  Results are the same.  Next
+     * IluSolverSetup. */
     LLJBASH_ILU_OPT_GRID_CLUSTER = 13,
     /* 1: record a per-block timeline of every line-pipeline sweep (read with
      * LLJBASH_IluSolverGetSweepTimeline); 0 (default) off.  Next IluSolverSetup. */
@@ -201,7 +204,7 @@ typedef struct LLJBASH_IluInfo {
     int grid_cta_y;       /* warps of a CTA along y and z */
     int grid_cta_z;
     int grid_blocks;      /* CTA-sized blocks of grid lines */
-    int grid_cluster;     /* CTAs per thread-block cluster of the line-pipeline sweeps, 0: none */
+    int grid_cluster;     /* CTAs per thread-block cluster of the FP64 line-pipeline sweeps, 0: none */
     int factor_subtree_parts; /* ticket order 2: subtree partitions (one CTA each) and their rows */
     int factor_subtree_rows;
 } LLJBASH_IluInfo;
