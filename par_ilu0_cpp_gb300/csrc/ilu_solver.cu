@@ -1042,7 +1042,8 @@ static LineFactorKernel line_factor_kernel(const LineGeom& g, bool cluster) {
     return cluster ? ilu_factor_line_kernel<8, true, true> : ilu_factor_line_kernel<8, true, false>;
 }
 
-// Sets up the line-pipeline factorisation for a grid; false when a CTA cannot be resident.
+// Sets up the line-pipeline factorisation for a grid; false when a CTA cannot be resident or
+// its operand stream does not fit in device memory.
 static bool setup_line_factor(LineFactorPack& G, int nx, int ny, int nz, int max_cluster, const DeviceInfo& dev,
                               cudaStream_t s) {
     if (nx < 3 || ny == 2) return false;  // elimination would change more than the diagonal
@@ -1061,8 +1062,15 @@ static bool setup_line_factor(LineFactorPack& G, int nx, int ny, int nz, int max
     if (G.grid == 0) return false;
     const std::vector<int> order = line_block_order(G.g);
     G.order.upload(order.data(), order.size(), s);
-    G.rows.reserve(static_cast<size_t>(line_factor_at(G.g.slots(), 0)));
-    G.xch.reserve(static_cast<size_t>(3 * G.g.nblk * G.g.xch_block()));
+    try {
+        G.rows.reserve(static_cast<size_t>(line_factor_at(G.g.slots(), 0)));
+        G.xch.reserve(static_cast<size_t>(3 * G.g.nblk * G.g.xch_block()));
+    } catch (const std::runtime_error&) {  // no room for the stream (64 B per row): the other kernels need none
+        cudaGetLastError();
+        G.rows.release();
+        G.xch.release();
+        return false;
+    }
     fill_sentinel(G.xch.get(), static_cast<long long>(G.xch.size()), s, dev.sms);
     GB_CUDA_CHECK(cudaStreamSynchronize(s));  // `order` must outlive the copy
     return true;
