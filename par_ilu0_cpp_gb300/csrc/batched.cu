@@ -757,10 +757,9 @@ __global__ void batch_trial_rhs_kernel(BatchDesc D, int nsys_run) {
 }
 
 template <int G>
-static void launch_batched(int grid, const BatchDesc& D, int nsys_run, int m, cudaStream_t s) {
+static void launch_batched(int grid, const BatchDesc& D, int nsys_run, int m, const DeviceInfo& dev, cudaStream_t s) {
     const size_t smem = group_smem_bytes(m, G);
-    GB_CUDA_CHECK(cudaFuncSetAttribute(batched_ilu_gmres_kernel<G>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       static_cast<int>(smem)));
+    allow_dynamic_smem(reinterpret_cast<const void*>(batched_ilu_gmres_kernel<G>), dev);
     batched_ilu_gmres_kernel<G><<<grid, kBatchThreads, smem, s>>>(D, nsys_run);
 }
 
@@ -827,9 +826,9 @@ float BatchSolver::launch(int ctas_per_sm, bool largest_first, int nsys_run, int
     }
     GB_CUDA_CHECK(cudaEventRecord(ev0_, stream_));
     switch (G) {
-        case 1: launch_batched<1>(grid, D, nsys_run, m_, stream_); break;
-        case 4: launch_batched<4>(grid, D, nsys_run, m_, stream_); break;
-        case 16: launch_batched<16>(grid, D, nsys_run, m_, stream_); break;
+        case 1: launch_batched<1>(grid, D, nsys_run, m_, dev_, stream_); break;
+        case 4: launch_batched<4>(grid, D, nsys_run, m_, dev_, stream_); break;
+        case 16: launch_batched<16>(grid, D, nsys_run, m_, dev_, stream_); break;
         default: throw std::runtime_error("batched: right-hand sides per item must be 1, 4 or 16");
     }
     GB_CUDA_CHECK(cudaGetLastError());

@@ -62,6 +62,18 @@ inline DeviceInfo current_device() {
     return d;
 }
 
+// Lets a kernel be launched with any dynamic shared memory that the device has room for beside
+// its static part; returns that limit.  The limit belongs to the kernel, for every solver and
+// thread of the process: set to what one solver needs, it would refuse the launches of another
+// that needs more.  (What a launch reserves is its own request, so occupancy is unaffected.)
+inline int allow_dynamic_smem(const void* kern, const DeviceInfo& dev) {
+    cudaFuncAttributes attr;
+    GB_CUDA_CHECK(cudaFuncGetAttributes(&attr, kern));
+    const int limit = dev.smem_optin - static_cast<int>(attr.sharedSizeBytes);
+    GB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, limit));
+    return limit;
+}
+
 // Grid of `blocks_per_sm` (or the occupancy limit, whichever is smaller) blocks per SM.
 template <class K>
 int persistent_grid(K kernel, int threads, int sms, int want_per_sm = 64) {

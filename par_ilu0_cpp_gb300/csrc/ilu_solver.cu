@@ -669,8 +669,6 @@ static void gather_block(const BlockPack& P, bool lower, const double* lu, cudaS
     GB_CUDA_CHECK(cudaGetLastError());
 }
 
-// Raises the kernel's dynamic shared-memory limit to the pack's footprint for type T and
-// records the number of resident CTAs.
 // Launch configuration of the cluster variant (clusters of P.cl CTAs along x).
 static cudaLaunchConfig_t cluster_launch_config(const BlockPack& P, int grid, size_t smem, cudaStream_t s,
                                                 cudaLaunchAttribute* attr) {
@@ -688,20 +686,20 @@ static cudaLaunchConfig_t cluster_launch_config(const BlockPack& P, int grid, si
     return cfg;
 }
 
-// Raises the kernel's dynamic shared-memory limit to the pack's footprint and records how
-// many CTAs to launch: the resident CTAs (plain variant) or the resident clusters times
-// the cluster size (cluster variant; 0 when a cluster cannot be scheduled).
+// Records how many CTAs to launch: the resident CTAs (plain variant) or the resident
+// clusters times the cluster size (cluster variant; 0 when a cluster cannot be scheduled).
 template <class T, bool UPPER, int KM, bool FIXED>
-static void configure_block_km(BlockPack& P, int sms) {
+static void configure_block_km(BlockPack& P, const DeviceInfo& dev) {
     const int bytes = static_cast<int>(std::max<size_t>(P.smem, 16));
     if (P.cl) {
         auto* kern = sptrsv_block_cluster_kernel<T, UPPER, KM, FIXED>;
-        GB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+        allow_dynamic_smem(reinterpret_cast<const void*>(kern), dev);
         // clusters above the portable 8 CTAs (clusters of 16: 2% faster 128^3 FP32 sweeps
         // than 8, fewer handoffs through L2); where they cannot be scheduled the
-        // occupancy query below reports 0 and the next schedule candidate is used
-        GB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed,
-                                           P.cl > kBlockCluster ? 1 : 0));
+        // occupancy query below reports 0 and the next schedule candidate is used (never
+        // forbidden again: other solvers' clusters use the same kernel)
+        if (P.cl > kBlockCluster)
+            GB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
         const int nq = ceil_div(P.nblk, P.cl);
         cudaLaunchAttribute attr[1];
         cudaLaunchConfig_t cfg = cluster_launch_config(P, nq * P.cl, static_cast<size_t>(bytes), nullptr, attr);
@@ -713,24 +711,23 @@ static void configure_block_km(BlockPack& P, int sms) {
         P.grid = std::min(nclusters, nq) * P.cl;
         return;
     }
-    GB_CUDA_CHECK(cudaFuncSetAttribute(sptrsv_block_kernel<T, UPPER, KM, FIXED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       bytes));
+    allow_dynamic_smem(reinterpret_cast<const void*>(sptrsv_block_kernel<T, UPPER, KM, FIXED>), dev);
     int per_sm = 0;
     GB_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sptrsv_block_kernel<T, UPPER, KM, FIXED>, P.threads,
                                                                static_cast<size_t>(bytes)));
-    P.grid = std::max(1, per_sm) * sms;
+    P.grid = std::max(1, per_sm) * dev.sms;
 }
 
 template <class T, bool UPPER>
-static void configure_block(BlockPack& P, int sms) {
+static void configure_block(BlockPack& P, const DeviceInfo& dev) {
     if (P.stride == 3)
-        configure_block_km<T, UPPER, 3, true>(P, sms);
+        configure_block_km<T, UPPER, 3, true>(P, dev);
     else if (P.stride == 4)
-        configure_block_km<T, UPPER, 4, true>(P, sms);
+        configure_block_km<T, UPPER, 4, true>(P, dev);
     else if (P.stride == kLaneEntries)
-        configure_block_km<T, UPPER, kLaneEntries, true>(P, sms);
+        configure_block_km<T, UPPER, kLaneEntries, true>(P, dev);
     else
-        configure_block_km<T, UPPER, kLaneEntries, false>(P, sms);
+        configure_block_km<T, UPPER, kLaneEntries, false>(P, dev);
 }
 
 template <class T, bool UPPER, int KM, bool FIXED>
@@ -913,8 +910,8 @@ static const void* line_kernel_ptr(const LineGeom& g, bool cluster, bool upper) 
                  : reinterpret_cast<const void*>(line_kernel<T, false>(g, cluster));
 }
 
-// Sizes the launch of line kernels of geometry g with `smem` bytes of dynamic shared memory
-// (raising their limit): chooses g.cl and returns the CTAs to launch, 0 when a CTA cannot be
+// Sizes the launch of line kernels of geometry g with `smem` bytes of dynamic shared
+// memory: chooses g.cl and returns the CTAs to launch, 0 when a CTA cannot be
 // resident.  With `max_cluster` 1 (automatic) clusters along z of the largest of 16
 // (non-portable), 8, 4 and 2 CTAs of which all are resident at once, or else of at most
 // `most`; with 2 .. 16, clusters of at most that many CTAs; with 0, none.  `wait_lines`:
@@ -924,7 +921,7 @@ static int size_line_launch(LineGeom& g, int threads, size_t smem, int max_clust
                             const std::vector<const void*>& clustered, const std::vector<const void*>& plain,
                             const DeviceInfo& dev) {
     auto prepare = [&](const void* kern, int cl) {
-        GB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+        allow_dynamic_smem(kern, dev);
         if (cl > 8) GB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     };
     g.cl = 0;
@@ -1419,11 +1416,11 @@ void IluSolver::SetupMatrix() {
                 build_block_pack(n, rp, ci, im.an.diag, false, B, elem, budget, cl, ub, s);
                 if (!(lb.fits && ub.fits)) continue;
                 if (elem == 8) {
-                    configure_block<double, false>(lb, im.dev.sms);
-                    configure_block<double, true>(ub, im.dev.sms);
+                    configure_block<double, false>(lb, im.dev);
+                    configure_block<double, true>(ub, im.dev);
                 } else {
-                    configure_block<float, false>(lb, im.dev.sms);
-                    configure_block<float, true>(ub, im.dev.sms);
+                    configure_block<float, false>(lb, im.dev);
+                    configure_block<float, true>(ub, im.dev);
                 }
                 if (lb.grid > 0 && ub.grid > 0) {
                     ok = true;
@@ -1503,8 +1500,7 @@ void IluSolver::SetupMatrix() {
         im.fact_pre = maxup > 2 * kWarp ? 8 : 2;
         im.fact_smem = static_cast<size_t>(warps * warp_bytes(cap));
         auto kern = im.fact_pre == 8 ? ilu_factor_kernel<8> : ilu_factor_kernel<2>;
-        GB_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           static_cast<int>(im.fact_smem)));
+        allow_dynamic_smem(reinterpret_cast<const void*>(kern), im.dev);
         int per_sm = 0;
         GB_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, warps * kWarp, im.fact_smem));
         im.grid_fact = std::max(1, per_sm) * im.dev.sms;
@@ -1566,8 +1562,7 @@ void IluSolver::SetupMatrix() {
         const size_t per_warp = im.fact_smem / static_cast<size_t>(im.fact_warps);
         im.sub_warps = std::max(1, std::min<int>(kSubtreeWarps, static_cast<int>(kFactSmemMax / per_warp)));
         im.sub_smem = per_warp * static_cast<size_t>(im.sub_warps);
-        GB_CUDA_CHECK(cudaFuncSetAttribute(sk, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           static_cast<int>(im.sub_smem)));
+        allow_dynamic_smem(reinterpret_cast<const void*>(sk), im.dev);
     }
     // Level-ordered kernels: warps draw tasks in level order and spin on the rows they
     // depend on.  Rows of one lane poll in rounds and want many warps ahead (1,216 warps
