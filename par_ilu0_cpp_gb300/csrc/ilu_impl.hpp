@@ -116,7 +116,7 @@ struct LinePack {
     int smem_floor = 0;  // dynamic shared memory requested at least (bytes; one CTA per SM)
     DeviceBuffer<int> order;   // [nblk] block of each ticket
     DeviceBuffer<T> l, u;      // operand streams
-    DeviceBuffer<T> lo, div;   // [slots] FP64 U: low part of the reciprocals, diagonal
+    DeviceBuffer<T> div;       // [slots] FP64 U: diagonal
     // Faces handed over through L2, at the sentinel between launches: [0] for the sweeps of
     // GMRES and Substitute (one stream at a time, as their ticket counters), [1] (FP64) for
     // the allocation-free entry point, which may run beside them.
@@ -131,7 +131,6 @@ struct LinePack {
         p.order = order.get();
         p.tl = tl[upper ? 1 : 0].get();
         p.coef = upper ? u.get() : l.get();
-        p.rlo = lo.get();
         p.div = div.get();
         p.xch = xch[set].get();
         return p;
@@ -196,7 +195,7 @@ struct IluSolver::Impl {
     int lf_ntask = 0, grid_lane_fact = 0;
     gb300::DeviceBuffer<double> lu;
     gb300::DeviceBuffer<double> shift;      // per-row diagonal shift (learned), optional
-    gb300::DeviceBuffer<double2> rinv;      // per-row reciprocal of the pivot in two parts (warp per row)
+    gb300::DeviceBuffer<double2> rinv;      // per-row reciprocal of the pivot and the pivot (warp per row)
     gb300::DeviceBuffer<int> done;          // per-row ready stamps of the factorisation
     gb300::DeviceBuffer<unsigned> counters;  // ticket counters [0] fact, [1] L, [2] U
     gb300::DeviceBuffer<int> status;         // StatusWord array

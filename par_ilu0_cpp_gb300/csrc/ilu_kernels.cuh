@@ -74,9 +74,9 @@ __device__ __forceinline__ bool gate_closed(const int* gate, int step) {
 // costs the elimination of the last few pivots, not of all of them.  1 / u_kk and the
 // strict-upper entries of the next pivot row (PRE per lane: 2, or 8 for matrices whose rows
 // have more than 64 entries above the diagonal) are loaded into registers while the current
-// pivot is eliminated, if that is ready.  A finished row leaves the two-part reciprocal of its
-// pivot (rinv), so that the sequential chain per pivot is two FP64 instructions instead of
-// a division, and a shared-memory search-and-update.  Factorisations, ms, with all pivots
+// pivot is eliminated, if that is ready.  A finished row leaves the reciprocal of its pivot
+// (rinv), so that the sequential chain per pivot is three FP64 instructions instead of a
+// division, and a shared-memory search-and-update.  Factorisations, ms, with all pivots
 // awaited first and a division each / now: 27-point ILU(2) of 30 x 27 x 25 41.4 / 2.7,
 // ILU(1) of 44 x 40 x 42 18.5 / 3.9, ILU(0) of 60^3 7.6 / 2.3; 7-point ILU(1) of 64^3 4.0 /
 // 2.1; 5-point ILU(2) of 300^2 9.3 / 4.2.  The update position of a column in row j is found by binary
@@ -224,11 +224,11 @@ __device__ __forceinline__ void ilu_factor_row(int j, const int* __restrict__ rp
             loaded = t + 1 < ready;
             if (loaded) load_pivot(t + 1);
             const double a = sval[t];
-            double l = line_quotient(a, r.x, r.y);
+            double l = line_quotient(a, r.y, r.x);
             int pos[PRE];  // (looked up while the quotient is computed)
 #pragma unroll
             for (int u = 0; u < PRE; ++u) pos[u] = cc[u] >= 0 ? locate(cc[u], t) : -1;
-            if (line_quotient_bad(l, a)) l = a / __ldcg(lu + skd[t]);
+            if (line_quotient_bad(l, a)) l = line_divide(a, r.y);
             if (lane == 0) lu[b + t] = l;
 #pragma unroll
             for (int u = 0; u < PRE; ++u)
@@ -241,9 +241,7 @@ __device__ __forceinline__ void ilu_factor_row(int j, const int* __restrict__ rp
             __syncwarp();
         }
         for (int t = dloc + lane; t < len; t += kWarp) lu[b + t] = sval[t];
-        double2 r;
-        line_pivot_reciprocal(sval[dloc], r.x, r.y);
-        if (lane == 0) rinv[j] = r;
+        if (lane == 0) rinv[j] = make_double2(line_pivot_reciprocal(sval[dloc]), sval[dloc]);
         if (WAIT) {
             __threadfence();
             __syncwarp();
@@ -278,9 +276,8 @@ __device__ __forceinline__ void ilu_factor_row(int j, const int* __restrict__ rp
             }
             __syncwarp();
         }
-        double2 r;
-        line_pivot_reciprocal(__ldcg(val + dloc), r.x, r.y);
-        if (lane == 0) rinv[j] = r;
+        const double pivot = __ldcg(val + dloc);
+        if (lane == 0) rinv[j] = make_double2(line_pivot_reciprocal(pivot), pivot);
         if (WAIT) {
             __threadfence();
             __syncwarp();

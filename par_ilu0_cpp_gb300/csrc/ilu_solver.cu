@@ -995,10 +995,7 @@ static bool configure_line(LinePack<T>& G, const DeviceInfo& dev, int max_cluste
     const size_t slots = static_cast<size_t>(G.g.slots());
     G.l.reserve(slots / 32 * line_step_values<T, false>());
     G.u.reserve(slots / 32 * line_step_values<T, true>());
-    if (sizeof(T) == 8) {
-        G.lo.reserve(slots);
-        G.div.reserve(slots);
-    }
+    if (sizeof(T) == 8) G.div.reserve(slots);
     return true;
 }
 
@@ -1009,8 +1006,8 @@ static int pack_line(LinePack<T>& G, int sweeps, const int* rp, const int* diag,
     const long long slots = G.g.slots();
     const int threads = 256;
     const int grid = static_cast<int>(std::max<long long>(1, std::min<long long>(ceil_div<long long>(slots, threads), 8LL * sms)));
-    if (sweeps & 1) line_pack_kernel<T, false><<<grid, threads, 0, s>>>(G.g, rp, diag, lu, G.l.get(), nullptr, nullptr);
-    if (sweeps & 2) line_pack_kernel<T, true><<<grid, threads, 0, s>>>(G.g, rp, diag, lu, G.u.get(), G.lo.get(), G.div.get());
+    if (sweeps & 1) line_pack_kernel<T, false><<<grid, threads, 0, s>>>(G.g, rp, diag, lu, G.l.get(), nullptr);
+    if (sweeps & 2) line_pack_kernel<T, true><<<grid, threads, 0, s>>>(G.g, rp, diag, lu, G.u.get(), G.div.get());
     GB_CUDA_CHECK(cudaGetLastError());
     return (sweeps & 1) + (sweeps >> 1);
 }
@@ -1061,7 +1058,7 @@ static bool setup_line_factor(LineFactorPack& G, int nx, int ny, int nz, int max
     G.order.upload(order.data(), order.size(), s);
     try {
         G.rows.reserve(static_cast<size_t>(line_factor_at(G.g.slots(), 0)));
-        G.xch.reserve(static_cast<size_t>(3 * G.g.nblk * G.g.xch_block()));
+        G.xch.reserve(static_cast<size_t>(kLinePivotParts * G.g.nblk * G.g.xch_block()));
     } catch (const std::runtime_error&) {  // no room for the stream (64 B per row): the other kernels need none
         cudaGetLastError();
         G.rows.release();

@@ -12,10 +12,10 @@
 // by bulk copies.
 //
 // What bounds it: the FP64 instructions of a row on one scheduler (64 cycles each, whatever
-// the lanes).  A division takes nine; here a row computes the two-part reciprocal of its own
-// pivot once (five, line_pivot_reciprocal) and hands it on with the pivot, so each of the
-// quotients takes two (line_quotient) and a 3-D row 14 instructions, 900 cycles, of which
-// eight lie on the chain along x.  The results are written to the operand stream, coalesced
+// the lanes).  A division takes nine; here a row computes the reciprocal of its own pivot once
+// (four, line_pivot_reciprocal) and hands it on with the pivot, so each of the quotients takes
+// three (line_quotient) and a 3-D row 16 instructions, 1024 cycles, of which eight lie on the
+// chain along x.  The results are written to the operand stream, coalesced
 // (a lane's rows lie a line apart in the CSR values: 32 sectors per entry), and a second
 // kernel takes them to the CSR values.  The warp-per-row kernel pays an L2 handoff and a
 // division chain per level.  Whole factorisations (packs of the sweeps included), ms, before
@@ -30,6 +30,7 @@ namespace gb300 {
 constexpr int kLineFactorWarps = 2;  // compute warps per CTA
 constexpr int kLineFactorRow = 8;    // staged values per row: a_ii, a_iz, a_iy, a_ix, a_zi, a_yi, a_xi, unused;
                                      // on return d_i, l_iz, l_iy, l_ix
+constexpr int kLinePivotParts = 2;   // values handed on per row: the pivot and its reciprocal
 constexpr int kLineFactorSlots = 3;
 constexpr int kLineFactorPolls = 16;  // (about 1 us)
 
@@ -37,7 +38,7 @@ struct LineFactor {
     LineGeom g;
     const int* order = nullptr;      // blocks (clusters) by ticket, as LineTri
     double* rows = nullptr;          // operand stream, line_factor_at
-    double* xch = nullptr;           // [nblk][3][xch_block()]: pivots, high and low reciprocals
+    double* xch = nullptr;           // [nblk][kLinePivotParts][xch_block()]
 };
 
 // Value e of a slot in the operand stream: a step's 32 rows lie together, four 16-byte parts
@@ -47,26 +48,26 @@ __host__ __device__ constexpr long long line_factor_at(long long slot, int e) {
 }
 
 struct LinePivot {
-    double d, hi, lo;
+    double d, z;  // z: its reciprocal
 };
 
 __device__ __forceinline__ bool line_late(const LinePivot& y, const LinePivot& z) {
-    return line_late(y.d, z.d) || line_late(y.hi, z.hi) || line_late(y.lo, z.lo);
+    return line_late(y.d, z.d) || line_late(y.z, z.z);
 }
 
-// Shared memory: per compute warp the staged rows; the three faces of every warp; the
+// Shared memory: per compute warp the staged rows; the faces of every warp; the
 // idle area; mbarriers (staged, computed) per warp and slot.
 __host__ __device__ inline long long line_factor_stage() {
     return static_cast<long long>(kLineFactorSlots) * kLineChunk * 32 * kLineFactorRow;
 }
 __host__ __device__ inline long long line_factor_bar_offset(const LineGeom& g) {
-    return (((g.nw() * (line_factor_stage() + 3ll * (g.face_y() + g.face_z())) + kLineIdle) * 8) + 15) & ~15ll;
+    return (((g.nw() * (line_factor_stage() + kLinePivotParts * (g.face_y() + g.face_z())) + kLineIdle) * 8) + 15) & ~15ll;
 }
 __host__ __device__ inline long long line_factor_smem_bytes(const LineGeom& g) {
     return line_factor_bar_offset(g) + 2ll * g.nw() * kLineFactorSlots * 8;
 }
 struct LineFactorSmem {
-    double *stage, *face_y, *face_z, *idle;  // faces: [warp][3][face]
+    double *stage, *face_y, *face_z, *idle;  // faces: [warp][kLinePivotParts][face]
     unsigned long long* bar;
     __device__ __forceinline__ double* slot(int w, int k) const {
         return stage + (w * kLineFactorSlots + k % kLineFactorSlots) * (kLineChunk * 32 * kLineFactorRow);
@@ -81,13 +82,13 @@ __device__ __forceinline__ LineFactorSmem line_factor_smem(const LineGeom& g, un
     LineFactorSmem m;
     m.stage = reinterpret_cast<double*>(base);
     m.face_y = m.stage + g.nw() * line_factor_stage();
-    m.face_z = m.face_y + 3ll * g.nw() * g.face_y();
-    m.idle = m.face_z + 3ll * g.nw() * g.face_z();
+    m.face_z = m.face_y + static_cast<long long>(kLinePivotParts) * g.nw() * g.face_y();
+    m.idle = m.face_z + static_cast<long long>(kLinePivotParts) * g.nw() * g.face_z();
     m.bar = reinterpret_cast<unsigned long long*>(base + line_factor_bar_offset(g));
     return m;
 }
 
-// One compute warp's rows of block `blk`.  to_y / to_z: the three faces (face_y() / face_z()
+// One compute warp's rows of block `blk`.  to_y / to_z: the faces (face_y() / face_z()
 // values apart) that its last lanes along y / z fill.
 template <int WY, bool D3>
 __device__ __forceinline__ void line_factor_compute(const LineFactor& P, int blk, int w, const LineFactorSmem& M, double* to_y,
@@ -104,8 +105,8 @@ __device__ __forceinline__ void line_factor_compute(const LineFactor& P, int blk
     const int nchunk = g.psteps / C;
     const int ylen = g.face_y(), zlen = g.face_z();
     const unsigned idle = shared_addr(M.idle);
-    unsigned fy = y_edge ? shared_addr(M.face_y + 3ll * w * ylen + shift * WZ + zz) : idle;
-    unsigned fz = z_edge ? shared_addr(M.face_z + 3ll * w * zlen + shift * WY + yy) : idle;
+    unsigned fy = y_edge ? shared_addr(M.face_y + static_cast<long long>(kLinePivotParts) * w * ylen + shift * WZ + zz) : idle;
+    unsigned fz = z_edge ? shared_addr(M.face_z + static_cast<long long>(kLinePivotParts) * w * zlen + shift * WY + yy) : idle;
     const unsigned fy_adv = y_edge ? WZ * Z : 0u, fz_adv = z_edge ? WY * Z : 0u;
     const unsigned fy_comp = y_edge ? ylen * Z : 0u, fz_comp = z_edge ? zlen * Z : 0u;
     const bool has_y = D3 && to_y != nullptr && yy == WY - 1;
@@ -116,7 +117,7 @@ __device__ __forceinline__ void line_factor_compute(const LineFactor& P, int blk
 
     // operands and faces one step ahead
     double v[kLineFactorRow];
-    LinePivot prev{1.0, 1.0, 0.0};  // the previous row of the line (none: its coefficient is 0)
+    LinePivot prev{1.0, 1.0};  // the previous row of the line (none: its coefficient is 0)
     LinePivot sy = prev, sz = prev, fyv{}, fzv{};
     auto load = [&](unsigned a) {
 #pragma unroll
@@ -130,18 +131,15 @@ __device__ __forceinline__ void line_factor_compute(const LineFactor& P, int blk
     };
     auto face = [&](unsigned a, unsigned comp, LinePivot& f) {
         lds_polled(a, f.d);
-        lds_polled(a + comp, f.hi);
-        lds_polled(a + 2 * comp, f.lo);
+        lds_polled(a + comp, f.z);
     };
     auto shuffle = [&](const LinePivot& p, LinePivot& y, LinePivot& z) {
         if (D3 && WY > 1) {
             y.d = __shfl_up_sync(0xffffffffu, p.d, 1);
-            y.hi = __shfl_up_sync(0xffffffffu, p.hi, 1);
-            y.lo = __shfl_up_sync(0xffffffffu, p.lo, 1);
+            y.z = __shfl_up_sync(0xffffffffu, p.z, 1);
         }
         z.d = __shfl_up_sync(0xffffffffu, p.d, WY);
-        z.hi = __shfl_up_sync(0xffffffffu, p.hi, WY);
-        z.lo = __shfl_up_sync(0xffffffffu, p.lo, WY);
+        z.z = __shfl_up_sync(0xffffffffu, p.z, WY);
     };
     mbar_wait(M.full(w, 0), 0u, status);
     __syncwarp();
@@ -171,10 +169,10 @@ __device__ __forceinline__ void line_factor_compute(const LineFactor& P, int blk
         LinePivot np, ny, nz;
         double lz, ly = 0.0, lx;
         auto quotient = [&](double a, const LinePivot& p, bool exact, bool& bad) {
-            double l = line_quotient(a, p.hi, p.lo);
+            double l = line_quotient(a, p.d, p.z);
             if (line_quotient_bad(l, a)) {
                 bad = true;
-                if (exact) l = line_divide(a, &p.d);
+                if (exact) l = line_divide(a, p.d);
             }
             return l;
         };
@@ -188,7 +186,7 @@ __device__ __forceinline__ void line_factor_compute(const LineFactor& P, int blk
             }
             lx = quotient(v[3], prev, exact, bad);
             np.d = fma(-v[6], lx, np.d);
-            line_pivot_reciprocal(np.d, np.hi, np.lo);
+            np.z = line_pivot_reciprocal(np.d);
             return bad;
         };
         const bool bad = solve(false);
@@ -196,8 +194,8 @@ __device__ __forceinline__ void line_factor_compute(const LineFactor& P, int blk
         if (late) {
             if (!wait.expired(status)) continue;
             // give up: zeros in place of what did not arrive
-            if (line_late(fyv, fyv)) fyv = LinePivot{0.0, 0.0, 0.0};
-            if (line_late(fzv, fzv)) fzv = LinePivot{0.0, 0.0, 0.0};
+            if (line_late(fyv, fyv)) fyv = LinePivot{0.0, 0.0};
+            if (line_late(fzv, fzv)) fzv = LinePivot{0.0, 0.0};
             __syncwarp();
             continue;
         }
@@ -214,16 +212,14 @@ __device__ __forceinline__ void line_factor_compute(const LineFactor& P, int blk
         sy = ny;
         sz = nz;
         // only the stored copies, which others poll, are kept off the sentinel
-        const double pd = off_sentinel(np.d), ph = off_sentinel(np.hi), pl = off_sentinel(np.lo);
+        const double pd = off_sentinel(np.d), pz_out = off_sentinel(np.z);
         if (D3) {
             st_relaxed_generic(has_y, oy, pd);
-            st_relaxed_generic(has_y, oy + ylen, ph);
-            st_relaxed_generic(has_y, oy + 2 * ylen, pl);
+            st_relaxed_generic(has_y, oy + ylen, pz_out);
             oy += WZ;
         }
         st_relaxed_generic(has_z, oz, pd);
-        st_relaxed_generic(has_z, oz + zlen, ph);
-        st_relaxed_generic(has_z, oz + 2 * zlen, pl);
+        st_relaxed_generic(has_z, oz + zlen, pz_out);
         oz += WY;
         row += kStep;
         if (--left == 0) {
@@ -252,23 +248,24 @@ __device__ __forceinline__ void line_factor_block(const LineFactor& P, int blk, 
     const int nw = g.nw();
     const int w = threadIdx.x >> 5;
     const int iy = blk % g.nby, iz = blk / g.nby;
-    const long long xb = 3 * g.xch_block();
+    constexpr long long parts = kLinePivotParts;
+    const long long xb = parts * g.xch_block();
     if (w < nw) {
         const int wyi = w % g.by, wzi = w / g.by;
         double* to_y = nullptr;
         double* to_z = nullptr;
         if (D3) {
             if (wyi + 1 < g.by)
-                to_y = M.face_y + 3ll * (w + 1) * g.face_y();
+                to_y = M.face_y + parts * (w + 1) * g.face_y();
             else if (iy + 1 < g.nby)
-                to_y = P.xch + (blk + 1) * xb + 3ll * wzi * g.face_y();
+                to_y = P.xch + (blk + 1) * xb + parts * wzi * g.face_y();
         }
         if (wzi + 1 < g.bz)
-            to_z = M.face_z + 3ll * (w + g.by) * g.face_z();
+            to_z = M.face_z + parts * (w + g.by) * g.face_z();
         else if (next_z != nullptr)
-            to_z = next_z + 3ll * wyi * g.face_z();
+            to_z = next_z + parts * wyi * g.face_z();
         else if (iz + 1 < g.nbz)
-            to_z = P.xch + (blk + g.nby) * xb + 3ll * g.bz * g.face_y() + 3ll * wyi * g.face_z();
+            to_z = P.xch + (blk + g.nby) * xb + parts * g.bz * g.face_y() + parts * wyi * g.face_z();
         line_factor_compute<WY, D3>(P, blk, w, M, to_y, to_z, status);
     } else if (w < 2 * nw) {  // helper: bulk copies of the staged rows
         const int cw = w - nw;
@@ -288,32 +285,32 @@ __device__ __forceinline__ void line_factor_block(const LineFactor& P, int blk, 
             __syncwarp();
         }
     } else {
-        // halo warps: the three components of a face one after the other, a warp each for
+        // halo warps: the components of a face one after the other, a warp each for
         // y and z would wait for the first to end; so each component has its own warp
         const int h = w - 2 * nw;
-        const int comp = h % 3;
-        if (h < 3) {
-            double* const x = P.xch + blk * xb + 3ll * g.bz * g.face_y() + static_cast<long long>(comp) * g.face_z();
+        const int comp = h % kLinePivotParts;
+        if (h < kLinePivotParts) {
+            double* const x = P.xch + blk * xb + parts * g.bz * g.face_y() + static_cast<long long>(comp) * g.face_z();
             if (iz > 0 && z_from_l2)
-                line_halo(x, M.face_z + static_cast<long long>(comp) * g.face_z(), 3 * g.face_z(), 1, g.by, WY, g.pad(), g.nx, status);
+                line_halo(x, M.face_z + static_cast<long long>(comp) * g.face_z(), kLinePivotParts * g.face_z(), 1, g.by, WY, g.pad(), g.nx, status);
         } else if (D3) {
             double* const x = P.xch + blk * xb + static_cast<long long>(comp) * g.face_y();
             if (iy > 0)
-                line_halo(x, M.face_y + static_cast<long long>(comp) * g.face_y(), 3 * g.face_y(), g.by, g.bz, 32 / WY, g.pad(), g.nx,
+                line_halo(x, M.face_y + static_cast<long long>(comp) * g.face_y(), kLinePivotParts * g.face_y(), g.by, g.bz, 32 / WY, g.pad(), g.nx,
                           status);
         }
     }
 }
-__host__ __device__ inline int line_factor_threads(const LineGeom& g) { return (2 * g.nw() + (g.ny > 1 ? 6 : 3)) * 32; }
+__host__ __device__ inline int line_factor_threads(const LineGeom& g) { return (2 * g.nw() + (g.ny > 1 ? 2 : 1) * kLinePivotParts) * 32; }
 
 __device__ __forceinline__ void line_factor_reset(const LineGeom& g, int iy, int iz, const LineFactorSmem& M, bool again) {
     const int lane = threadIdx.x & 31;
     const int nwarp = static_cast<int>(blockDim.x >> 5);
     const int nw = g.nw();
-    for (int f = static_cast<int>(threadIdx.x >> 5); f < 3 * (g.ny > 1 ? 2 * nw : nw); f += nwarp) {
-        const bool z = f < 3 * nw;
-        const int c = z ? f : f - 3 * nw;  // 3 w + component
-        const int w = c / 3;
+    for (int f = static_cast<int>(threadIdx.x >> 5); f < kLinePivotParts * (g.ny > 1 ? 2 * nw : nw); f += nwarp) {
+        const bool z = f < kLinePivotParts * nw;
+        const int c = z ? f : f - kLinePivotParts * nw;  // kLinePivotParts w + component
+        const int w = c / kLinePivotParts;
         const int width = z ? g.wy : g.wz;
         const int len = z ? g.face_z() : g.face_y();
         double* const p = (z ? M.face_z : M.face_y) + static_cast<long long>(c) * len;
@@ -332,7 +329,7 @@ __device__ __forceinline__ void line_factor_reset(const LineGeom& g, int iy, int
 // Factorises the operand stream in place.  Launched with clusters of g.cl CTAs along z
 // (CLUSTER), or without.
 template <int WY, bool D3, bool CLUSTER>
-__global__ void __launch_bounds__((2 * kLineFactorWarps + 6) * kWarp, 1)
+__global__ void __launch_bounds__((2 * kLineFactorWarps + 2 * kLinePivotParts) * kWarp, 1)
     ilu_factor_line_kernel(LineFactor P, unsigned* counter, int* status) {
     extern __shared__ __align__(16) unsigned char line_smem[];
     const LineFactorSmem M = line_factor_smem(P.g, line_smem);

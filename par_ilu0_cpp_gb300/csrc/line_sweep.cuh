@@ -27,11 +27,11 @@
 // the results in chunks of 8 steps through shared memory: the coefficient stream by bulk
 // copies, right-hand side and results 8 consecutive rows of a line at a time (the first
 // product with `scale` included).  The compute warp touches only staged values, its faces
-// and the shuffles, a step is 70 ns (FP32) or 160 / 235 ns (FP64 forward / backward, whose
-// FP64 instructions alone take 93 / 155 ns on a scheduler), and a handoff between warps costs
-// two to three steps.  Inside GMRES, forward / backward, us: 128^3 FP32 88 / 83 (151 / 137
-// with a lane's own accesses), FP64 128 / 177 (247 / 622, block-local backward 566); 256^2
-// FP32 43 / 39 (95 / 84), FP64 72 / 111 (204 / block-local 447).
+// and the shuffles, a step is 70 ns (FP32) or 160 / 265 ns (FP64 forward / backward, whose
+// FP64 instructions alone take 93 / 186 ns on a scheduler), and a handoff between warps costs
+// two to three steps.  Inside GMRES, forward / backward, us: 128^3 FP32 87 / 84 (151 / 137
+// with a lane's own accesses), FP64 128 / 194 (247 / 622, block-local backward 566); 256^2
+// FP32 44 / 39 (95 / 84), FP64 71 / 123 (204 / block-local 447).
 //
 // Blocks are taken from a ticket counter in dependency order (anti-diagonals of the block
 // grid), so a block only waits for blocks of smaller tickets, whose CTAs are running or
@@ -95,11 +95,9 @@ struct LineTri {
     LineGeom g;
     const int* order = nullptr;  // [nblk] block (iy + nby iz, sweep coordinates) of each ticket;
                                  // with clusters [nby nbzc]: cluster (iy + nby izc) of each ticket
-    const T* coef = nullptr;     // per slot c_z, c_y, c_x, and for U the reciprocal of u_ii
-                                 // (FP32: RN(1 / u_ii); FP64: its high part, see line_quotient),
+    const T* coef = nullptr;     // per slot c_z, c_y, c_x, and for U the reciprocal RN(1 / u_ii),
                                  // in the order of line_coef_at
-    const T* rlo = nullptr;      // FP64 U: [slots] low part of the reciprocal
-    const T* div = nullptr;      // FP64 U: [slots] u_ii
+    const T* div = nullptr;      // FP64 U: [slots] u_ii (line_quotient)
     T* xch = nullptr;            // [nblk][xch_block()] faces handed over through L2, at the sentinel
                                  // between launches (in x' in [0, nx))
     unsigned long long* tl = nullptr;  // per-block timeline [nblk][kLineTimeline] (null: off)
@@ -339,7 +337,7 @@ __device__ __forceinline__ void line_load_coef(unsigned a, int lane, LineCoef<do
 }
 
 // Shared memory of a CTA: per compute warp and slot a chunk of the coefficient stream
-// (and for FP64 of the low reciprocals) and its right-hand side [lane][kLinePitch]; per
+// (and for FP64 of the divisors) and its right-hand side [lane][kLinePitch]; per
 // compute warp a ring of kLineSlots + 1 chunks of results [lane][kLinePitch]; then the faces (consumer-indexed: slot w holds what warp w reads;
 // y-faces [nw][face_y()], z-faces [nw][face_z()]); then kLineIdle zeros that lanes without
 // a face read and kLineIdle values that lanes without a consumer write (so that no access
@@ -348,9 +346,9 @@ __device__ __forceinline__ void line_load_coef(unsigned a, int lane, LineCoef<do
 template <class T, bool UPPER>
 struct LineStage {
     static constexpr int kCoef = kLineChunk * line_step_values<T, UPPER>();
-    static constexpr int kLo = UPPER && sizeof(T) == 8 ? kLineChunk * 32 : 0;
+    static constexpr int kDiv = UPPER && sizeof(T) == 8 ? kLineChunk * 32 : 0;
     static constexpr int kVec = 32 * kLinePitch<T>;
-    static constexpr int kSlot = kCoef + kLo + kVec;  // a multiple of 16 bytes
+    static constexpr int kSlot = kCoef + kDiv + kVec;  // a multiple of 16 bytes
     static constexpr int kWarp = kLineSlots * kSlot + (kLineSlots + 1) * kVec;
 };
 constexpr int kLineIdle = kLineStepAlign * 32 + 32;  // offsets within a chunk stay inside
@@ -416,7 +414,6 @@ __device__ __forceinline__ bool line_compute(const LineTri<T>& P, int blk, int w
     const bool z_edge = zz == 0;
     constexpr unsigned Z = sizeof(T);
     const unsigned idle = shared_addr(M.idle);
-    const T* div = DIV ? P.div + P.g.slot(blk, w, 0, lane) : nullptr;
     unsigned fy = y_edge ? shared_addr(M.face_y + static_cast<long long>(w) * P.g.face_y() + shift * WZ + zz) : idle;
     unsigned fz = z_edge ? shared_addr(M.face_z + static_cast<long long>(w) * P.g.face_z() + shift * WY + yy) : idle;
     const bool dry = WARM && !line_first_faces<T>(fy, fz) && !wait.expired(status);
@@ -432,17 +429,17 @@ __device__ __forceinline__ bool line_compute(const LineTri<T>& P, int blk, int w
     mbar_wait(M.full(w, 0), 0u, status);
     __syncwarp();
     constexpr int V = 16 / sizeof(T);  // steps per access of the right-hand side and the results
-    constexpr unsigned kLo = St::kCoef * Z, kB = kLo + St::kLo * Z, kStep = line_step_values<T, UPPER>() * Z;
+    constexpr unsigned kDiv = St::kCoef * Z, kB = kDiv + St::kDiv * Z, kStep = line_step_values<T, UPPER>() * Z;
     const unsigned laneZ = lane * Z, laneP = lane * (kLinePitch<T> * Z);
     unsigned row = shared_addr(M.slot(w, 0));
     // operands: coefficients loaded two steps ahead, right-hand side by groups of V steps,
     // faces one step ahead
     LineCoef<T> c[2];
-    T lo[2] = {T(0), T(0)}, bc[V], bn[V], res[V];
+    T d[2] = {T(0), T(0)}, bc[V], bn[V], res[V];
     T pfy = T(0), pfz;
     auto load = [&](unsigned slot, int step, int e) {
         line_load_coef<UPPER>(slot + step * kStep, lane, c[e]);
-        if constexpr (DIV) lds(slot + laneZ + (kLo + step * 32 * Z), lo[e]);
+        if constexpr (DIV) lds(slot + laneZ + (kDiv + step * 32 * Z), d[e]);
     };
     load(row, 0, 0);
     load(row, 1, 1);
@@ -461,7 +458,7 @@ __device__ __forceinline__ bool line_compute(const LineTri<T>& P, int blk, int w
 #pragma unroll
         for (int i = 0; i < C; ++i) {
             const LineCoef<T> q = c[i % 2];
-            const T ql = lo[i % 2], a0 = bc[i % V];
+            const T qd = d[i % 2], a0 = bc[i % V];
             const T fyv = pfy, fzv = pfz;
             // the row, as if every predecessor were there and the quotient final
             T acc;
@@ -469,7 +466,7 @@ __device__ __forceinline__ bool line_compute(const LineTri<T>& P, int blk, int w
                 acc = fma(-q.cz, z_edge ? fz_v : sh_z, a0);
                 if (D3) acc = fma(-q.cy, y_edge ? fy_v : sh_y, acc);
                 acc = fma(-q.cx, prev, acc);
-                if constexpr (DIV) return line_quotient(acc, q.d, ql);  // the reference's division
+                if constexpr (DIV) return line_quotient(acc, qd, q.d);  // the reference's division
                 if constexpr (UPPER) return acc * q.d;
                 return acc;
             };
@@ -494,7 +491,7 @@ __device__ __forceinline__ bool line_compute(const LineTri<T>& P, int blk, int w
                 __syncwarp();
                 r = solve(fy_v, fz_v);
                 if constexpr (DIV) {
-                    if (line_quotient_bad(r, acc)) r = line_divide(acc, div + i * 32);
+                    if (line_quotient_bad(r, acc)) r = line_divide(acc, qd);
                     __syncwarp();
                 }
                 shuffle(r, ny, nz);
@@ -516,7 +513,6 @@ __device__ __forceinline__ bool line_compute(const LineTri<T>& P, int blk, int w
         __syncwarp();
         if (lane == 0 && !dry) mbar_arrive(M.done(w, k));
         row = next;
-        if constexpr (DIV) div += C * 32;
         fy += fy_adv;
         fz += fz_adv;
         oy += oy_adv;
@@ -579,12 +575,12 @@ __device__ __forceinline__ void line_helper(const LineTri<T>& P, int blk, int w,
         unsigned long long* const full = M.full(w, k);
         if (lane == 0) {
             constexpr unsigned cb = St::kCoef * sizeof(T);
-            constexpr unsigned lb = St::kLo * sizeof(T);
-            mbar_arrive_expect(full, cb + lb);
+            constexpr unsigned db = St::kDiv * sizeof(T);
+            mbar_arrive_expect(full, cb + db);
             bulk_load(slot, P.coef + line_coef_at<T, UPPER>(first + static_cast<long long>(k) * C * 32, 0), cb, full);
-            if (lb > 0) bulk_load(slot + St::kCoef, P.rlo + first + static_cast<long long>(k) * C * 32, lb, full);
+            if (db > 0) bulk_load(slot + St::kCoef, P.div + first + static_cast<long long>(k) * C * 32, db, full);
         }
-        T* const b = slot + St::kCoef + St::kLo + q * kLinePitch<T> + i;
+        T* const b = slot + St::kCoef + St::kDiv + q * kLinePitch<T> + i;
 #pragma unroll
         for (int r = 0; r < C; ++r) {
             if (scaled) v[r] = v[r] * sc;
@@ -748,7 +744,7 @@ __device__ __forceinline__ void line_prefetch(const LineTri<T>& P, int blk) {
     const long long s0 = P.g.slot(blk, w, 0, 0);
     const long long n = static_cast<long long>(P.g.psteps) * static_cast<long long>(sizeof(T));
     prefetch_l2_range(P.coef + line_coef_at<T, UPPER>(s0, 0), n * line_step_values<T, UPPER>(), threadIdx.x & 31);
-    if (UPPER && sizeof(T) == 8) prefetch_l2_range(P.rlo + s0, n * 32, threadIdx.x & 31);
+    if (UPPER && sizeof(T) == 8) prefetch_l2_range(P.div + s0, n * 32, threadIdx.x & 31);
 }
 
 // Forward (UPPER = false): out = L^{-1} (scale * in), in rescaled in place when `scale`
@@ -837,11 +833,10 @@ __global__ void __launch_bounds__((2 * kLineMaxWarps + 2) * kWarp, sizeof(T) == 
 // r - nx ny, r - nx, r - 1, each present only inside the grid).  U: c_z, c_y, c_x are the
 // strict-upper entries r + nx ny, r + nx, r + 1 (columns descending) and the reciprocal of
 // u_ii: FP32 RN(1 / u_ii), computed in FP64 and rounded once (as the other FP32 kernels);
-// FP64 in two parts (line_reciprocal), and u_ii itself.  Slots without a row hold zeros.
+// FP64 line_reciprocal, and u_ii itself.  Slots without a row hold zeros.
 template <class T, bool UPPER>
 __global__ void line_pack_kernel(LineGeom g, const int* __restrict__ rp, const int* __restrict__ diag,
-                                 const double* __restrict__ lu, T* __restrict__ dst, T* __restrict__ rlo,
-                                 T* __restrict__ div) {
+                                 const double* __restrict__ lu, T* __restrict__ dst, T* __restrict__ div) {
     const long long total = g.slots();
     const int nw = g.nw();
     for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
@@ -858,7 +853,7 @@ __global__ void line_pack_kernel(LineGeom g, const int* __restrict__ rp, const i
         const int yq = (iy * g.by + wyi) * g.wy + yy;
         const int zq = (iz * g.bz + wzi) * g.wz + zz;
         const int xq = s - (yy + zz);
-        double cz = 0.0, cy = 0.0, cx = 0.0, d = 0.0, lo = 0.0, u = 0.0;
+        double cz = 0.0, cy = 0.0, cx = 0.0, d = 0.0, u = 0.0;
         if (yq < g.ny && zq < g.nz && xq >= 0 && xq < g.nx) {
             const int X = UPPER ? g.nx - 1 - xq : xq;
             const int Y = UPPER ? g.ny - 1 - yq : yq;
@@ -875,20 +870,14 @@ __global__ void line_pack_kernel(LineGeom g, const int* __restrict__ rp, const i
                 if (X < g.nx - 1) cx = lu[p++];
                 if (Y < g.ny - 1) cy = lu[p++];
                 if (Z < g.nz - 1) cz = lu[p++];
-                if (sizeof(T) == 4)
-                    d = 1.0 / u;
-                else
-                    line_reciprocal(u, d, lo);
+                d = sizeof(T) == 4 ? 1.0 / u : line_reciprocal(u);
             }
         }
         dst[line_coef_at<T, UPPER>(i, 0)] = static_cast<T>(cz);
         dst[line_coef_at<T, UPPER>(i, 1)] = static_cast<T>(cy);
         dst[line_coef_at<T, UPPER>(i, 2)] = static_cast<T>(cx);
         if constexpr (UPPER || sizeof(T) == 4) dst[line_coef_at<T, UPPER>(i, 3)] = static_cast<T>(d);
-        if constexpr (UPPER && sizeof(T) == 8) {
-            rlo[i] = lo;
-            div[i] = u;
-        }
+        if constexpr (UPPER && sizeof(T) == 8) div[i] = u;
     }
 }
 
