@@ -895,14 +895,17 @@ template <class T, bool UPPER>
 using LineKernel = void (*)(LineTri<T>, T*, const double*, T*, unsigned*, int*, const int*, int);
 template <class T, bool UPPER>
 static LineKernel<T, UPPER> line_kernel(const LineGeom& g, bool cluster) {
-    constexpr bool W3 = sizeof(T) == 8 && UPPER;  // (line_stays_warm of 3-D grids)
-    if (g.ny == 1 && line_stays_warm(g, sizeof(T), UPPER))
+    const bool warm = line_stays_warm(g, sizeof(T), UPPER);
+    if (g.ny == 1 && warm)
         return cluster ? sptrsv_line_cluster_kernel<T, UPPER, 1, false, true> : sptrsv_line_kernel<T, UPPER, 1, false, true>;
     if (g.ny == 1)
         return cluster ? sptrsv_line_cluster_kernel<T, UPPER, 1, false, false> : sptrsv_line_kernel<T, UPPER, 1, false, false>;
-    if (g.wy == 1) return cluster ? sptrsv_line_cluster_kernel<T, UPPER, 1, true, W3> : sptrsv_line_kernel<T, UPPER, 1, true, W3>;
-    if (g.wy == 4) return cluster ? sptrsv_line_cluster_kernel<T, UPPER, 4, true, W3> : sptrsv_line_kernel<T, UPPER, 4, true, W3>;
-    return cluster ? sptrsv_line_cluster_kernel<T, UPPER, 8, true, W3> : sptrsv_line_kernel<T, UPPER, 8, true, W3>;
+    // (8 lanes along y in both variants; 1 by an option, 4 for ny <= 4: as the backward sweep has it)
+    if (g.wy == 1) return cluster ? sptrsv_line_cluster_kernel<T, UPPER, 1, true, UPPER> : sptrsv_line_kernel<T, UPPER, 1, true, UPPER>;
+    if (g.wy == 4) return cluster ? sptrsv_line_cluster_kernel<T, UPPER, 4, true, UPPER> : sptrsv_line_kernel<T, UPPER, 4, true, UPPER>;
+    if constexpr (!UPPER)
+        if (!warm) return cluster ? sptrsv_line_cluster_kernel<T, false, 8, true, false> : sptrsv_line_kernel<T, false, 8, true, false>;
+    return cluster ? sptrsv_line_cluster_kernel<T, UPPER, 8, true, true> : sptrsv_line_kernel<T, UPPER, 8, true, true>;
 }
 template <class T>
 static const void* line_kernel_ptr(const LineGeom& g, bool cluster, bool upper) {
@@ -983,10 +986,12 @@ static bool configure_line(LinePack<T>& G, const DeviceInfo& dev, int max_cluste
     // for grids that do not fit at once clusters of 8 for FP32 and 4 for FP64 (the
     // measurements above line_geometry)
     const int most = G.g.ny == 1 ? 16 : (sizeof(T) == 4 ? 8 : 4);
-    // 3-D blocks more than 130 (FP64) or 300 lines deep would wait past about 50 us, after which
-    // a block's first steps run five times slower (their instructions have left the cache):
-    // they are left to the CTAs that finish first (96^3 FP64 backward: 172 us with all 144
-    // blocks resident, 125 us with 120 or 128).  2-D sweeps keep them warm (line_stays_warm).
+    // 3-D blocks more than 130 (FP64) or 300 lines deep would wait past about 50 us: they are left
+    // to the CTAs that finish first.  Forward sweeps whose instructions leave the cache meanwhile
+    // would run their first steps five times slower (96^3 FP64, all 144 blocks resident 172 us, 120 or
+    // 128 125 us); sweeps that keep them warm (line_stays_warm) take polls and votes from the
+    // blocks at work (with / without the limit, us: FP64 backward 40 x 40 x 500 288 / 309, 30 x
+    // 200 x 200 216 / 236, 96^3 130 / 131; FP32 40 x 40 x 500 129 / 133, 128^3 90 / 90).
     const int wait_lines = G.g.ny == 1 ? 1 << 30 : (sizeof(T) == 8 ? 130 : 300);
     G.grid = size_line_launch(G.g, G.threads, smem, max_cluster, most, wait_lines,
                               {line_kernel_ptr<T>(G.g, true, false), line_kernel_ptr<T>(G.g, true, true)},

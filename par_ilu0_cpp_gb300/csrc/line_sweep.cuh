@@ -59,7 +59,8 @@ constexpr int kLineSlots = 3;
 // compute warps) and 16 bytes more, which spread the lanes over the banks.
 template <class T>
 constexpr int kLinePitch = kLineChunk + 16 / static_cast<int>(sizeof(T));
-constexpr int kLineWarmLines = 300;  // FP32: lines that are passed in about 50 us
+constexpr int kLineWarmLines = 300;  // FP32, 2-D: lines that are passed in about 50 us
+constexpr int kLineWarmDepth = 280;  // 3-D: lines along y and z
 constexpr int kLineStepAlign = 8;  // steps of a warp are rounded up to a multiple of this
 
 struct LineGeom {
@@ -266,14 +267,22 @@ __device__ __forceinline__ bool line_late(double y, double z) {
 }
 
 // Whether waiting warps keep their instructions warm (WARM, line_compute), chosen per grid,
-// type (elem bytes) and sweep.  us, without / with, forward and backward: 1000^2 (blocks wait
-// for 300 us and more) FP32 214 / 156 and 195 / 139, FP64 392 / 267 and 694 / 405; FP64
-// backward 96^3 143 / 128 and 256^2 121 / 111.  It costs a little where the waits are short:
-// 256^2 FP32 44 / 46 and 39 / 41; 128^3, whose deep blocks are left to later CTAs, FP32 87 /
-// 90 and 83 / 85, FP64 forward 128 / 135.
+// type (elem bytes) and sweep.  us, without / with:
+// * 2-D: 1000^2 (blocks wait for 300 us and more) forward and backward FP32 214 / 156 and 195 /
+//   139, FP64 392 / 267 and 694 / 405; it costs a little where the waits are short: FP32 256^2 44
+//   / 46 and 39 / 41.  (256 and 1,000 lines were measured; the line between them stands where a
+//   wait reaches about 50 us.)
+// * 3-D backward: FP32 40 x 40 x 500 353 / 129, 64 x 64 x 200 89 / 75, 128^3 85 / 85, 96^3 63 / 63;
+//   FP64 96^3 143 / 128.
+// * 3-D forward: FP32 gains from about 300 lines along y and z (60 x 100 x 200 146 / 96, 32 x 32 x
+//   300 110 / 80, 24 x 24 x 1000 801 / 223; 160^3 and 200^3 lose, 126 / 131 and 193 / 200) and
+//   loses below (128^3 87 / 90, 96^3 63 / 66, 64 x 64 x 200 70 / 75); FP64, whose blocks are
+//   smaller, gains on narrow grids alone, where few blocks share an SM (20 x 20 x 300 265 / 117, 24
+//   x 24 x 1000 645 / 399; 40 x 40 x 500 218 / 230, 128^3 128 / 135).
 inline bool line_stays_warm(const LineGeom& g, int elem, bool upper) {
     if (g.ny == 1) return elem == 8 || g.nz > kLineWarmLines;
-    return elem == 8 && upper;
+    if (upper) return true;
+    return g.ny + g.nz > kLineWarmDepth && (elem == 4 || g.nby <= 2);
 }
 // Polls a warp's faces at its first step for about 20 us; whether all have arrived.
 template <class T>
