@@ -419,7 +419,7 @@ __device__ __forceinline__ void progressive_rows(int row, int K, const int (&c)[
 }
 
 // Progressive solve of rows of up to G * kLaneEntries entries with G lanes per row
-// (G = 2 .. 32, a warp holds 32 / G rows).  Lane j of a row's group holds entries
+// (G = 4 .. 32, a warp holds 32 / G rows).  Lane j of a row's group holds entries
 // [j K, j K + K) of the row in registers (K = the task's entries per lane; columns -1
 // pad the row's tail).  Every round each lane loads, all at once, the dependencies it
 // holds that are still unconsumed and still read as the sentinel (published values
@@ -486,6 +486,66 @@ __device__ __forceinline__ void group_rows(int row, int K, int lane, const int (
         if (!done && o >= G) {
             if (j == 0) st_relaxed(out + row, Sentinel<T>::canon(finish(acc)));
             done = true;
+        }
+        if (wb.expired(status)) {
+            if (!done) atomicExch(status + kStatusTimeout, 1);
+            break;
+        }
+    }
+}
+
+// The same for two lanes per row: the owner consumes its ready prefix, entry by entry, and the
+// sum is handed on (with a vote) at most twice in a round.  With a single hop to save, the
+// masks and the ballot of group_rows cost more than they spare: FP32 forward / backward, us,
+// group_rows and this: 27-point ILU(0) of 60 x 50 x 56 439 / 442 and 356 / 362, 7-point ILU(2) of 40
+// x 37 x 45 520 / 527 and 415 / 432, a band of 12 1064 / 1134 and 973 / 1042 (FP64 forward 815
+// and 709, 1014 and 842, 2154 and 2055).  From four lanes on group_rows is the faster one, up
+// to twice (only bands, where one row waits for the next, differ by 7 % either way).
+template <class T, bool UPPER>
+__device__ __forceinline__ void pair_rows(int row, int K, int lane, const int (&c)[kLaneEntries],
+                                          const T (&v)[kLaneEntries], T acc, T d, const T* dep, T* out, int* status) {
+    const int j = lane & 1;
+    const int gb = lane - j;
+    T x[kLaneEntries];
+#pragma unroll
+    for (int u = 0; u < kLaneEntries; ++u) x[u] = Sentinel<T>::value();
+    const RowFinish<UPPER, T> finish(d);
+    int o = 0;  // owner: lane of the first unconsumed entry (2 = row done)
+    int k = 0;  // next entry of this lane to consume (meaningful in the owner)
+    bool done = row < 0;
+    WaitBudget wb;
+    while (!__all_sync(0xffffffffu, done)) {
+        if (!done && j >= o) {
+            const int k0 = j == o ? k : 0;
+#pragma unroll
+            for (int u = 0; u < kLaneEntries; ++u)
+                if (u >= k0 && u < K && c[u] >= 0 && Sentinel<T>::is(x[u])) x[u] = ld_relaxed_nb(dep + c[u]);
+        }
+#pragma unroll 1
+        for (int step = 0; step < 2; ++step) {
+            bool fin = false;
+            if (!done && j == o) {
+#pragma unroll
+                for (int u = 0; u < kLaneEntries; ++u) {
+                    if (k == u && u < K) {
+                        if (c[u] < 0) {
+                            ++k;
+                        } else if (!Sentinel<T>::is(x[u])) {
+                            acc = fma(-v[u], x[u], acc);
+                            ++k;
+                        }
+                    }
+                }
+                fin = k >= K;
+            }
+            const int src = gb + min(o, 1);
+            const bool moved = __shfl_sync(0xffffffffu, fin, src);
+            acc = __shfl_sync(0xffffffffu, acc, src);
+            if (moved && ++o == 2) {
+                if (j == 0) st_relaxed(out + row, Sentinel<T>::canon(finish(acc)));
+                done = true;
+            }
+            if (!__any_sync(0xffffffffu, moved)) break;
         }
         if (wb.expired(status)) {
             if (!done) atomicExch(status + kStatusTimeout, 1);
@@ -603,7 +663,9 @@ __global__ void __launch_bounds__(kSolveWarps * kWarp, 1)
             int c[kLaneEntries];
             T v[kLaneEntries];
             load_lane_entries(L, off, K, lane, c, v);
-            if (G > 1)
+            if constexpr (G == 2)
+                pair_rows<T, false>(row, K, lane, c, v, acc, T(1), y, y, status);
+            else if constexpr (G > 2)
                 group_rows<T, false, G>(row, K, lane, c, v, acc, T(1), y, y, status);
             else
                 progressive_rows<T, false>(row, K, c, v, acc, T(1), y, y, status);
@@ -643,7 +705,9 @@ __global__ void __launch_bounds__(kSolveWarps * kWarp, 1)
             int c[kLaneEntries];
             T v[kLaneEntries];
             load_lane_entries(U, off, K, lane, c, v);
-            if (G > 1)
+            if constexpr (G == 2)
+                pair_rows<T, true>(row, K, lane, c, v, acc, d, x, x, status);
+            else if constexpr (G > 2)
                 group_rows<T, true, G>(row, K, lane, c, v, acc, d, x, x, status);
             else
                 progressive_rows<T, true>(row, K, c, v, acc, d, x, x, status);
