@@ -226,6 +226,37 @@ __device__ inline GroupSmem group_smem(unsigned char* base, int m, int G) {
 // Gram-Schmidt vectors one at a time, now 165.
 constexpr int kBatchEntries = 3;
 constexpr int kBatchJ = 4;  // basis vectors per batch of the Gram-Schmidt passes
+// SMALL: a level's loads one after the other and the Gram-Schmidt vectors one at a time.  In a
+// batch of small systems most of a CTA's warps have no row of a level, and what the pipeline
+// has them do beside the few that do is the longer part.  Small is a batch whose largest system
+// has at most kBatchSmall<G> rows.  Pipeline / this, ms: 1 right-hand side per item, sides 12 to
+// 16 2.36 / 2.04, 20 to 24 5.04 / 4.65, 24 to 28 6.78 / 6.98; 4: 12 to 16 1.37 / 1.11, 16 to 20
+// 1.99 / 1.84, 20 to 24 2.94 / 3.08; 16: 8 to 12 3.00 / 2.79, 12 to 16 2.23 / 2.22, 16 to 20 3.70 /
+// 4.13.  (A kernel of its own: both in one slowed the larger batches by a tenth.)
+template <int G>
+constexpr int kBatchSmall = G == 1 ? 576 : (G == 4 ? 400 : 200);
+
+template <int G, bool UPPER>
+__device__ __forceinline__ void small_level_sweep(const SysView& S, const float* in, float* out, int rl, int RT) {
+    const int nlev = UPPER ? S.nlevU : S.nlevL;
+    const int* lptr = UPPER ? S.lptrU : S.lptrL;
+    const int* ord = UPPER ? S.ordU : S.ordL;
+    for (int l = 0; l < nlev; ++l) {
+        for (int q = lptr[l] + rl; q < lptr[l + 1]; q += RT) {
+            const int row = ord[q];
+            float t = in[static_cast<long long>(row) * G];
+            if (UPPER) {
+                for (int p = S.rp[row + 1] - 1; p > S.diag[row]; --p) t = fmaf(-S.lu32[p], out[static_cast<long long>(S.ci[p]) * G], t);
+                out[static_cast<long long>(row) * G] = t * S.dinv[row];
+            } else {
+                for (int p = S.rp[row]; p < S.diag[row]; ++p) t = fmaf(-S.lu32[p], out[static_cast<long long>(S.ci[p]) * G], t);
+                out[static_cast<long long>(row) * G] = t;
+            }
+        }
+        __syncthreads();
+    }
+}
+
 template <int G, bool UPPER>
 __device__ __forceinline__ void level_sweep(const SysView& S, const float* in, float* out, int rl, int RT) {
     const int nlev = UPPER ? S.nlevU : S.nlevL;
@@ -301,7 +332,7 @@ __device__ __forceinline__ void level_sweep(const SysView& S, const float* in, f
     }
 }
 
-template <int G>
+template <int G, bool SMALL>
 __device__ void solve_group(const BatchDesc& D, int s, int r0, const GroupSmem& S2) {
     if (threadIdx.x == 0) *S2.flag = wait_flag(D.ready + s, D.epoch, D.status) ? 1 : 0;
     __syncthreads();
@@ -390,8 +421,15 @@ __device__ void solve_group(const BatchDesc& D, int s, int r0, const GroupSmem& 
         for (int i = 0; i < m; ++i) {
             if (tid < G && S2.cyc[tid]) ++S2.its[tid];
             // z = L^{-1} v (ascending entries), then z = U^{-1} z (descending, in place)
-            level_sweep<G, false>(S, V + static_cast<long long>(i) * ws * G + g, Z + static_cast<long long>(i) * ws * G + g, rl, RT);
-            level_sweep<G, true>(S, Z + static_cast<long long>(i) * ws * G + g, Z + static_cast<long long>(i) * ws * G + g, rl, RT);
+            const float* const vi = V + static_cast<long long>(i) * ws * G + g;
+            float* const zi = Z + static_cast<long long>(i) * ws * G + g;
+            if constexpr (SMALL) {
+                small_level_sweep<G, false>(S, vi, zi, rl, RT);
+                small_level_sweep<G, true>(S, zi, zi, rl, RT);
+            } else {
+                level_sweep<G, false>(S, vi, zi, rl, RT);
+                level_sweep<G, true>(S, zi, zi, rl, RT);
+            }
             // w = A z (FP32)
             for (int k = rl; k < n; k += RT) {
                 float acc = 0.f;
@@ -400,20 +438,21 @@ __device__ void solve_group(const BatchDesc& D, int s, int r0, const GroupSmem& 
             }
             // CGS2: two projections, per-warp partial sums in FP32, combined in FP64
             // (basis vectors in batches: more loads in flight, w read once per batch)
+            constexpr int J = SMALL ? 1 : kBatchJ;
             float nn = 0.f;
             for (int pass = 0; pass < 2; ++pass) {
                 for (int q = tid; q < (i + 1) * G; q += T) S2.acc[q] = 0.0;
                 __syncthreads();
-                for (int j0 = 0; j0 <= i; j0 += kBatchJ) {
-                    float part[kBatchJ] = {};
+                for (int j0 = 0; j0 <= i; j0 += J) {
+                    float part[J] = {};
 #pragma unroll 2
                     for (int k = rl; k < n; k += RT) {
                         const float wv = *vec(V, i + 1, k);
 #pragma unroll
-                        for (int u = 0; u < kBatchJ; ++u) part[u] = fmaf(*vec(V, min(j0 + u, i), k), wv, part[u]);
+                        for (int u = 0; u < J; ++u) part[u] = fmaf(*vec(V, min(j0 + u, i), k), wv, part[u]);
                     }
 #pragma unroll
-                    for (int u = 0; u < kBatchJ; ++u) {
+                    for (int u = 0; u < J; ++u) {
                         part[u] = warp_sum_g<G>(part[u]);
                         if (j0 + u <= i && (tid & 31) < G)
                             atomicAdd(S2.acc + (j0 + u) * G + (tid & 31), static_cast<double>(part[u]));
@@ -434,12 +473,12 @@ __device__ void solve_group(const BatchDesc& D, int s, int r0, const GroupSmem& 
                 for (int k = rl; k < n; k += RT) {
                     float a = *vec(V, i + 1, k);
                     int j = 0;
-                    for (; j + kBatchJ <= i + 1; j += kBatchJ) {
-                        float v[kBatchJ];
+                    for (; j + J <= i + 1; j += J) {
+                        float v[J];
 #pragma unroll
-                        for (int u = 0; u < kBatchJ; ++u) v[u] = *vec(V, j + u, k);
+                        for (int u = 0; u < J; ++u) v[u] = *vec(V, j + u, k);
 #pragma unroll
-                        for (int u = 0; u < kBatchJ; ++u) a = fmaf(-S2.cf[(g) * S2.ld + j + u], v[u], a);
+                        for (int u = 0; u < J; ++u) a = fmaf(-S2.cf[(g) * S2.ld + j + u], v[u], a);
                     }
                     for (; j <= i; ++j) a = fmaf(-S2.cf[(g) * S2.ld + j], *vec(V, j, k), a);
                     *vec(V, i + 1, k) = a;
@@ -537,7 +576,7 @@ __device__ void solve_group(const BatchDesc& D, int s, int r0, const GroupSmem& 
 // Two CTAs per SM (64 registers per thread): the autotuner's two-CTA shapes must really
 // be resident, and the solve items are latency-bound, so two per SM beat one.  G: right-
 // hand sides per solve item.
-template <int G>
+template <int G, bool SMALL>
 __global__ void __launch_bounds__(kBatchThreads, 2) batched_ilu_gmres_kernel(BatchDesc D, int nsys_run) {
     __shared__ double red[kBatchWarps];
     __shared__ float P[kMlpParams];
@@ -552,7 +591,7 @@ __global__ void __launch_bounds__(kBatchThreads, 2) batched_ilu_gmres_kernel(Bat
             factor_system(D, D.sys_of_slot[job], red, P);
         } else {
             const int k = job - nsys_run;
-            solve_group<G>(D, D.sys_of_slot[k / groups], (k % groups) * G, S2);
+            solve_group<G, SMALL>(D, D.sys_of_slot[k / groups], (k % groups) * G, S2);
         }
     }
 }
@@ -757,10 +796,11 @@ __global__ void batch_trial_rhs_kernel(BatchDesc D, int nsys_run) {
 }
 
 template <int G>
-static void launch_batched(int grid, const BatchDesc& D, int nsys_run, int m, const DeviceInfo& dev, cudaStream_t s) {
+static void launch_batched(int grid, const BatchDesc& D, int nsys_run, int nmax, int m, const DeviceInfo& dev, cudaStream_t s) {
     const size_t smem = group_smem_bytes(m, G);
-    allow_dynamic_smem(reinterpret_cast<const void*>(batched_ilu_gmres_kernel<G>), dev);
-    batched_ilu_gmres_kernel<G><<<grid, kBatchThreads, smem, s>>>(D, nsys_run);
+    const auto kern = nmax <= kBatchSmall<G> ? batched_ilu_gmres_kernel<G, true> : batched_ilu_gmres_kernel<G, false>;
+    allow_dynamic_smem(reinterpret_cast<const void*>(kern), dev);
+    kern<<<grid, kBatchThreads, smem, s>>>(D, nsys_run);
 }
 
 float BatchSolver::launch(int ctas_per_sm, bool largest_first, int nsys_run, int G) {
@@ -826,9 +866,9 @@ float BatchSolver::launch(int ctas_per_sm, bool largest_first, int nsys_run, int
     }
     GB_CUDA_CHECK(cudaEventRecord(ev0_, stream_));
     switch (G) {
-        case 1: launch_batched<1>(grid, D, nsys_run, m_, dev_, stream_); break;
-        case 4: launch_batched<4>(grid, D, nsys_run, m_, dev_, stream_); break;
-        case 16: launch_batched<16>(grid, D, nsys_run, m_, dev_, stream_); break;
+        case 1: launch_batched<1>(grid, D, nsys_run, nmax_, m_, dev_, stream_); break;
+        case 4: launch_batched<4>(grid, D, nsys_run, nmax_, m_, dev_, stream_); break;
+        case 16: launch_batched<16>(grid, D, nsys_run, nmax_, m_, dev_, stream_); break;
         default: throw std::runtime_error("batched: right-hand sides per item must be 1, 4 or 16");
     }
     GB_CUDA_CHECK(cudaGetLastError());
