@@ -419,7 +419,7 @@ __device__ __forceinline__ void progressive_rows(int row, int K, const int (&c)[
 }
 
 // Progressive solve of rows of up to G * kLaneEntries entries with G lanes per row
-// (G = 4 .. 32, a warp holds 32 / G rows).  Lane j of a row's group holds entries
+// (G = 8 .. 32, a warp holds 32 / G rows).  Lane j of a row's group holds entries
 // [j K, j K + K) of the row in registers (K = the task's entries per lane; columns -1
 // pad the row's tail).  Every round each lane loads, all at once, the dependencies it
 // holds that are still unconsumed and still read as the sentinel (published values
@@ -432,8 +432,7 @@ __device__ __forceinline__ void progressive_rows(int row, int K, const int (&c)[
 // per chunk of entries.  How far the sum will travel is known from the lanes' ready masks
 // (one ballot) before it starts, so that a hop is the products and one shuffle; the masks
 // worked out entry by entry on the way and a vote after each hop took 210 cycles a hop.
-// 27-point ILU(1) of 44 x 40 x 42 (530 levels), FP32 forward sweep: 8 lanes 850 us, now 649; 4
-// lanes 616, now 604 (there a level is one handoff through L2).
+// 27-point ILU(1) of 44 x 40 x 42 (530 levels), FP32 forward sweep on 8 lanes: 850 us, now 649.
 // Lane 0 of the group publishes the row.  Rounds are bounded as in progressive_rows.
 template <class T, bool UPPER, int G>
 __device__ __forceinline__ void group_rows(int row, int K, int lane, const int (&c)[kLaneEntries],
@@ -494,23 +493,26 @@ __device__ __forceinline__ void group_rows(int row, int K, int lane, const int (
     }
 }
 
-// The same for two lanes per row: the owner consumes its ready prefix, entry by entry, and the
-// sum is handed on (with a vote) at most twice in a round.  With a single hop to save, the
-// masks and the ballot of group_rows cost more than they spare: FP32 forward / backward, us,
-// group_rows and this: 27-point ILU(0) of 60 x 50 x 56 439 / 442 and 356 / 362, 7-point ILU(2) of 40
-// x 37 x 45 520 / 527 and 415 / 432, a band of 12 1064 / 1134 and 973 / 1042 (FP64 forward 815
-// and 709, 1014 and 842, 2154 and 2055).  From four lanes on group_rows is the faster one, up
-// to twice (only bands, where one row waits for the next, differ by 7 % either way).
-template <class T, bool UPPER>
-__device__ __forceinline__ void pair_rows(int row, int K, int lane, const int (&c)[kLaneEntries],
+// The same for two and four lanes per row: the owner consumes its ready prefix, entry by entry,
+// and hands the sum on with a vote, as often as it moves in a round.  With few hops to spare, the
+// masks and the ballot of group_rows cost more than they save.  us, forward / backward,
+// group_rows and this: two lanes FP32, 27-point ILU(0) of 60 x 50 x 56 439 / 442 and 333 / 347,
+// 7-point ILU(2) of 40 x 37 x 45 520 / 527 and 389 / 407 (FP64 forward 815 and 685, 1014 and 812);
+// four lanes FP32, 27-point ILU(1) of 40 x 44 x 42 611 / 633 and 562 / 578, a band of 20 954 / 950
+// and 814 / 818, random rows of up to 20 41 / 41 and 44 / 45 (FP64 1475 / 1530 and 1376 / 1509, 2014 /
+// 2196 and 1971 / 2068, 96 / 97 and 87 / 97).  From eight lanes on group_rows: FP32 27-point ILU(2) of
+// 30 x 27 x 25 609 / 636 and 669 / 664, a band of 200 483 / 511 and 597 / 662 (bands of 40 and 60, one
+// row waiting for the next, differ by up to a quarter either way with the SMs they get).
+template <class T, bool UPPER, int G>
+__device__ __forceinline__ void vote_rows(int row, int K, int lane, const int (&c)[kLaneEntries],
                                           const T (&v)[kLaneEntries], T acc, T d, const T* dep, T* out, int* status) {
-    const int j = lane & 1;
+    const int j = lane & (G - 1);
     const int gb = lane - j;
     T x[kLaneEntries];
 #pragma unroll
     for (int u = 0; u < kLaneEntries; ++u) x[u] = Sentinel<T>::value();
     const RowFinish<UPPER, T> finish(d);
-    int o = 0;  // owner: lane of the first unconsumed entry (2 = row done)
+    int o = 0;  // owner: group position of the first unconsumed entry (G = row done)
     int k = 0;  // next entry of this lane to consume (meaningful in the owner)
     bool done = row < 0;
     WaitBudget wb;
@@ -522,7 +524,7 @@ __device__ __forceinline__ void pair_rows(int row, int K, int lane, const int (&
                 if (u >= k0 && u < K && c[u] >= 0 && Sentinel<T>::is(x[u])) x[u] = ld_relaxed_nb(dep + c[u]);
         }
 #pragma unroll 1
-        for (int step = 0; step < 2; ++step) {
+        for (int step = 0; step < G; ++step) {
             bool fin = false;
             if (!done && j == o) {
 #pragma unroll
@@ -538,10 +540,10 @@ __device__ __forceinline__ void pair_rows(int row, int K, int lane, const int (&
                 }
                 fin = k >= K;
             }
-            const int src = gb + min(o, 1);
+            const int src = gb + min(o, G - 1);
             const bool moved = __shfl_sync(0xffffffffu, fin, src);
             acc = __shfl_sync(0xffffffffu, acc, src);
-            if (moved && ++o == 2) {
+            if (moved && ++o == G) {
                 if (j == 0) st_relaxed(out + row, Sentinel<T>::canon(finish(acc)));
                 done = true;
             }
@@ -663,9 +665,9 @@ __global__ void __launch_bounds__(kSolveWarps * kWarp, 1)
             int c[kLaneEntries];
             T v[kLaneEntries];
             load_lane_entries(L, off, K, lane, c, v);
-            if constexpr (G == 2)
-                pair_rows<T, false>(row, K, lane, c, v, acc, T(1), y, y, status);
-            else if constexpr (G > 2)
+            if constexpr (G == 2 || G == 4)
+                vote_rows<T, false, G>(row, K, lane, c, v, acc, T(1), y, y, status);
+            else if constexpr (G > 4)
                 group_rows<T, false, G>(row, K, lane, c, v, acc, T(1), y, y, status);
             else
                 progressive_rows<T, false>(row, K, c, v, acc, T(1), y, y, status);
@@ -705,9 +707,9 @@ __global__ void __launch_bounds__(kSolveWarps * kWarp, 1)
             int c[kLaneEntries];
             T v[kLaneEntries];
             load_lane_entries(U, off, K, lane, c, v);
-            if constexpr (G == 2)
-                pair_rows<T, true>(row, K, lane, c, v, acc, d, x, x, status);
-            else if constexpr (G > 2)
+            if constexpr (G == 2 || G == 4)
+                vote_rows<T, true, G>(row, K, lane, c, v, acc, d, x, x, status);
+            else if constexpr (G > 4)
                 group_rows<T, true, G>(row, K, lane, c, v, acc, d, x, x, status);
             else
                 progressive_rows<T, true>(row, K, c, v, acc, d, x, x, status);
