@@ -271,11 +271,12 @@ __device__ __forceinline__ void line_factor_block(const LineFactor& P, int blk, 
         const int cw = w - nw;
         const int nchunk = g.psteps / kLineChunk;
         const long long first = g.slot(blk, cw, 0, 0);
-        for (int k = 0; k < nchunk; ++k) {
-            if (k >= kLineFactorSlots) {
-                mbar_wait(M.done(cw, k - kLineFactorSlots), M.parity(k - kLineFactorSlots), status);
-                __syncwarp();
-            }
+        int k = 0;
+        for (; k < nchunk; ++k) {
+            // (given up: nothing more is staged, and the compute warp's waits give up as well)
+            if (k >= kLineFactorSlots && !__all_sync(0xffffffffu, mbar_wait(M.done(cw, k - kLineFactorSlots),
+                                                                            M.parity(k - kLineFactorSlots), status)))
+                break;
             if ((threadIdx.x & 31) == 0) {
                 constexpr unsigned bytes = kLineChunk * 32 * kLineFactorRow * 8;
                 mbar_arrive_expect(M.full(cw, k), bytes);
@@ -284,6 +285,8 @@ __device__ __forceinline__ void line_factor_block(const LineFactor& P, int blk, 
             }
             __syncwarp();
         }
+        for (int q = max(0, k - kLineFactorSlots); q < k; ++q) mbar_land(M.full(cw, q), M.parity(q));
+        __syncwarp();
     } else {
         // halo warps: the components of a face one after the other, a warp each for
         // y and z would wait for the first to end; so each component has its own warp

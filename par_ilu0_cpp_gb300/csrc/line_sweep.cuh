@@ -220,6 +220,13 @@ static __device__ __noinline__ bool mbar_wait_long(unsigned long long* b, unsign
 __device__ __forceinline__ bool mbar_wait(unsigned long long* b, unsigned parity, int* status) {
     return mbar_test(b, parity) || mbar_wait_long(b, parity, status);
 }
+// Waits for a bulk copy that has been issued to land: a block's barriers are initialised again, and
+// its shared memory given back, only then, also when a wait elsewhere gave up.  A copy comes to
+// its end whatever else happens; the bound is for form.
+__device__ __forceinline__ void mbar_land(unsigned long long* b, unsigned parity) {
+    for (int polls = 0; polls < (1 << 24) && !mbar_test(b, parity); ++polls) {
+    }
+}
 
 // A value that may be stored where others poll for the sentinel: the sentinel's own bit
 // pattern (a NaN) becomes the canonical NaN.  Integer compares: an FP64 compare would
@@ -574,12 +581,11 @@ __device__ __forceinline__ void line_helper(const LineTri<T>& P, int blk, int w,
         for (int r = 0; r < C; ++r)
             if (valid(r, k)) out[row0[r] + sx * C * k] = o[Q * r * kLinePitch<T>];
     };
-    // chunk k, its right-hand side in v; v is left with that of chunk k + 2
-    auto stage = [&](int k, T (&v)[C]) {
-        if (k >= S) {  // the slot's previous chunk is computed
-            mbar_wait(M.done(w, k - S), M.parity(k - S), status);
-            __syncwarp();
-        }
+    // chunk k, its right-hand side in v; v is left with that of chunk k + 2.  False when the
+    // slot's previous chunk is not computed in time: then nothing more is staged, and the
+    // compute warp's waits give up as well.
+    auto stage = [&](int k, T (&v)[C]) -> bool {
+        if (k >= S && !__all_sync(0xffffffffu, mbar_wait(M.done(w, k - S), M.parity(k - S), status))) return false;
         T* const slot = M.slot(w, k);
         unsigned long long* const full = M.full(w, k);
         if (lane == 0) {
@@ -604,21 +610,22 @@ __device__ __forceinline__ void line_helper(const LineTri<T>& P, int blk, int w,
         }
         if (k + 2 < nchunk) fetch(k + 2, v);
         if (k >= S) flush(k - S);
+        return true;
     };
     // right-hand sides are loaded two chunks ahead: a chunk's loads take as long as the
     // rest of the work on a chunk
     T va[C], vb[C];
     fetch(0, va);
     if (nchunk > 1) fetch(1, vb);
-    for (int k = 0; k < nchunk; k += 2) {
-        stage(k, va);
-        if (k + 1 < nchunk) stage(k + 1, vb);
-    }
-    for (int k = max(0, nchunk - S); k < nchunk; ++k) {
+    int staged = 0;
+    while (staged < nchunk && stage(staged, va) && ++staged < nchunk && stage(staged, vb)) ++staged;
+    for (int k = max(0, staged - S); k < staged; ++k) {
         mbar_wait(M.done(w, k), M.parity(k), status);
         __syncwarp();
         flush(k);
+        mbar_land(M.full(w, k), M.parity(k));
     }
+    __syncwarp();
 }
 
 // A halo warp of block `blk`: copies faces that the previous block hands over through its
