@@ -303,13 +303,15 @@ __device__ __forceinline__ bool line_first_faces(unsigned fy, unsigned fz) {
     return false;
 }
 
-// Bound of a wait made of many polls at a time: the clock is read every 16th time.
+// Bound of a warp's wait made of many polls at a time: the clock is read every 16th time.  All
+// lanes call it together and get one answer, whatever time each of them reads: shuffles and
+// votes of the whole warp follow.
 struct LineWait {
     WaitBudget wb;
     int calls = 0;
     __device__ __forceinline__ bool expired(int* status) {
         if ((++calls & 15) != 0) return false;
-        return slow(status);
+        return __any_sync(0xffffffffu, slow(status));
     }
     __device__ __noinline__ bool slow(int* status) {
         wb.polls |= 1023;  // so that expired() looks at the clock and at the status word
