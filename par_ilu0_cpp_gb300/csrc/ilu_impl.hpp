@@ -281,8 +281,9 @@ struct IluSolver::Impl {
     const void* subst_key() const;
     // Throws when a dependency wait timed out since the last call.
     void check_status(cudaStream_t s);
-    // Puts the line kernels' exchange buffers back to the sentinel (after a timeout).
-    void reset_exchange(cudaStream_t s);
+    // Puts exchange buffer `set` of the line sweeps back to the sentinel (after a call that uses
+    // it gave up; the other set may be in use on another stream).
+    void reset_exchange(int set, cudaStream_t s);
     // Writes wait_limit_us into the device status words (when they exist).
     void push_wait_limit();
 };

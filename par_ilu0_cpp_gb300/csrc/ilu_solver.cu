@@ -1275,16 +1275,15 @@ void IluSolver::Impl::check_status(cudaStream_t s) {
         GB_CUDA_CHECK(cudaMemcpy(status.get() + kStatusTimeout, &zero, sizeof(int), cudaMemcpyHostToDevice));
         // a kernel that gave up may leave its ticket counters or grid-barrier words set
         GB_CUDA_CHECK(cudaMemset(counters.get(), 0, sizeof(unsigned) * 8));
-        reset_exchange(s);
+        reset_exchange(0, s);
         GB_CUDA_CHECK(cudaStreamSynchronize(s));
         throw std::runtime_error("dependency wait timed out on the device");
     }
 }
 
-void IluSolver::Impl::reset_exchange(cudaStream_t s) {
-    for (auto& x : GP64.xch) fill_sentinel(x.get(), static_cast<long long>(x.size()), s, dev.sms);
-    for (auto& x : GP32.xch) fill_sentinel(x.get(), static_cast<long long>(x.size()), s, dev.sms);
-    fill_sentinel(GF.xch.get(), static_cast<long long>(GF.xch.size()), s, dev.sms);
+void IluSolver::Impl::reset_exchange(int set, cudaStream_t s) {
+    fill_sentinel(GP64.xch[set].get(), static_cast<long long>(GP64.xch[set].size()), s, dev.sms);
+    fill_sentinel(GP32.xch[set].get(), static_cast<long long>(GP32.xch[set].size()), s, dev.sms);
 }
 
 IluSolver::Impl* IluSolver::impl_ensure() {
@@ -1705,7 +1704,7 @@ bool IluSolver::FactorizeFrom(const double* values, bool on_device) {
         if (h[kStatusTimeout] != 0) {
             im.factorized = false;
             GB_CUDA_CHECK(cudaMemsetAsync(im.counters.get(), 0, sizeof(unsigned) * 8, s));
-            im.reset_exchange(s);
+            fill_sentinel(im.GF.xch.get(), static_cast<long long>(im.GF.xch.size()), s, im.dev.sms);
             GB_CUDA_CHECK(cudaStreamSynchronize(s));
             throw std::runtime_error("dependency wait timed out on the device");
         }
@@ -1865,7 +1864,7 @@ void IluSolver::SubstituteDeviceNoAlloc(const double* d_b, double* d_x) {
     GB_CUDA_CHECK(cudaMemcpyAsync(h, status, sizeof(h), cudaMemcpyDeviceToHost, s));
     GB_CUDA_CHECK(cudaStreamSynchronize(s));
     if (h[kStatusTimeout] != 0) {
-        im.reset_exchange(s);
+        im.reset_exchange(1, s);
         GB_CUDA_CHECK(cudaStreamSynchronize(s));
         throw std::runtime_error("dependency wait timed out on the device");
     }
