@@ -115,8 +115,16 @@ struct LinePack {
     int grid = 0;     // CTAs launched
     int smem_floor = 0;  // dynamic shared memory requested at least (bytes; one CTA per SM)
     DeviceBuffer<int> order;   // [nblk] block of each ticket
-    DeviceBuffer<T> l, u;      // operand streams
-    DeviceBuffer<T> div;       // [slots] FP64 U: diagonal
+    // Operand streams: L, U, and for FP64 U's diagonal [slots] (8 values per slot in all; the
+    // line factorisation keeps its own stream here while it runs).
+    DeviceBuffer<T> ops;
+    T* l() const { return ops.get(); }
+    T* u() const { return ops.get() + g.slots() / 32 * line_step_values<T, false>(); }
+    T* div() const { return sizeof(T) == 8 ? u() + g.slots() / 32 * line_step_values<T, true>() : nullptr; }
+    size_t ops_size() const {
+        return static_cast<size_t>(g.slots() / 32 * (line_step_values<T, false>() + line_step_values<T, true>()) +
+                                   (sizeof(T) == 8 ? g.slots() : 0));
+    }
     // Faces handed over through L2, at the sentinel between launches: [0] for the sweeps of
     // GMRES and Substitute (one stream at a time, as their ticket counters), [1] (FP64) for
     // the allocation-free entry point, which may run beside them.
@@ -130,10 +138,15 @@ struct LinePack {
         p.g = g;
         p.order = order.get();
         p.tl = tl[upper ? 1 : 0].get();
-        p.coef = upper ? u.get() : l.get();
-        p.div = div.get();
+        p.coef = upper ? u() : l();
+        p.div = div();
         p.xch = xch[set].get();
         return p;
+    }
+    void release() {
+        ops.release();
+        for (auto& x : xch) x.release();
+        for (auto& t : tl) t.release();
     }
 };
 
@@ -142,14 +155,22 @@ struct LineFactorPack {
     LineGeom g;
     int grid = 0;  // CTAs launched
     DeviceBuffer<int> order;    // blocks (clusters) by ticket
-    DeviceBuffer<double> rows;  // operand stream, packed from A by every factorisation
+    // Operand stream, packed from A by every factorisation: in the FP64 sweeps' streams, which are
+    // packed from its result, or where these are too small or missing in its own buffer.
+    double* rows = nullptr;
+    DeviceBuffer<double> own;
     DeviceBuffer<double> xch;   // faces handed over through L2, at the sentinel between launches
 
+    void release() {
+        rows = nullptr;
+        own.release();
+        xch.release();
+    }
     LineFactor view() const {
         LineFactor p;
         p.g = g;
         p.order = order.get();
-        p.rows = rows.get();
+        p.rows = rows;
         p.xch = xch.get();
         return p;
     }

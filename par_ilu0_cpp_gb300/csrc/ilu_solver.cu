@@ -976,8 +976,7 @@ static int size_line_launch(LineGeom& g, int threads, size_t smem, int max_clust
     return per_sm < 1 ? 0 : std::min({g.nblk, per_sm * dev.sms, early});
 }
 
-// Configures the sweeps of value type T and allocates their packed operands; false when a
-// CTA cannot be resident.
+// Configures the sweeps of value type T; false when a CTA cannot be resident.
 template <class T>
 static bool configure_line(LinePack<T>& G, const DeviceInfo& dev, int max_cluster) {
     const size_t smem = std::max(static_cast<size_t>(std::max(line_smem_bytes<T, false>(G.g), line_smem_bytes<T, true>(G.g))),
@@ -996,12 +995,7 @@ static bool configure_line(LinePack<T>& G, const DeviceInfo& dev, int max_cluste
     G.grid = size_line_launch(G.g, G.threads, smem, max_cluster, most, wait_lines,
                               {line_kernel_ptr<T>(G.g, true, false), line_kernel_ptr<T>(G.g, true, true)},
                               {line_kernel_ptr<T>(G.g, false, false), line_kernel_ptr<T>(G.g, false, true)}, dev);
-    if (G.grid == 0) return false;
-    const size_t slots = static_cast<size_t>(G.g.slots());
-    G.l.reserve(slots / 32 * line_step_values<T, false>());
-    G.u.reserve(slots / 32 * line_step_values<T, true>());
-    if (sizeof(T) == 8) G.div.reserve(slots);
-    return true;
+    return G.grid > 0;
 }
 
 // Packs the factor values into the operand streams of type T (`sweeps`: bit 0 L, bit 1 U);
@@ -1011,8 +1005,8 @@ static int pack_line(LinePack<T>& G, int sweeps, const int* rp, const int* diag,
     const long long slots = G.g.slots();
     const int threads = 256;
     const int grid = static_cast<int>(std::max<long long>(1, std::min<long long>(ceil_div<long long>(slots, threads), 8LL * sms)));
-    if (sweeps & 1) line_pack_kernel<T, false><<<grid, threads, 0, s>>>(G.g, rp, diag, lu, G.l.get(), nullptr);
-    if (sweeps & 2) line_pack_kernel<T, true><<<grid, threads, 0, s>>>(G.g, rp, diag, lu, G.u.get(), G.div.get());
+    if (sweeps & 1) line_pack_kernel<T, false><<<grid, threads, 0, s>>>(G.g, rp, diag, lu, G.l(), nullptr);
+    if (sweeps & 2) line_pack_kernel<T, true><<<grid, threads, 0, s>>>(G.g, rp, diag, lu, G.u(), G.div());
     GB_CUDA_CHECK(cudaGetLastError());
     return (sweeps & 1) + (sweeps >> 1);
 }
@@ -1041,10 +1035,24 @@ static LineFactorKernel line_factor_kernel(const LineGeom& g, bool cluster) {
     return cluster ? ilu_factor_line_kernel<8, true, true> : ilu_factor_line_kernel<8, true, false>;
 }
 
+// Runs the allocations of an optional schedule; false, and `pack` empty again, when there is no
+// room for them.
+template <class P, class F>
+static bool reserve_optional(P& pack, F reserve) {
+    try {
+        reserve();
+        return true;
+    } catch (const std::runtime_error&) {
+        cudaGetLastError();
+        pack.release();
+        return false;
+    }
+}
+
 // Sets up the line-pipeline factorisation for a grid; false when a CTA cannot be resident or
-// its operand stream does not fit in device memory.
-static bool setup_line_factor(LineFactorPack& G, int nx, int ny, int nz, int max_cluster, const DeviceInfo& dev,
-                              cudaStream_t s) {
+// its operand stream does not fit in device memory.  `sweeps`: the FP64 sweeps, set up, or null.
+static bool setup_line_factor(LineFactorPack& G, const LinePack<double>* sweeps, int nx, int ny, int nz, int max_cluster,
+                              const DeviceInfo& dev, cudaStream_t s) {
     if (nx < 3 || ny == 2) return false;  // elimination would change more than the diagonal
     G.grid = 0;
     for (int by : {kLineFactorWarps, 1}) {
@@ -1059,17 +1067,17 @@ static bool setup_line_factor(LineFactorPack& G, int nx, int ny, int nz, int max
         if (G.grid > 0) break;
     }
     if (G.grid == 0) return false;
+    const size_t rows = static_cast<size_t>(line_factor_at(G.g.slots(), 0));
+    const bool shared = sweeps != nullptr && sweeps->ops.size() >= rows;
+    if (!reserve_optional(G, [&] {
+            if (!shared) G.own.reserve(rows);
+            G.xch.reserve(static_cast<size_t>(kLinePivotParts * G.g.nblk * G.g.xch_block()));
+        }))
+        return false;
+    if (shared) G.own.release();
+    G.rows = shared ? sweeps->ops.get() : G.own.get();
     const std::vector<int> order = line_block_order(G.g);
     G.order.upload(order.data(), order.size(), s);
-    try {
-        G.rows.reserve(static_cast<size_t>(line_factor_at(G.g.slots(), 0)));
-        G.xch.reserve(static_cast<size_t>(kLinePivotParts * G.g.nblk * G.g.xch_block()));
-    } catch (const std::runtime_error&) {  // no room for the stream (64 B per row): the other kernels need none
-        cudaGetLastError();
-        G.rows.release();
-        G.xch.release();
-        return false;
-    }
     fill_sentinel(G.xch.get(), static_cast<long long>(G.xch.size()), s, dev.sms);
     GB_CUDA_CHECK(cudaStreamSynchronize(s));  // `order` must outlive the copy
     return true;
@@ -1081,7 +1089,7 @@ static void launch_line_factor(const LineFactorPack& G, const int* rp, const int
     const long long slots = G.g.slots();
     const int threads = 256;
     const int grid = static_cast<int>(std::min<long long>(ceil_div<long long>(slots, threads), 8LL * dev.sms));
-    line_factor_pack_kernel<<<grid, threads, 0, s>>>(G.g, rp, diag, lu, shift, G.rows.get());
+    line_factor_pack_kernel<<<grid, threads, 0, s>>>(G.g, rp, diag, lu, shift, G.rows);
     const size_t smem = static_cast<size_t>(line_factor_smem_bytes(G.g));
     const auto kern = line_factor_kernel(G.g, G.g.cl > 0);
     if (G.g.cl > 0) {
@@ -1091,7 +1099,7 @@ static void launch_line_factor(const LineFactorPack& G, const int* rp, const int
     } else {
         kern<<<G.grid, line_factor_threads(G.g), smem, s>>>(G.view(), counter, status);
     }
-    line_factor_unpack_kernel<<<grid, threads, 0, s>>>(G.g, rp, G.rows.get(), lu, status);
+    line_factor_unpack_kernel<<<grid, threads, 0, s>>>(G.g, rp, G.rows, lu, status);
     GB_CUDA_CHECK(cudaGetLastError());
 }
 
@@ -1161,8 +1169,9 @@ static void tune_line(IluSolver::Impl& im, cudaStream_t s) {
     im.check_status(s);
 }
 
-// Sets up the line-pipeline sweeps of value type T for a grid: geometry, kernels, exchange
-// buffers, timelines.  False when a CTA of one warp cannot be resident.
+// Sets up the line-pipeline sweeps of value type T for a grid: geometry, kernels, operand
+// streams, exchange buffers, timelines.  False when a CTA of one warp cannot be resident or the
+// buffers do not fit in device memory.
 template <class T>
 static bool setup_line(IluSolver::Impl& im, LinePack<T>& G, int nx, int ny, int nz, cudaStream_t s) {
     // the requested (or automatic) CTA shape, halved along its longer side until its
@@ -1180,21 +1189,22 @@ static bool setup_line(IluSolver::Impl& im, LinePack<T>& G, int nx, int ny, int 
         bz = G.g.bz;
         (bz >= by ? bz : by) = std::max(1, (bz >= by ? bz : by) / 2);
     }
-    for (int u = 0; u < 2; ++u) {
-        G.tl[u].release();
-        if (im.sweep_timeline && ok) {
-            const size_t len = static_cast<size_t>(G.g.nblk) * kLineTimeline;
-            G.tl[u].reserve(len);
-            GB_CUDA_CHECK(cudaMemsetAsync(G.tl[u].get(), 0, len * sizeof(unsigned long long), s));
-        }
-    }
-    if (!ok) return false;
+    for (auto& t : G.tl) t.release();
+    const size_t tl_len = static_cast<size_t>(G.g.nblk) * kLineTimeline;
+    constexpr int sets = sizeof(T) == 8 ? 2 : 1;
+    if (!ok || !reserve_optional(G, [&] {
+            G.ops.reserve(G.ops_size());
+            for (int set = 0; set < sets; ++set) G.xch[set].reserve(static_cast<size_t>(G.g.nblk * G.g.xch_block()));
+            for (auto& t : G.tl)
+                if (im.sweep_timeline) t.reserve(tl_len);
+        }))
+        return false;
+    for (auto& t : G.tl)
+        if (im.sweep_timeline) GB_CUDA_CHECK(cudaMemsetAsync(t.get(), 0, tl_len * sizeof(unsigned long long), s));
     const std::vector<int> order = line_block_order(G.g);
     G.order.upload(order.data(), order.size(), s);
-    for (int set = 0; set < (sizeof(T) == 8 ? 2 : 1); ++set) {
-        G.xch[set].reserve(static_cast<size_t>(G.g.nblk * G.g.xch_block()));
+    for (int set = 0; set < sets; ++set)
         fill_sentinel(G.xch[set].get(), static_cast<long long>(G.xch[set].size()), s, im.dev.sms);
-    }
     GB_CUDA_CHECK(cudaStreamSynchronize(s));  // `order` must outlive the copy
     return true;
 }
@@ -1247,7 +1257,7 @@ template <class T>
 const void* IluSolver::Impl::subst_key() const {
     if (levelsync) return LS.cols.get();
     if (const int bits = sizeof(T) == 8 ? line_use64 : line_use32; bits != 0)  // the schedule is part of the key
-        return reinterpret_cast<const char*>(line_pack<T>().l.get()) + bits;
+        return reinterpret_cast<const char*>(line_pack<T>().ops.get()) + bits;
     if (sizeof(T) == 8 ? blk64 : blk32) return (sizeof(T) == 8 ? LB64 : LB32).codes.get();
     return L.cols.get();
 }
@@ -1369,26 +1379,27 @@ void IluSolver::SetupMatrix() {
     // structured-grid line-pipeline sweeps: 7- / 5-point stencil factors in natural order
     // (automatic, grid_mode 0: when the other schedules are automatic too; 1: always)
     im.grid64 = im.grid32 = im.fact_line = false;
-    if (im.grid_mode == 1 || (im.grid_mode == 0 && im.block_rows == 0)) {
+    auto setup_grid = [&] {
         int gx = 0, gy = 0, gz = 0;
-        if (detect_grid(n, rp, ci, im.an.diag, gx, gy, gz)) {
-            im.grid64 = setup_line(im, im.GP64, gx, gy, gz, s);
-            // (one geometry for both types while timelines are recorded, so that one
-            // LLJBASH_IluInfo describes them)
-            im.grid32 = setup_line(im, im.GP32, gx, gy, gz, s);
-            // Factorisation: the line pipeline unless a kernel or a ticket order is asked for
-            // (five to nine times faster than the warp-per-row kernel from 32^2 and 16^3 to
-            // 1024^2 and 200^3, flat and deep grids included)
-            if (im.factor_kernel == 0 && im.ticket_order == 0)
-                im.fact_line = setup_line_factor(im.GF, gx, gy, gz, im.grid_cluster, im.dev, s);
-        }
-    }
+        if (!detect_grid(n, rp, ci, im.an.diag, gx, gy, gz)) return;
+        im.grid64 = setup_line(im, im.GP64, gx, gy, gz, s);
+        // (one geometry for both types while timelines are recorded, so that one
+        // LLJBASH_IluInfo describes them)
+        im.grid32 = setup_line(im, im.GP32, gx, gy, gz, s);
+        // Factorisation: the line pipeline unless a kernel or a ticket order is asked for
+        // (three to five times faster than the warp-per-row kernel on every shape measured: 16^3
+        // to 200^3, 32^2 to 1024^2, 64 x 64 x 3, 300 x 300 x 3, 3 x 2000 x 3, 5 x 5 x 2000, 3 x 3 x 50000,
+        // 3 x 20000, 40 x 40 x 500)
+        if (im.factor_kernel == 0 && im.ticket_order == 0)
+            im.fact_line = setup_line_factor(im.GF, im.grid64 ? &im.GP64 : nullptr, gx, gy, gz, im.grid_cluster, im.dev, s);
+    };
+    // (automatic: below, after every buffer that the other schedules cannot do without)
+    if (im.grid_mode == 1) setup_grid();
     // forced (grid_mode 1): every sweep of a configured type; automatic: timed against the
     // other schedules at the first Factorize (tune_line_sweeps)
     const bool line_forced = im.grid_mode == 1;
     im.line_use64 = line_forced && im.grid64 ? 3 : 0;
     im.line_use32 = line_forced && im.grid32 ? 3 : 0;
-    im.line_tuned = line_forced || !(im.grid64 || im.grid32);
     const bool grid_both = line_forced && im.grid64 && im.grid32;
     im.blk64 = im.blk32 = false;
     if (im.block_rows >= 0 && !grid_both) {
@@ -1468,13 +1479,21 @@ void IluSolver::SetupMatrix() {
     im.sy32.reserve(nv);
     fill_sentinel(im.sy64.get(), static_cast<long long>(nv), s, im.dev.sms);
     fill_sentinel(im.sy32.get(), static_cast<long long>(nv), s, im.dev.sms);
-    // Factorisation kernel: warp per row (automatic), or lane per row for short rows when
-    // requested
+    // Factorisation kernel: lane per row for short rows when requested, else the line pipeline
+    // or a warp per row
     im.fact_lane = false;
     if (im.factor_kernel == 2 && im.ticket_order != 2 && n > 0)
         im.fact_lane = build_lane_factor(n, rp, ci, im.an.diag,
                                          im.ticket_order == 1 ? tree_order : im.an.order_l, im, s);
-    if (!im.fact_line && !im.fact_lane) im.rinv.reserve(static_cast<size_t>(std::max(n, 1)));
+    if (im.grid_mode == 0 && im.block_rows == 0) setup_grid();
+    const bool by_rows = !im.fact_line && !im.fact_lane;  // a warp per row
+    auto reserve_rinv = [&] { im.rinv.reserve(static_cast<size_t>(std::max(n, 1))); };
+    if (by_rows && !line_forced && !reserve_optional(im.rinv, reserve_rinv)) im.grid64 = im.grid32 = false;
+    if (!im.fact_line) im.GF.release();
+    if (!im.grid64) im.GP64.release();
+    if (!im.grid32) im.GP32.release();
+    if (by_rows) reserve_rinv();
+    im.line_tuned = line_forced || !(im.grid64 || im.grid32);
     // Factorisation launch: rows staged in shared memory up to the longest row where a
     // warp's share fits (fewer warps per block for long rows), a wider register window
     // of the next pivot row when pivot rows are long.
