@@ -194,7 +194,7 @@ typedef struct LLJBASH_IluInfo {
     int block_cluster_fp32; /* the same for the FP32 sweeps */
     int row_lanes_lower;  /* lanes per row of the level-ordered lower / upper sweeps */
     int row_lanes_upper;
-    int factor_lane;      /* 1: the factorisation runs one lane per row (else one warp per row) */
+    int factor_lane;      /* 1: the factorisation runs one lane per row (else factor_line, else one warp per row) */
     int grid_fp64;        /* FP64 / FP32 sweeps on the line-pipeline schedule: bit 0 the
                            * forward, bit 1 the backward sweep */
     int grid_fp32;
@@ -207,6 +207,7 @@ typedef struct LLJBASH_IluInfo {
     int grid_cluster;     /* CTAs per thread-block cluster of the FP64 line-pipeline sweeps, 0: none */
     int factor_subtree_parts; /* ticket order 2: subtree partitions (one CTA each) and their rows */
     int factor_subtree_rows;
+    int factor_line;      /* 1: the factorisation runs on the line pipeline */
 } LLJBASH_IluInfo;
 int LLJBASH_IluSolverGetInfo(IluSolverHdl hdl, LLJBASH_IluInfo* info);
 

@@ -391,6 +391,7 @@ int LLJBASH_IluSolverGetInfo(IluSolverHdl hdl, LLJBASH_IluInfo* info) {
     info->row_lanes_lower = im->level_packs ? im->L.group : 0;
     info->row_lanes_upper = im->level_packs ? im->U.group : 0;
     info->factor_lane = im->fact_lane ? 1 : 0;
+    info->factor_line = im->fact_line ? 1 : 0;
     info->factor_subtree_parts = im->ticket_order == 2 ? im->sub_parts : 0;
     info->factor_subtree_rows = im->ticket_order == 2 ? im->sub_rows : 0;
     info->grid_fp64 = im->line_use64;
