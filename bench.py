@@ -152,10 +152,11 @@ def algorithmic_bytes(kind, a, nnz_l, nnz_u, tsize, steps_hist):
 def measured_traffic(kernel, size, block_rows, cluster, line=False):
     """DRAM bytes per launch (dram__bytes_read.sum + dram__bytes_write.sum) of `kernel`
     for this workload and substitution schedule, from the ncu captures recorded in
-    profiles/dram_traffic.json (entries: kernel, size, schedule "line" with the CTAs per
-    cluster of the line-pipeline kernel (0: none), or block_rows / cluster of the
-    block-local kernel, bytes, source); None when no capture matches the kernel and
-    schedule that ran."""
+    profiles/dram_traffic.json (entries: kernel, size, schedule "line" with the launch shape
+    of the line-pipeline kernel, [warps of a CTA along y, along z, CTAs per cluster], or
+    block_rows / cluster of the block-local kernel, bytes, source; a line entry with a plain
+    number of CTAs per cluster is of the earlier line kernel without helper warps); None
+    when no capture matches the kernel and schedule that ran."""
     path = os.path.join(ROOT, "profiles", "dram_traffic.json")
     if not os.path.isfile(path):
         return None
@@ -659,12 +660,14 @@ def run_ours(args):
                 "fp64_cluster": int(info_m.block_cluster_fp64), "fp32_cluster": int(info_m.block_cluster_fp32),
                 # line-pipeline sweeps (bit 0 forward, bit 1 backward), chosen by timing at setup
                 "fp64_line": int(info_m.grid_fp64), "fp32_line": int(info_m.grid_fp32),
-                "line_shape": [int(info_m.grid_warp_y), int(info_m.grid_warp_z), int(info_m.grid_cta_y),
-                               int(info_m.grid_cta_z), int(info_m.grid_blocks)],
-                "line_cluster": int(info_m.grid_cluster)}
+                # the FP32 sweeps' lanes of a warp along y and z, warps of a CTA, blocks
+                "line_shape": [int(info_m.grid_warp_y), int(info_m.grid_warp_z), int(info_m.grid32_cta_y),
+                               int(info_m.grid32_cta_z), int(info_m.grid32_blocks)],
+                "line_cluster": int(info_m.grid32_cluster)}
     dom_line = bool(schedule["fp32_line"] & (1 if dom == "sptrsv_lower" else 2 if dom == "sptrsv_upper" else 0))
     traffic = measured_traffic(dom, args.size, schedule["fp32_block_rows"],
-                               schedule["line_cluster"] if dom_line else schedule["fp32_cluster"], dom_line)
+                               schedule["line_shape"][2:4] + [schedule["line_cluster"]] if dom_line
+                               else schedule["fp32_cluster"], dom_line)
 
     batched = None
     others = None

@@ -201,13 +201,17 @@ typedef struct LLJBASH_IluInfo {
     int grid_nx, grid_ny, grid_nz;  /* its grid (2-D: grid_ny = 1) */
     int grid_warp_y;      /* lanes of a warp along y and z */
     int grid_warp_z;
-    int grid_cta_y;       /* warps of a CTA along y and z */
+    int grid_cta_y;       /* warps of a CTA along y and z (FP64 sweeps; FP32's where FP64 has none) */
     int grid_cta_z;
-    int grid_blocks;      /* CTA-sized blocks of grid lines */
-    int grid_cluster;     /* CTAs per thread-block cluster of the FP64 line-pipeline sweeps, 0: none */
+    int grid_blocks;      /* CTA-sized blocks of grid lines (as grid_cta_y) */
+    int grid_cluster;     /* CTAs per thread-block cluster, 0: none (as grid_cta_y) */
     int factor_subtree_parts; /* ticket order 2: subtree partitions (one CTA each) and their rows */
     int factor_subtree_rows;
     int factor_line;      /* 1: the factorisation runs on the line pipeline */
+    int grid32_cta_y;     /* grid_cta_y .. grid_cluster of the FP32 line-pipeline sweeps */
+    int grid32_cta_z;
+    int grid32_blocks;
+    int grid32_cluster;
 } LLJBASH_IluInfo;
 int LLJBASH_IluSolverGetInfo(IluSolverHdl hdl, LLJBASH_IluInfo* info);
 

@@ -56,7 +56,9 @@ class IluInfo(ctypes.Structure):
                 ("grid_ny", ctypes.c_int), ("grid_nz", ctypes.c_int), ("grid_warp_y", ctypes.c_int),
                 ("grid_warp_z", ctypes.c_int), ("grid_cta_y", ctypes.c_int), ("grid_cta_z", ctypes.c_int),
                 ("grid_blocks", ctypes.c_int), ("grid_cluster", ctypes.c_int), ("factor_subtree_parts", ctypes.c_int),
-                ("factor_subtree_rows", ctypes.c_int), ("factor_line", ctypes.c_int)]
+                ("factor_subtree_rows", ctypes.c_int), ("factor_line", ctypes.c_int),
+                ("grid32_cta_y", ctypes.c_int), ("grid32_cta_z", ctypes.c_int), ("grid32_blocks", ctypes.c_int),
+                ("grid32_cluster", ctypes.c_int)]
 
 
 class GmresReport(ctypes.Structure):

@@ -408,6 +408,13 @@ int LLJBASH_IluSolverGetInfo(IluSolverHdl hdl, LLJBASH_IluInfo* info) {
         info->grid_blocks = g.nblk;
         info->grid_cluster = g.cl;
     }
+    if (im->grid32) {
+        const gb300::LineGeom& g = im->GP32.g;
+        info->grid32_cta_y = g.by;
+        info->grid32_cta_z = g.bz;
+        info->grid32_blocks = g.nblk;
+        info->grid32_cluster = g.cl;
+    }
     return 0;
 }
 

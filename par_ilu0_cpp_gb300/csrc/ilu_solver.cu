@@ -1179,7 +1179,7 @@ static bool setup_line(IluSolver::Impl& im, LinePack<T>& G, int nx, int ny, int 
     int by = im.grid_by, bz = im.grid_bz;
     bool ok = false;
     for (int attempt = 0; attempt < 8; ++attempt) {
-        G.g = line_geometry(nx, ny, nz, im.grid_wy, by, bz, im.sweep_timeline ? 8 : static_cast<int>(sizeof(T)));
+        G.g = line_geometry(nx, ny, nz, im.grid_wy, by, bz, static_cast<int>(sizeof(T)));
         G.threads = G.g.threads();
         // one CTA per SM on request: more than half of an SM's shared memory
         G.smem_floor = im.grid_one_cta_per_sm ? std::min(im.dev.smem_per_sm / 2 + 1024, im.dev.smem_optin - 1024) : 0;
@@ -1383,8 +1383,6 @@ void IluSolver::SetupMatrix() {
         int gx = 0, gy = 0, gz = 0;
         if (!detect_grid(n, rp, ci, im.an.diag, gx, gy, gz)) return;
         im.grid64 = setup_line(im, im.GP64, gx, gy, gz, s);
-        // (one geometry for both types while timelines are recorded, so that one
-        // LLJBASH_IluInfo describes them)
         im.grid32 = setup_line(im, im.GP32, gx, gy, gz, s);
         // Factorisation: the line pipeline unless a kernel or a ticket order is asked for
         // (three to five times faster than the warp-per-row kernel on every shape measured: 16^3

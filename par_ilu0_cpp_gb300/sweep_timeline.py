@@ -19,6 +19,7 @@ from __future__ import annotations
 
 import argparse
 import json
+from types import SimpleNamespace
 
 import numpy as np
 
@@ -26,9 +27,23 @@ from . import api
 from . import generators as gen
 
 
-def summarize(tl: np.ndarray, info: api.IluInfo) -> dict:
+def geometry(info: api.IluInfo, fp32: bool):
+    """The grid, its lanes and the CTA shape, blocks and cluster of one type's sweeps, under the
+    names of IluInfo's grid_* fields."""
+    shape = ("cta_y", "cta_z", "blocks", "cluster")
+    g = {"grid_" + k: getattr(info, "grid_" + k) for k in ("nx", "ny", "nz", "warp_y", "warp_z") + shape}
+    if fp32:
+        g.update({"grid_" + k: getattr(info, "grid32_" + k) for k in shape})
+    return SimpleNamespace(**g)
+
+
+def line_shape(g) -> list:
+    return [g.grid_warp_y, g.grid_warp_z, g.grid_cta_y, g.grid_cta_z, g.grid_blocks]
+
+
+def summarize(tl: np.ndarray, info) -> dict:
     """Splits one sweep's per-block timeline (LLJBASH_IluSolverGetSweepTimeline) into
-    per-step and per-handoff costs.  Block index b = iy + nby iz in sweep coordinates."""
+    per-step and per-handoff costs (info: geometry() of its type).  Block index b = iy + nby iz in sweep coordinates."""
     wy, wz, by, bz = info.grid_warp_y, info.grid_warp_z, info.grid_cta_y, info.grid_cta_z
     nx, ny, nz = info.grid_nx, info.grid_ny, info.grid_nz
     nw = by * bz
@@ -96,8 +111,7 @@ def run(size: int, cta=(0, 0), cluster: int = 1, one_cta_per_sm: bool = False) -
     res = gm.solve(a, b)
     info = ilu.info()
     out = {"workload": f"convdiff3d {size}^3 ILU(0), mixed GMRES(50)", "iterations": int(res.iterations),
-           "line_shape": [info.grid_warp_y, info.grid_warp_z, info.grid_cta_y, info.grid_cta_z, info.grid_blocks],
-           "cluster": int(info.grid_cluster), "one_cta_per_sm": bool(one_cta_per_sm),
+           "one_cta_per_sm": bool(one_cta_per_sm),
            "fp64_line": int(info.grid_fp64), "fp32_line": int(info.grid_fp32),
            "sweeps": {}}
     for fp32 in (True, False):
@@ -109,7 +123,8 @@ def run(size: int, cta=(0, 0), cluster: int = 1, one_cta_per_sm: bool = False) -
             if not tl[:, 0].any():
                 continue  # no line-pipeline sweep of this kind ran
             name = f"{'fp32' if fp32 else 'fp64'}_{'backward' if upper else 'forward'}"
-            out["sweeps"][name] = summarize(tl, info)
+            g = geometry(info, fp32)
+            out["sweeps"][name] = dict(line_shape=line_shape(g), cluster=int(g.grid_cluster), **summarize(tl, g))
     return out
 
 
