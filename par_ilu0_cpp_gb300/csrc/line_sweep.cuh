@@ -59,7 +59,7 @@ constexpr int kLineSlots = 3;
 // compute warps) and 16 bytes more, which spread the lanes over the banks.
 template <class T>
 constexpr int kLinePitch = kLineChunk + 16 / static_cast<int>(sizeof(T));
-constexpr int kLineWarmLines = 300;  // FP32, 2-D: lines that are passed in about 50 us
+constexpr int kLineWarmLines = 700;  // FP32, 2-D: lines
 constexpr int kLineWarmDepth = 280;  // 3-D: lines along y and z
 constexpr int kLineStepAlign = 8;  // steps of a warp are rounded up to a multiple of this
 
@@ -276,9 +276,9 @@ __device__ __forceinline__ bool line_late(double y, double z) {
 // Whether waiting warps keep their instructions warm (WARM, line_compute), chosen per grid,
 // type (elem bytes) and sweep.  us, without / with:
 // * 2-D: 1000^2 (blocks wait for 300 us and more) forward and backward FP32 214 / 156 and 195 /
-//   139, FP64 392 / 267 and 694 / 405; it costs a little where the waits are short: FP32 256^2 44
-//   / 46 and 39 / 41.  (256 and 1,000 lines were measured; the line between them stands where a
-//   wait reaches about 50 us.)
+//   139, FP64 392 / 267 and 694 / 405.  FP32 loses up to 600 lines (100 x 300 39 / 41 and 35 / 38,
+//   500^2 79 / 83 and 70 / 77, 100 x 600 58 / 62 and 53 / 57) and gains from 800 (100 x 800 82 / 75 and
+//   73 / 70, 800^2 130 / 127 and 115 / 118, 64 x 1500 171 / 117 and 167 / 110).
 // * 3-D backward: FP32 40 x 40 x 500 353 / 129, 64 x 64 x 200 89 / 75, 128^3 85 / 85, 96^3 63 / 63;
 //   FP64 96^3 143 / 128.
 // * 3-D forward: FP32 gains from about 300 lines along y and z (60 x 100 x 200 146 / 96, 32 x 32 x

@@ -1,6 +1,6 @@
-"""Sweeps of deep 3-D grids, whose last blocks wait long for their first faces: results bit for bit
-those of the other schedules on both sides of the depth and the width at which the sweeps keep
-their instructions warm meanwhile; and on a deep, narrow grid the line sweeps of both types are
+"""Sweeps of deep grids, whose last blocks wait long for their first faces: results bit for bit those
+of the other schedules on both sides of the depth and the width at which the sweeps keep their
+instructions warm meanwhile, in 3-D and in 2-D; and on a deep, narrow grid the line sweeps of both types are
 the faster ones (two to three times), so that the automatic choice takes them."""
 import numpy as np
 import pytest
@@ -19,10 +19,11 @@ def solver(a, grid):
     return ilu
 
 
-@pytest.mark.parametrize("shape", [(10, 10, 270), (10, 10, 271), (9, 32, 249), (9, 33, 248), (5, 270, 12), (24, 24, 500)],
+@pytest.mark.parametrize("shape", [(10, 10, 270), (10, 10, 271), (9, 32, 249), (9, 33, 248), (5, 270, 12), (24, 24, 500),
+                                   (40, 700), (40, 701)],
                          ids=lambda s: "x".join(map(str, s)))
 def test_deep_grids_change_nothing(shape):
-    a = g.convdiff3d(*shape)
+    a = g.convdiff3d(*shape) if len(shape) == 3 else g.laplace2d(*shape)
     a = g.Csr(a.n, a.row_ptr, a.col_idx, a.values * np.random.default_rng(1).uniform(0.9, 1.1, a.values.size))
     _, b = g.random_rhs(a, seed=2)
     out = {}
