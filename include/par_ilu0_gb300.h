@@ -104,7 +104,7 @@ enum {
     LLJBASH_ILU_OPT_GRID = 6,
     /* shape of the line-pipeline sweeps (0 = automatic), next IluSolverSetup: lanes of a
      * warp along y (1, 4, 8; the rest along z; 2-D grids use 1), warps of a CTA along y
-     * and along z (at most 4 compute warps in all). */
+     * and along z (at most 4 compute warps in all: larger products are halved). */
     LLJBASH_ILU_OPT_GRID_WARP_Y = 7,
     LLJBASH_ILU_OPT_GRID_CTA_Y = 8,
     LLJBASH_ILU_OPT_GRID_CTA_Z = 9,
@@ -119,7 +119,8 @@ enum {
     LLJBASH_ILU_OPT_TICKET_ORDER = 11,
     /* factorisation kernel (results are the same for every choice): 0 (default,
      * automatic): the line pipeline for 7- / 5-point stencils in natural order (when
-     * LLJBASH_ILU_OPT_GRID allows it and the ticket order is 0), else one warp per row;
+     * LLJBASH_ILU_OPT_GRID allows it, the ticket order is 0, and a grid line fits in shared
+     * memory: up to 910 cells in 3-D, 11,000 in 2-D), else one warp per row;
      * 1: one warp per row; 2: one lane per row when no row has more than
      * 16 entries (each finished row publishes u_kk and its upper entries, rows waiting for
      * it poll exactly those values), else one warp per row.  Next IluSolverSetup. */

@@ -29,8 +29,8 @@ REF_SO = os.path.join(HERE, "_ref", "libref.so")
 REF_STRICT_SO = os.path.join(HERE, "_ref", "libref_strict.so")
 REF_OMP_SO = os.path.join(HERE, "_ref", "libref_omp.so")
 REF_STAGE = os.path.join(HERE, "_ref", "src")
-# where the reference checkout is read from (PAR_ILU0_REFERENCE_DIR overrides)
-DEFAULT_REFERENCE_DIR = "/root/reference"
+# where the reference checkout is read from (PAR_ILU0_REFERENCE_DIR overrides): beside this one
+DEFAULT_REFERENCE_DIR = os.path.join(os.path.dirname(os.path.dirname(HERE)), "reference")
 
 
 def reference_dir() -> str:

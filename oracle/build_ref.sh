@@ -12,8 +12,8 @@
 #
 #   oracle/build_ref.sh [REFERENCE_DIR]
 #
-# REFERENCE_DIR defaults to $PAR_ILU0_REFERENCE_DIR, else /root/reference.  When the
-# checkout is there, the sources are compiled where they lie and the files this build
+# REFERENCE_DIR defaults to $PAR_ILU0_REFERENCE_DIR, else the folder `reference` beside this
+# repository's.  When the checkout is there, the sources are compiled where they lie and the files this build
 # reads (and the reference's C test programs test/test.c, test/amd_test.c, which the
 # tests compile unchanged against this library's headers) are also staged under
 # oracle/_ref/src, so that a machine the working tree is
@@ -21,7 +21,7 @@
 # source this script accepts).  Nothing is copied into tracked files.
 set -euo pipefail
 HERE="$(cd "$(dirname "${BASH_SOURCE[0]}")" && pwd)"
-REF="${1:-${PAR_ILU0_REFERENCE_DIR:-/root/reference}}"
+REF="${1:-${PAR_ILU0_REFERENCE_DIR:-$(dirname "$(dirname "$HERE")")/reference}}"
 OUT="$HERE/_ref"
 STAGE="$OUT/src"
 mkdir -p "$OUT"

@@ -822,10 +822,10 @@ static bool detect_grid(int n, const int* rp, const int* ci, const std::vector<i
 // wz = 32 / wy along z; a 2-D grid, ny = 1, has wy = 1) and warps of a CTA along y and z
 // (by, bz).  Requested values (0 = automatic) are clamped to what the grid allows.
 // Automatic: 2-D one warp per CTA (handoffs through distributed shared memory cost no more
-// than those in a CTA, and each warp has an SM's pipes); 3-D 2 x 2 warps for FP32 and 2 x 1
-// for FP64 (elem 8), which leaves fewer blocks waiting beside the working ones: 128^3 FP64
-// forward / backward 131 / 176 us with 2 x 1 in clusters of 4, 192 / 297 us with 2 x 2;
-// FP32 82 / 77 us with 2 x 2 in clusters of 8, 96 / 87 us with 2 x 1).
+// than those in a CTA, and each warp has an SM's pipes); 3-D 2 x 2 warps for FP32 (forward /
+// backward, us, 2 x 2 and 2 x 1, in clusters of 8: 128^3 89 / 83 and 112 / 88, 96^3 66 / 64 and 67 /
+// 63, 200^3 196 / 196 and 195 / 185) and 2 x 1 for FP64 (elem 8), of whose stages and faces four
+// warps' fit one CTA only up to nx = 62.
 static LineGeom line_geometry(int nx, int ny, int nz, int wy_req, int by_req, int bz_req, int elem) {
     LineGeom g;
     g.nx = nx;
@@ -982,8 +982,10 @@ static bool configure_line(LinePack<T>& G, const DeviceInfo& dev, int max_cluste
     const size_t smem = std::max(static_cast<size_t>(std::max(line_smem_bytes<T, false>(G.g), line_smem_bytes<T, true>(G.g))),
                                  static_cast<size_t>(G.smem_floor));
     if (smem + 1024 > static_cast<size_t>(dev.smem_optin)) return false;
-    // for grids that do not fit at once clusters of 8 for FP32 and 4 for FP64 (the
-    // measurements above line_geometry)
+    // for grids that do not fit at once clusters of 8 for FP32 and 4 for FP64: forward / backward,
+    // us, in clusters of 4, 8 and 16: FP32 128^3 114 / 88, 89 / 83, 94 / 92, 200^3 174 / 170, 196 / 196,
+    // 229 / 232, 96^3 (all resident) 68 / 66, 66 / 64, 64 / 63; FP64 128^3 135 / 195, 145 / 217, 163 /
+    // 255, 200^3 299 / 464, 365 / 583, 484 / 775, 96^3 99 / 140, 92 / 135, 117 / 178
     const int most = G.g.ny == 1 ? 16 : (sizeof(T) == 4 ? 8 : 4);
     // 3-D blocks more than 130 (FP64) or 300 lines deep would wait past about 50 us: they are left
     // to the CTAs that finish first.  Forward sweeps whose instructions leave the cache meanwhile

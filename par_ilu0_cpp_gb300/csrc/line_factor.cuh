@@ -19,8 +19,11 @@
 // (a lane's rows lie a line apart in the CSR values: 32 sectors per entry), and a second
 // kernel takes them to the CSR values.  The warp-per-row kernel pays an L2 handoff and a
 // division chain per level.  Whole factorisations (packs of the sweeps included), ms, before
-// (warp per row) and now: 128^3 4.6 / 0.78, 101 x 90 x 75 2.4 / 0.37, 200^3 14.5 / 2.7, 384 x
-// 301 4.2 / 0.46, 1024^2 13.0 / 1.4, 32^2 0.35 / 0.07; a step takes 0.58 us.
+// (warp per row) and now: 128^3 4.6 / 0.79, 101 x 90 x 75 2.4 / 0.36, 200^3 14.5 / 2.3, 384 x
+// 301 4.2 / 0.47, 1024^2 13.0 / 1.4, 32^2 0.35 / 0.07; a step takes 0.58 us.  A CTA of one warp
+// fits in shared memory up to nx = 910 in 3-D (its faces hold 192 B per cell along x, its
+// stages 48 KB) and nx = 11,000 in 2-D; longer lines are factorised by the warp-per-row kernel
+// (900 x 12 x 12 0.82 ms, 950 x 12 x 12 3.8 ms).
 #pragma once
 
 #include "line_sweep.cuh"

@@ -29,9 +29,9 @@
 // product with `scale` included).  The compute warp touches only staged values, its faces
 // and the shuffles, a step is 70 ns (FP32) or 160 / 265 ns (FP64 forward / backward, whose
 // FP64 instructions alone take 93 / 186 ns on a scheduler), and a handoff between warps costs
-// two to three steps.  Inside GMRES, forward / backward, us: 128^3 FP32 87 / 84 (151 / 137
-// with a lane's own accesses), FP64 128 / 194 (247 / 622, block-local backward 566); 256^2
-// FP32 44 / 39 (95 / 84), FP64 71 / 123 (204 / block-local 447).
+// two to three steps.  Inside GMRES, forward / backward, us: 128^3 FP32 89 / 83 (151 / 137
+// with a lane's own accesses), FP64 135 / 194 (247 / 622, block-local backward 492); 256^2
+// FP32 45 / 40 (95 / 84), FP64 72 / 129 (204 / block-local 313).
 //
 // Blocks are taken from a ticket counter in dependency order (anti-diagonals of the block
 // grid), so a block only waits for blocks of smaller tickets, whose CTAs are running or
@@ -358,8 +358,8 @@ __device__ __forceinline__ void line_load_coef(unsigned a, int lane, LineCoef<do
 // (and for FP64 of the divisors) and its right-hand side [lane][kLinePitch]; per
 // compute warp a ring of kLineSlots + 1 chunks of results [lane][kLinePitch]; then the faces (consumer-indexed: slot w holds what warp w reads;
 // y-faces [nw][face_y()], z-faces [nw][face_z()]); then kLineIdle zeros that lanes without
-// a face read and kLineIdle values that lanes without a consumer write (so that no access
-// needs a predicate); then per compute warp and slot two mbarriers: [0] the chunk is staged (and the result ring has room for it), [1] the
+// a face read (so that no load needs a predicate) and kLineIdle values, the address of lanes
+// without a consumer, whose stores are predicated off; then per compute warp and slot two mbarriers: [0] the chunk is staged (and the result ring has room for it), [1] the
 // chunk is computed.
 template <class T, bool UPPER>
 struct LineStage {

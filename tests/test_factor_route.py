@@ -41,6 +41,15 @@ def test_requests_for_other_kernels_are_kept(options):
     assert info(stencil((20, 11, 13), seed=1), options).factor_line == 0
 
 
+@pytest.mark.parametrize("nx,line", [(910, 1), (911, 0)])
+def test_longest_grid_lines(nx, line):
+    """The last line whose faces fit in a CTA's shared memory, and the next, which the other kernel
+    takes, with the same factors."""
+    a = stencil((nx, 5, 3), seed=2)
+    assert info(a).factor_line == line
+    assert same(factor(a, 0)[0], factor(a, 1)[0])
+
+
 def test_other_patterns_do_not():
     assert info(g.lognormal27(8, seed=1)).factor_line == 0
     assert info(api.iluk_symbolic(g.laplace2d(30), 1)[0]).factor_line == 0
